@@ -194,29 +194,29 @@ SPC5CUDA_API spc5cuda_status spc5cuda_mat_info(const spc5cuda_mat* mat, spc5cuda
  *             stream);
  *   ROWS   -- the thread-per-sub-row kernel; SPC5CUDA_ERR_UNSUPPORTED on a
  *             converted matrix with a block-row that does not fit;
- *   SORTED -- the length-sorted plan: the handle holds its headers and
- *             values with the block-rows sorted by size (the largest ones
- *             as multiply-add chains at r = 2, 4, 8, in segments at r = 1)
- *             instead of in the reference order, and SpMV runs each size
- *             class with the kernel and lanes per block-row that suit it.
- *             AUTO uses it when some block-row does not fit the row kernel
- *             (power-law and other irregular matrices).
+ *   SORTED -- the sorted plan: the handle holds its values with the rows
+ *             sorted by size, long rows four (float layout: two) to a warp,
+ *             short rows one to a lane, each value with its x index, instead
+ *             of in the reference order.  AUTO uses it when some block-row
+ *             does not fit the row kernel (power-law and other irregular
+ *             matrices).
  * spc5cuda_mat_kernel reports the kernel SpMV uses now (GROUPS, ROWS or
  * SORTED; AUTO before conversion).  Selecting SORTED (or AUTO, where it picks
  * the plan) on a converted matrix builds the plan and releases the
- * reference-order arrays; selecting GROUPS or ROWS rebuilds them from the
+ * reference-order values; selecting GROUPS or ROWS rebuilds them from the
  * plan and releases the plan.  Both synchronise the device.
  * spc5cuda_get_arrays and spc5cuda_decode_coo return the reference order
  * whichever form the handle holds; spc5cuda_batch_create rebuilds it into the
- * handle (which then holds both). */
+ * handle, which then holds them twice. */
 #define SPC5CUDA_KERNEL_AUTO 0
 #define SPC5CUDA_KERNEL_GROUPS 1
 #define SPC5CUDA_KERNEL_ROWS 2
 #define SPC5CUDA_KERNEL_SORTED 3
 SPC5CUDA_API spc5cuda_status spc5cuda_mat_set_kernel(spc5cuda_mat* mat, int kernel);
 SPC5CUDA_API spc5cuda_status spc5cuda_mat_kernel(const spc5cuda_mat* mat, int* kernel);
-/* Kernel launches one spc5cuda_spmv of a converted handle makes now (one
- * per part of the length-sorted plan, else 1; 0 for an empty matrix). */
+/* Kernel launches one spc5cuda_spmv of a converted handle makes now (the
+ * sorted plan: one for its long rows, one for its short rows; else 1; 0 for an
+ * empty matrix). */
 SPC5CUDA_API spc5cuda_status spc5cuda_mat_spmv_launches(const spc5cuda_mat* mat, int* launches);
 
 /* SPC5_{r}rVc_block_count (spc5.hpp:510-513, 635-638, 764-767, 890-893):
@@ -341,12 +341,9 @@ typedef struct spc5cuda_server_config {
     long hbm_budget;  /* bytes for resident matrices + staging buffers    */
     int mixed;        /* 0: F64 matrices, double x/y; 1: F32 or F32_V8
                          matrices, float x, double y (FP64 accumulation)  */
-    int plan_serial;  /* 0 (default): a sorted-plan matrix forks its parts
-                         onto the plan's own two streams (measured faster:
-                         15.5k against 13.7k req/s at saturation on the
-                         serving bench); 1: the parts run in order on the
-                         slot's stream, so launches of one matrix in
-                         different slots share no plan stream             */
+    int plan_serial;  /* accepted, without effect: a sorted-plan matrix runs
+                         on the slot's own stream, so launches of one matrix
+                         in different slots share nothing                 */
 } spc5cuda_server_config;
 
 typedef struct spc5cuda_server_stats {

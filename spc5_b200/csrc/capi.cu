@@ -77,8 +77,7 @@ void spc5cuda::valptr_from_headers(int mask_bytes, int r, int nbr, const int* br
 }
 
 // The library's own stream-ordered memory pool on the current device: the
-// per-call scratch of the drop-in symbols and of the plan's chain part comes
-// from it, and it keeps freed memory for the next call (release threshold:
+// per-call scratch of the drop-in symbols comes from it, and it keeps freed memory for the next call (release threshold:
 // never), so repeated calls do not go back to the driver.  One pool per
 // device for the process lifetime.
 cudaMemPool_t spc5cuda::scratch_pool() {
@@ -329,11 +328,11 @@ spc5cuda_status spc5cuda_mat_set_kernel(spc5cuda_mat* m, int kernel) {
         m->kernel = kernel;
         if (m->r != 0 && m->wants_plan() && !m->plan) build_sorted_plan(m, nullptr);
         // the group and row kernels run on the handle's own arrays: bring
-        // them back from the sorted copy if it held the only one, then
-        // release the copy
+        // the values back from the plan if it held the only copy, then
+        // release it
         if (m->plan && !m->use_plan()) {
-            m->restore_original(nullptr);
-            SPC5_CUDA(cudaDeviceSynchronize());  // no SpMV may still read the copy
+            m->restore_values(nullptr);
+            SPC5_CUDA(cudaDeviceSynchronize());  // no SpMV may still read the plan
             m->plan.reset();
         }
     });
@@ -344,11 +343,7 @@ spc5cuda_status spc5cuda_mat_spmv_launches(const spc5cuda_mat* m, int* launches)
         require(m && launches, SPC5CUDA_ERR_INVALID, "null");
         require(m->r != 0, SPC5CUDA_ERR_FORMAT, "matrix is not converted");
         if (m->nrows == 0) *launches = 0;
-        else if (m->use_plan()) {
-            *launches = 0;
-            for (const auto& part : m->plan->parts) *launches += part.chains ? 2 : 1;
-        }
-        else *launches = 1;
+        else *launches = m->use_plan() ? m->plan->launches() : 1;
     });
 }
 
@@ -421,19 +416,16 @@ spc5cuda_status spc5cuda_get_arrays(const spc5cuda_mat* m, int* rowsSize, unsign
         const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
         if (rowsSize)
             SPC5_CUDA(cudaMemcpyAsync(rowsSize, m->brptr.p, m->brptr.bytes, kind, s));
-        const void* hsrc = m->headers.p;
         const void* vsrc = m->values.p;
-        // the sorted copy holds the only one: the reference order, rebuilt
-        const bool rebuild = m->original_dropped && (headers || values);
-        DevBuf th(rebuild ? std::max<size_t>(16, m->header_bytes()) : 0, s);
+        // the plan holds the only copy of the values: the reference order, rebuilt
+        const bool rebuild = m->values_dropped && values;
         DevBuf tv(rebuild ? std::max<size_t>(16, m->value_bytes()) : 0, s);
         if (rebuild) {
-            rebuild_original(m, th.as<uint8_t>(), tv.p, s);
-            hsrc = th.p;
+            rebuild_values(m, tv.p, s);
             vsrc = tv.p;
         }
         if (headers && m->header_bytes())
-            SPC5_CUDA(cudaMemcpyAsync(headers, hsrc, m->header_bytes(), kind, s));
+            SPC5_CUDA(cudaMemcpyAsync(headers, m->headers.p, m->header_bytes(), kind, s));
         if (values && m->value_bytes())
             SPC5_CUDA(cudaMemcpyAsync(values, vsrc, m->value_bytes(), kind, s));
         if (to_host) SPC5_CUDA(cudaStreamSynchronize(s));

@@ -106,12 +106,10 @@ spc5cuda_status spc5cuda_decode_coo(const spc5cuda_mat* m, int* rows, int* cols,
         const int nbr = m->nbr();
         const uint8_t* hdr = m->headers.as<uint8_t>();
         const void* vals = m->values.p;
-        const bool rebuild = m->original_dropped;  // the sorted copy holds the only one
-        DevBuf th(rebuild ? std::max<size_t>(16, m->header_bytes()) : 0, s);
+        const bool rebuild = m->values_dropped;  // the plan holds the only copy
         DevBuf tv(rebuild ? std::max<size_t>(16, m->value_bytes()) : 0, s);
         if (rebuild) {
-            rebuild_original(m, th.as<uint8_t>(), tv.p, s);
-            hdr = th.as<uint8_t>();
+            rebuild_values(m, tv.p, s);
             vals = tv.p;
         }
         if (mask_bytes_of(m->value_type) == 1)

@@ -4,10 +4,9 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <memory>
-#include <mutex>
 #include <new>
-#include <vector>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -135,90 +134,46 @@ inline void require(bool cond, spc5cuda_status s, const char* what) {
 }
 
 
-// One part of the length-sorted plan: sorted block-rows [a, b), run by the
-// row kernel with `lanes` lanes per block-row (split: one range per warp), or
-// by the group kernel when lanes == 0 (split: one range per group); split
-// holds nsplit + 1 block-row starts.  The part of the block-rows too large
-// to stage (nseg = b - a > 0, a = 0) is either the chain part (chains: the
-// multiply-add chains below; two launches) or segmented: cut into segments
-// that are, interleaved per warp; vbrptr / vvalptr are the segments' block
-// and value offsets and split their per-warp ranges.
-struct SpmvPart {
-    int lanes = 0;
-    int a = 0, b = 0;
-    int nseg = 0;
-    bool chains = false;
-    Owned split;
-    int nsplit = 0;
-    Owned vbrptr, vvalptr;
-    // the chain part (chain.cu): one multiply-add chain per (block-row,
-    // sub-row, column) of the nseg largest block-rows, chain id
-    // (i * r + s) * VS + c.  The nchains non-empty ones, sorted by length
-    // (slen, corder: chain ids), cut into slices of 32 chains, entry j of the
-    // slice's lane l at slice_off[slice] + 32 j + l (cval: value, ccol: x
-    // index); cmask[i * r + s] bit c: chain c of that sub-row is not empty.
-    long nchains = 0;
-    long entries = 0;  // values in the chains
-    int nslices = 0;
-    Owned slen, corder, slice_off, cval, ccol, cmask;
-};
-
-// A copy of the matrix with its block-rows sorted by size (plan.cu).  Its
-// parts write disjoint rows of y, so an SpMV forks them onto two streams of
-// the plan and joins them back to the caller's stream.
+// The sorted plan of an irregular matrix (plan.cu): the rows sorted by size,
+// the long rows stored as warp streams, the short rows one per lane
+// (stream.cuh); it holds the plan's only copy of the values.  Launches share
+// no state, so calls on different streams overlap freely.
 struct SortedPlan {
-    Owned sbrptr, sheaders, svalues, svalptr, perm;
-    std::vector<SpmvPart> parts;
-    bool in_order = false;  // run the parts one after another on the caller's stream
-    cudaStream_t aux[2] = {nullptr, nullptr};
-    cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
-    std::mutex mu;  // one fork/join at a time (the events are shared)
-    SortedPlan() = default;
-    SortedPlan(const SortedPlan&) = delete;
-    SortedPlan& operator=(const SortedPlan&) = delete;
-    ~SortedPlan() {
-        for (auto& st : aux)
-            if (st) cudaStreamDestroy(st);
-        if (fork) cudaEventDestroy(fork);
-        for (auto& e : join)
-            if (e) cudaEventDestroy(e);
-    }
+    static constexpr int CLASSES = 5;
+    static constexpr int SHORT_VALUES = 16;
+    Owned perm;   // nrows: matrix row of each sorted row
+    Owned key;    // nrows: sort key of each sorted row (stream.cuh)
+    Owned val;    // values: the long rows' in step order, then the short rows' in lane order
+    Owned col;    // their x indices
+    Owned mask;   // long rows: active-lane mask of every step
+    Owned sstep;  // long slabs + 1: first step of each
+    Owned sval;   // long slabs + 1: first value of each
+    Owned chains; // short rows: mask of the non-empty chains
+    int row_end[CLASSES] = {0};   // sorted rows up to the end of each class of long rows
+    int slab_end[CLASSES] = {0};  // slabs up to the end of each class
+    int short_rows[SHORT_VALUES + 1] = {0};  // rows of n values; they follow the long ones
+    int short_slabs = 0;
+    long long_values = 0;
     long bytes() const {
-        long n = long(sbrptr.bytes + sheaders.bytes + svalues.bytes + svalptr.bytes + perm.bytes);
-        for (const auto& p : parts)
-            n += long(p.split.bytes + p.vbrptr.bytes + p.vvalptr.bytes + p.slen.bytes + p.corder.bytes +
-                      p.slice_off.bytes + p.cval.bytes + p.ccol.bytes + p.cmask.bytes);
-        return n;
+        return long(perm.bytes + key.bytes + val.bytes + col.bytes + mask.bytes + sstep.bytes + sval.bytes +
+                    chains.bytes);
     }
+    // kernel launches of one SpMV: the long rows', the short rows'
+    int launches() const { return (slab_end[CLASSES - 1] > 0 ? 1 : 0) + (short_slabs > 0 ? 1 : 0); }
 };
 
-// The length-sorted plan of a converted matrix (plan.cu; synchronises s),
-// and the view of one of its parts.
+// The sorted plan of a converted matrix (synchronises s).
 void build_sorted_plan(spc5cuda_mat* m, cudaStream_t s);
-BetaView plan_view(const spc5cuda_mat* m, const SpmvPart& part);
-// The reference-order headers and values of a handle whose plan holds the
-// only copy, written to device buffers of m->headers / m->values size.
-void rebuild_original(const spc5cuda_mat* m, uint8_t* headers, void* values, cudaStream_t s);
-// The chain part (chain.cu): built from the sorted copy's block-rows
-// [0, part.nseg), whose values it then drops from the copy (synchronises s);
-// its values back in the reference order; y += A x and Y += A X over it.
-void build_chains(spc5cuda_mat* m, SortedPlan* plan, SpmvPart& part, cudaStream_t s);
-void unchain_values(const spc5cuda_mat* m, const SpmvPart& part, void* values, cudaStream_t s);
-void chain_part_spmv(const spc5cuda_mat* m, const SpmvPart& part, const void* x, void* y, bool mixed,
-                     cudaStream_t s);
-void chain_part_spmm(const spc5cuda_mat* m, const SpmvPart& part, int k, const void* x, long ldx, long xcs, void* y,
-                     long ldy, long ycs, bool mixed, cudaStream_t s);
-void launch_iota(long n, int* a, cudaStream_t s);
+// The reference-order values of a handle whose plan holds the only copy,
+// written to a device buffer of m->value_bytes().
+void rebuild_values(const spc5cuda_mat* m, void* values, cudaStream_t s);
 // y += A x through the plan (x, y of the handle's types; mixed: F32 or
-// F32_V8 handle, float x, double y).  fork: run the parts concurrently on the
-// plan's two streams and join them back to s (one such call at a time per
-// handle); otherwise one after another on s, so that calls on different
-// streams (the request loop's slots) overlap without sharing plan streams.
-void plan_spmv(const spc5cuda_mat* m, const void* x, void* y, bool mixed, cudaStream_t s, bool fork = true);
-// Y += A X through the plan with the staged SpMM (element (row i, rhs q) of
-// X at x[i * ldx + q * xcs], likewise Y).
+// F32_V8 handle, float x, double y).
+void plan_spmv(const spc5cuda_mat* m, const void* x, void* y, bool mixed, cudaStream_t s);
+// Y += A X through the plan (element (row i, rhs q) of X at
+// x[i * ldx + q * xcs], likewise Y).
 void plan_spmm(const spc5cuda_mat* m, int k, const void* x, long ldx, long xcs, void* y, long ldy, long ycs,
-               bool mixed, cudaStream_t s, bool fork = true);
+               bool mixed, cudaStream_t s);
 
 }  // namespace spc5cuda
 
@@ -244,10 +199,10 @@ struct spc5cuda_mat {
     int nwarps = 0;
     int kernel = SPC5CUDA_KERNEL_AUTO;  // SpMV kernel choice (spc5cuda_mat_set_kernel)
     bool rows_ok = false;               // every block-row fits the row kernel's buffers
-    std::unique_ptr<spc5cuda::SortedPlan> plan;  // length-sorted copy (irregular matrices)
-    // the plan holds the only copy of headers and values (set when the plan
-    // is built and serves SpMV): the reference order is rebuilt on demand
-    bool original_dropped = false;
+    std::unique_ptr<spc5cuda::SortedPlan> plan;  // rows sorted by size (irregular matrices)
+    // the plan holds the only copy of the values (set when the plan is built
+    // and serves SpMV): the reference order is rebuilt on demand
+    bool values_dropped = false;
 
     int nbr() const { return r ? spc5cuda::div_up(nrows, r) : 0; }
     BetaView view() const {
@@ -300,24 +255,21 @@ struct spc5cuda_mat {
         return size_t(nblocks) * size_t(4 + r * spc5cuda::mask_bytes_of(value_type));
     }
     size_t value_bytes() const { return size_t(nnz) * size_t(spc5cuda::value_bytes_of(value_type)); }
-    // Bring the reference-order headers and values back into the handle
-    // (synchronises s); a no-op unless the plan holds the only copy.
-    void restore_original(cudaStream_t s) {
-        if (!original_dropped) return;
-        Owned h, v;
-        h.alloc(std::max<size_t>(header_bytes(), 16));
+    // Bring the reference-order values back into the handle (synchronises s);
+    // a no-op unless the plan holds the only copy.
+    void restore_values(cudaStream_t s) {
+        if (!values_dropped) return;
+        Owned v;
         v.alloc(std::max<size_t>(value_bytes(), 16));
-        spc5cuda::rebuild_original(this, h.as<uint8_t>(), v.p, s);
+        spc5cuda::rebuild_values(this, v.p, s);
         SPC5_CUDA(cudaStreamSynchronize(s));
-        headers = std::move(h);
         values = std::move(v);
-        original_dropped = false;
+        values_dropped = false;
     }
     long device_bytes() const {
         return long(rowptr.bytes + colidx.bytes + values.bytes + brptr.bytes + headers.bytes +
                     valptr.bytes + gstart.bytes + wstart.bytes) + (plan ? plan->bytes() : 0L);
     }
-    // The per-group block-row ranges for the current device.
     // The per-group block-row ranges for the current device, and the per-warp
     // ranges of the thread-per-sub-row kernel when every block-row fits it.
     void build_partition(cudaStream_t s) {
@@ -336,7 +288,7 @@ struct spc5cuda_mat {
             nwarps = 0;
             wstart.release();
         }
-        restore_original(s);  // the plan may hold the only copy
+        restore_values(s);  // the plan may hold the only copy
         plan.reset();
         if (wants_plan()) spc5cuda::build_sorted_plan(this, s);
     }

@@ -51,13 +51,6 @@ struct BetaView {
     // starts of the per-warp ranges; null selects the group kernel
     const int* wstart = nullptr;
     int nwarps = 0;
-    int lanes = 0;               // row kernel: lanes per block-row (0: r)
-    // row kernel: > 0 when these arrays hold the segments of nseg long
-    // block-rows, interleaved per warp (the sorted plan's largest part)
-    int nseg = 0;
-    // block-row of y for each block-row of these arrays (null: the same);
-    // set when the arrays are a reordered copy of the matrix
-    const int* perm = nullptr;
     // when set, the launch does its work only if *run_if == run_if_value (a
     // device word written by an earlier kernel on the same stream)
     const int* run_if = nullptr;
@@ -70,8 +63,6 @@ int spmv_groups(int vs, int r);
 
 // gstart[0..ngroups] = block-row ranges holding ~nblocks/ngroups blocks each.
 void launch_partition(int nbr, const int* brptr, int ngroups, int* gstart, cudaStream_t s);
-// The same over block-rows [a, b): gstart[0] = a, gstart[ngroups] = b.
-void launch_partition_range(int a, int b, const int* brptr, int ngroups, int* gstart, cudaStream_t s);
 
 void launch_spmv_f64(const BetaView& m, const double* x, double* y, cudaStream_t s);
 
@@ -80,21 +71,8 @@ void launch_spmv_f64(const BetaView& m, const double* x, double* y, cudaStream_t
 // staging buffers, and the largest block-row of a converted matrix
 // (synchronises s).
 // (vt: the handle's value type, SPC5CUDA_F64 / F32 / F32_V8.)
-int rows_warps(int vt, int r, int lanes = 0);
+int rows_warps(int vt, int r);
 bool rows_fit(int vt, int r, int max_blocks, int max_values);
-// Size of a block-row in units of one lane's share of a row-kernel chunk:
-// the block-row fits a chunk of 32 / L block-rows with L lanes each when
-// rows_lane_units(...) <= L * rows_unit().
-long rows_lane_units(int vt, int r, int nblocks, int nvalues);
-long rows_unit();
-// Lanes per block-row of the segmented part of a sorted plan (the largest
-// block-rows), measured on B200 on the N = 4M power-law matrix: more lanes
-// give longer segments and more warps, fewer give more block-rows per warp
-// instruction.
-constexpr int seg_lanes(int r) { return r == 1 ? 4 : (r == 2 ? 8 : r); }
-// Header and value bytes of one warp's staging buffer.
-int rows_hb();
-int rows_vb();
 void blockrow_max(int nbr, const int* brptr, const int* valptr, int* max_blocks, int* max_values,
                   cudaStream_t s);
 // The same test on the device, without a host round trip: work[0] = 1 when
@@ -163,9 +141,8 @@ int batch_kc(int r, int k);
 void launch_batch(int kind, int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs,
                   int ctas, cudaStream_t s);
 // Right-hand sides per pass of the staged SpMM for VS columns per block,
-// rows-per-block r and k right-hand sides left (seg: the segmented part of a
-// sorted plan, run with seg_lanes(r) lanes per block-row).
-int spmm_rows_kc(int vs, int r, int k, bool seg = false);
+// rows-per-block r and k right-hand sides left.
+int spmm_rows_kc(int vs, int r, int k);
 // Most right-hand sides per pass of the staged SpMM with `lanes` lanes per
 // block-row: r x (vs / lanes columns per lane) x kc accumulators stay at
 // most 32, kc at most 16.

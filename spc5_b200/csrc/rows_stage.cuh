@@ -27,8 +27,8 @@ constexpr int WARPS = THREADS / 32;
 constexpr int HB = 1536;  // header bytes of one warp's staging buffer
 constexpr int VB = 6144;  // value bytes of one warp's staging buffer
 // The multi-RHS kernels are limited by registers to 4 CTAs per SM, so they
-// stage larger chunks (every block-row or segment cut for the buffers above
-// fits these).
+// stage larger chunks (every block-row that fits the buffers above fits
+// these).
 constexpr int MM_HB = 2048;
 constexpr int MM_VB = 8192;
 constexpr unsigned FULL = 0xffffffffu;
@@ -71,15 +71,14 @@ struct Chunk {
 // Walks block-rows [r_begin, r_stop) of one matrix (warp-uniform bounds):
 // stage a chunk into wbuf, load the next chunk's bounds while the copies fly,
 // call compute(chunk, staged header words, staged values), repeat.  A chunk
-// holds at most `cap` (<= 32 / L) block-rows: as many as fit the buffer.  The
+// holds at most cap = 32 / L block-rows: as many as fit the buffer.  The
 // caller guarantees that every block-row alone fits the buffer.
 template <class LT, int R, class V, int L, int HB_ = HB, int VB_ = VB, class F>
 __device__ __forceinline__ void walk(const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
                                      const V* __restrict__ values, const int* __restrict__ valptr,
-                                     int r_begin, int r_stop, unsigned char* wbuf, F&& compute,
-                                     int cap = 32 / L) {
+                                     int r_begin, int r_stop, unsigned char* wbuf, F&& compute) {
     using G = Geo<LT, R, V, L>;
-    constexpr int S = G::STRIDE, EPU = G::EPU;
+    constexpr int S = G::STRIDE, EPU = G::EPU, cap = 32 / L;
     if (r_begin >= r_stop) return;
     const int lane = threadIdx.x & 31;
     const uint32_t s_h = uint32_t(__cvta_generic_to_shared(wbuf));

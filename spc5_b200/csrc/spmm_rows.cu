@@ -8,8 +8,7 @@
 // staged header once, loads its KC x values per column (only where some
 // sub-row has a value in that column: blocks at the right edge may reach
 // past the last column), reads each of its values once from shared memory
-// and issues KC multiply-adds with it.  The sorted plan's parts run here too
-// (the block-row permutation, and the segments of its largest block-rows).
+// and issues KC multiply-adds with it.
 //
 // Arithmetic per right-hand side j is the SpMV's (src/spc5.hpp:2309-2715):
 // accumulator (i, j) of column c receives fma(value, x[col + c][j], acc) for
@@ -33,30 +32,22 @@ using rows::FULL;
 
 // Lanes per block-row of the staged SpMM: one column per lane for double
 // blocks (8 columns); for float blocks (16 columns) two per lane, except at
-// r = 8 where one column per lane keeps four right-hand sides per pass.  The
-// segmented part of a sorted plan keeps the plan's lanes (seg_lanes).
-template <class LT, int R, bool SEG>
+// r = 8 where one column per lane keeps four right-hand sides per pass.
+template <class LT, int R>
 constexpr int mm_lanes() {
-    if constexpr (SEG) return seg_lanes(R);
     return (Layout<LT>::VS == 16 && R == 8) ? 16 : 8;
 }
 
 // Y += A X over block-rows [r_begin, r_stop) of one matrix for right-hand
-// sides [0, KC) of xm / ym (already offset to the pass's first one); perm
-// (if not null) maps a block-row of these arrays to its block-row of Y.  SEG:
-// the block-rows are the interleaved segments of ng long block-rows (chunk k
-// holds segment k of each, as the segmented row kernel reads them), whose
-// block-rows of Y are perm[seg_base + slot]; a lane keeps its accumulators
-// over all chunks and Y is updated once, after the last.
-template <class LT, int R, int KC, class V, class X, class A, class Y, bool SEG>
+// sides [0, KC) of xm / ym (already offset to the pass's first one).
+template <class LT, int R, int KC, class V, class X, class A, class Y>
 __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brptr,
                                          const uint8_t* __restrict__ headers, const V* __restrict__ values,
                                          const int* __restrict__ valptr, int r_begin, int r_stop,
-                                         const int* __restrict__ perm, int ng, int seg_base,
                                          const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym,
                                          long ldy, long ycs, unsigned char* wbuf) {
     constexpr int VS = Layout<LT>::VS;
-    constexpr int L = mm_lanes<LT, R, SEG>();  // lanes per block-row
+    constexpr int L = mm_lanes<LT, R>();  // lanes per block-row
     constexpr int CPL = VS / L;                // columns per lane: q + L k
     constexpr int LOGL = L == 16 ? 4 : (L == 8 ? 3 : (L == 4 ? 2 : (L == 2 ? 1 : 0)));
     using G = rows::Geo<LT, R, V, L, rows::MM_HB, rows::MM_VB>;
@@ -159,7 +150,7 @@ __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brpt
         const int b_stop = mine ? b_mine : 0;
         int v = (mine ? (slot > 0 ? v_prev : ch.v_lo) : 0) - ch.v_al;
 
-        if constexpr (!SEG) zero();
+        zero();
         while (__any_sync(FULL, b < b_stop)) {
             int col[U];
             uint32_t mw[U][MW];
@@ -209,37 +200,25 @@ __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brpt
             }
             b += U;
         }
-        if constexpr (!SEG) flush(mine, mine ? (perm ? __ldg(perm + ch.r0 + slot) : ch.r0 + slot) : 0);
+        flush(mine, ch.r0 + slot);
     };
-    if constexpr (SEG) {
-        zero();
-        rows::walk<LT, R, V, L, rows::MM_HB, rows::MM_VB>(brptr, headers, values, valptr, r_begin, r_stop, wbuf,
-                                                          compute, ng);
-        flush(slot < ng, slot < ng ? __ldg(perm + seg_base + slot) : 0);
-    } else {
-        rows::walk<LT, R, V, L, rows::MM_HB, rows::MM_VB>(brptr, headers, values, valptr, r_begin, r_stop, wbuf,
-                                                          compute);
-    }
+    rows::walk<LT, R, V, L, rows::MM_HB, rows::MM_VB>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
 }
 
-// One matrix: warp w owns block-rows [wstart[w], wstart[w + 1]).  SEG: warp
-// w owns the segments of long block-rows w * 32 / L + slot (nseg in all).
-template <class LT, int R, int KC, class V, class X, class A, class Y, bool SEG>
+// One matrix: warp w owns block-rows [wstart[w], wstart[w + 1]).
+template <class LT, int R, int KC, class V, class X, class A, class Y>
 __global__ void __launch_bounds__(rows::THREADS)
     k_spmm_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
                 const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart,
-                int nwarps, const int* __restrict__ perm, int nseg, const X* __restrict__ xm, long ldx, long xcs,
-                Y* __restrict__ ym, long ldy, long ycs) {
-    constexpr int L = mm_lanes<LT, R, SEG>();
-    using G = rows::Geo<LT, R, V, L, rows::MM_HB, rows::MM_VB>;
+                int nwarps, const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym, long ldy, long ycs) {
+    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), rows::MM_HB, rows::MM_VB>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
     const int warp = blockIdx.x * rows::WARPS + wi;
     if (warp >= nwarps) return;  // warp-uniform
     const int r_begin = __ldg(wstart + warp), r_stop = __ldg(wstart + warp + 1);
-    const int ng = SEG ? min(G::SPW, nseg - warp * G::SPW) : 0;
-    mm_range<LT, R, KC, V, X, A, Y, SEG>(nrows, brptr, headers, values, valptr, r_begin, r_stop, perm, ng,
-                                         warp * G::SPW, xm, ldx, xcs, ym, ldy, ycs, smem + wi * G::BUF_BYTES);
+    mm_range<LT, R, KC, V, X, A, Y>(nrows, brptr, headers, values, valptr, r_begin, r_stop, xm, ldx, xcs, ym, ldy, ycs,
+                                    smem + wi * G::BUF_BYTES);
 }
 
 // Batched: warps walk the job list with the grid's warp count as stride; job
@@ -248,18 +227,16 @@ __global__ void __launch_bounds__(rows::THREADS)
 template <class LT, int R, int KC, class V, class X, class A, class Y>
 __global__ void __launch_bounds__(rows::THREADS)
     k_spmm_rows_batch(const BatchMat* __restrict__ mats, const BatchJob* __restrict__ jobs, int njobs) {
-    using G = rows::Geo<LT, R, V, mm_lanes<LT, R, false>(), rows::MM_HB, rows::MM_VB>;
+    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), rows::MM_HB, rows::MM_VB>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
     const int nw = gridDim.x * rows::WARPS;
     for (int j = blockIdx.x * rows::WARPS + wi; j < njobs; j += nw) {  // warp-uniform
         const BatchJob job = jobs[j];
         const BatchMat& m = mats[job.mat];
-        mm_range<LT, R, KC, V, X, A, Y, false>(m.nrows, m.brptr, m.headers, static_cast<const V*>(m.values),
-                                               m.valptr, job.r_begin, job.r_end, nullptr, 0, 0,
-                                               static_cast<const X*>(m.x) + job.kofs, m.ldx, 1L,
-                                               static_cast<Y*>(m.y) + job.kofs, m.ldy, 1L,
-                                               smem + wi * G::BUF_BYTES);
+        mm_range<LT, R, KC, V, X, A, Y>(m.nrows, m.brptr, m.headers, static_cast<const V*>(m.values), m.valptr,
+                                        job.r_begin, job.r_end, static_cast<const X*>(m.x) + job.kofs, m.ldx, 1L,
+                                        static_cast<Y*>(m.y) + job.kofs, m.ldy, 1L, smem + wi * G::BUF_BYTES);
     }
 }
 
@@ -270,12 +247,12 @@ void set_smem(K kernel, int bytes) {
 
 // Calls f(integral_constant<R>, integral_constant<KC>) for r in {1, 2, 4, 8}
 // and kc a power of two up to mm_kc_limit of the kernel's lanes.
-template <class LT, bool SEG, class F>
+template <class LT, class F>
 void dispatch_rkc(int r, int kc, F&& f) {
     using std::integral_constant;
     auto with_r = [&](auto RC) {
         constexpr int R_ = decltype(RC)::value;
-        constexpr int KMAX = mm_kc_limit(Layout<LT>::VS, R_, mm_lanes<LT, R_, SEG>());
+        constexpr int KMAX = mm_kc_limit(Layout<LT>::VS, R_, mm_lanes<LT, R_>());
         switch (kc) {
             case 1: f(RC, integral_constant<int, 1>{}); return true;
             case 2: if constexpr (KMAX >= 2) { f(RC, integral_constant<int, 2>{}); return true; } break;
@@ -295,35 +272,24 @@ void dispatch_rkc(int r, int kc, F&& f) {
     if (!done) throw Error(SPC5CUDA_ERR_INVALID, "unsupported (r, right-hand sides per pass)");
 }
 
-template <class LT, bool SEG, class V, class X, class A, class Y>
-void spmm_rows_run(const BetaView& m, int k, const X* x, long ldx, long xcs, Y* y, long ldy, long ycs,
-                   cudaStream_t s) {
-    const int ctas = (m.nwarps + rows::WARPS - 1) / rows::WARPS;
-    const V* vals = static_cast<const V*>(m.values);
-    for (int k0 = 0; k0 < k;) {
-        const int kc = spmm_rows_kc(Layout<LT>::VS, m.r, k - k0, SEG);
-        dispatch_rkc<LT, SEG>(m.r, kc, [&](auto RC, auto KCC) {
-            constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-            constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_, SEG>(), rows::MM_HB, rows::MM_VB>::SMEM;
-            auto kern = k_spmm_rows<LT, R_, KC_, V, X, A, Y, SEG>;
-            set_smem(kern, SMEM);
-            kern<<<ctas, rows::THREADS, SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart,
-                                                   m.nwarps, m.perm, m.nseg, x + long(k0) * xcs, ldx, xcs,
-                                                   y + long(k0) * ycs, ldy, ycs);
-        });
-        k0 += kc;
-    }
-}
-
 template <class LT, class V, class X, class A, class Y>
 void spmm_rows_impl(const BetaView& m, int k, const X* x, long ldx, long xcs, Y* y, long ldy, long ycs,
                     cudaStream_t s) {
     if (m.nbr <= 0 || k <= 0 || m.nwarps <= 0) return;
-    if (m.nseg > 0) {
-        if (m.lanes != seg_lanes(m.r)) throw Error(SPC5CUDA_ERR_INVALID, "segment lanes");
-        spmm_rows_run<LT, true, V, X, A, Y>(m, k, x, ldx, xcs, y, ldy, ycs, s);
-    } else {
-        spmm_rows_run<LT, false, V, X, A, Y>(m, k, x, ldx, xcs, y, ldy, ycs, s);
+    const int ctas = (m.nwarps + rows::WARPS - 1) / rows::WARPS;
+    const V* vals = static_cast<const V*>(m.values);
+    for (int k0 = 0; k0 < k;) {
+        const int kc = spmm_rows_kc(Layout<LT>::VS, m.r, k - k0);
+        dispatch_rkc<LT>(m.r, kc, [&](auto RC, auto KCC) {
+            constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
+            constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), rows::MM_HB, rows::MM_VB>::SMEM;
+            auto kern = k_spmm_rows<LT, R_, KC_, V, X, A, Y>;
+            set_smem(kern, SMEM);
+            kern<<<ctas, rows::THREADS, SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart,
+                                                   m.nwarps, x + long(k0) * xcs, ldx, xcs, y + long(k0) * ycs, ldy,
+                                                   ycs);
+        });
+        k0 += kc;
     }
     SPC5_CUDA(cudaGetLastError());
 }
@@ -331,9 +297,9 @@ void spmm_rows_impl(const BetaView& m, int k, const X* x, long ldx, long xcs, Y*
 template <class LT, class V, class X, class A, class Y>
 void batch_rows_impl(int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs, int ctas,
                      cudaStream_t s) {
-    dispatch_rkc<LT, false>(r, kc, [&](auto RC, auto KCC) {
+    dispatch_rkc<LT>(r, kc, [&](auto RC, auto KCC) {
         constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_, false>(), rows::MM_HB, rows::MM_VB>::SMEM;
+        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), rows::MM_HB, rows::MM_VB>::SMEM;
         auto kern = k_spmm_rows_batch<LT, R_, KC_, V, X, A, Y>;
         set_smem(kern, SMEM);
         int per_sm = 0;
@@ -345,8 +311,8 @@ void batch_rows_impl(int r, int kc, const BatchMat* mats, const BatchJob* jobs, 
 
 }  // namespace
 
-int spmm_rows_kc(int vs, int r, int k, bool seg) {
-    const int lanes = seg ? seg_lanes(r) : ((vs == 16 && r == 8) ? 16 : 8);
+int spmm_rows_kc(int vs, int r, int k) {
+    const int lanes = (vs == 16 && r == 8) ? 16 : 8;
     const int kmax = mm_kc_limit(vs, r, lanes);
     int kc = 1;
     while (kc * 2 <= k && kc * 2 <= kmax) kc *= 2;

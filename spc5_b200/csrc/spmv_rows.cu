@@ -12,8 +12,7 @@
 // columns; otherwise lane q owns the columns q + L k of every sub-row.
 // Either way a lane holds r * VS / L accumulators in registers, a block
 // costs it one header decode and predicated multiply-adds, and the row sums
-// need at most log2(L) shuffles per block-row.  The sorted plan (plan.cu)
-// also runs this kernel on segments of block-rows too large to stage.
+// need at most log2(L) shuffles per block-row.
 //
 // Arithmetic (bit-identical to the reference kernels core_SPC5_{r}rVc_Spmv_*,
 // src/spc5.hpp:2309-2715): accumulator c of sub-row s receives
@@ -113,19 +112,11 @@ __device__ __forceinline__ void rows_subrow_blocks(const uint32_t* hw, long h_al
     }
 }
 
-// SEG: the block-rows are segments of long block-rows (the length-sorted
-// plan's largest ones), laid out so that chunk k of warp w holds segment k of
-// each of the block-rows w * 32 / L + slot (nseg of them, ng = min(32 / L,
-// nseg - w * 32 / L) in warp w): a lane keeps its accumulators from chunk to
-// chunk and adds its row sum to y after the last one (perm[w * 32 / L +
-// slot] is the block-row of y).  The FMA chain of every (sub-row, column) is
-// the block-row's own, in block order.
-template <class LT, int R, class V, class X, class A, class Y, int L, bool SEG>
+template <class LT, int R, class V, class X, class A, class Y, int L>
 __global__ void __launch_bounds__(ROWS_THREADS)
     k_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
            const V* __restrict__ values, const int* __restrict__ valptr,
-           const int* __restrict__ wstart, int nwarps, const int* __restrict__ perm, int nseg,
-           const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
+           const int* __restrict__ wstart, int nwarps, const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
     // a launch gated on a device word (see BetaView::run_if)
     if (run_if && __ldg(run_if) != run_if_value) return;
     using G = RowGeo<LT, R, V, L>;
@@ -139,9 +130,7 @@ __global__ void __launch_bounds__(ROWS_THREADS)
     // R * CPL = VS accumulators, held per column: acc[c / CPL][c % CPL]).  A
     // column lane pays the offset arithmetic of every mask field per block; a
     // sub-row lane finds its values contiguous, after the masks below its own.
-    // Not in the segmented part at r = 4, where the column lanes' x loads of 8
-    // blocks per step hide the gathers better (measured on B200).
-    constexpr bool TRANS = R >= 2 && L == R && !(R == 4 && SEG);
+    constexpr bool TRANS = R >= 2 && L == R;
     extern __shared__ __align__(16) unsigned char smem[];
 
     const int lane = threadIdx.x & 31;
@@ -216,7 +205,7 @@ __global__ void __launch_bounds__(ROWS_THREADS)
         const int b_stop = mine ? b_mine : 0;
         int v = (mine ? (slot > 0 ? v_prev : ch.v_lo) : 0) - ch.v_al;  // buffer index of the block's values
 
-        if constexpr (!SEG) zero();
+        zero();
         if constexpr (TRANS) {
             rows_subrow_blocks<LT, R, V, X, A, CPL>(hw, ch.h_al, vbuf, x, q, b, b_stop, v, pol_x, acc);
         } else {
@@ -267,19 +256,11 @@ __global__ void __launch_bounds__(ROWS_THREADS)
                 b += U;
             }
         }
-        if constexpr (!SEG) flush(mine, mine ? (perm ? __ldg(perm + ch.r0 + slot) : ch.r0 + slot) : 0);
+        flush(mine, ch.r0 + slot);
     };
 
     unsigned char* wbuf = smem + wi * G::BUF_BYTES;
-    if constexpr (SEG) {
-        if (warp >= nwarps) return;  // warp-uniform
-        const int ng = min(SPW, nseg - warp * SPW);
-        zero();
-        rows::walk<LT, R, V, L>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute, ng);
-        flush(slot < ng, slot < ng ? __ldg(perm + warp * SPW + slot) : 0);
-    } else {
-        rows::walk<LT, R, V, L>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
-    }
+    rows::walk<LT, R, V, L>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
 }
 
 template <class K>
@@ -287,51 +268,25 @@ void set_smem(K kernel, int bytes) {
     SPC5_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
-// Calls f(std::integral_constant<int, R>, std::integral_constant<int, L>)
-// for a supported (r, lanes-per-block-row) pair: L >= r, L in {1, 2, 4, 8}.
+// Calls f(std::integral_constant<int, R>{}) for r in {1, 2, 4, 8}.
 template <class F>
-void dispatch_rl(int r, int lanes, F&& f) {
-    using std::integral_constant;
-    const int L = lanes ? lanes : r;
+void dispatch_r(int r, F&& f) {
     switch (r) {
-        case 1:
-            switch (L) {
-                case 1: f(integral_constant<int, 1>{}, integral_constant<int, 1>{}); return;
-                case 2: f(integral_constant<int, 1>{}, integral_constant<int, 2>{}); return;
-                case 4: f(integral_constant<int, 1>{}, integral_constant<int, 4>{}); return;
-                case 8: f(integral_constant<int, 1>{}, integral_constant<int, 8>{}); return;
-            }
-            break;
-        case 2:
-            switch (L) {
-                case 2: f(integral_constant<int, 2>{}, integral_constant<int, 2>{}); return;
-                case 4: f(integral_constant<int, 2>{}, integral_constant<int, 4>{}); return;
-                case 8: f(integral_constant<int, 2>{}, integral_constant<int, 8>{}); return;
-            }
-            break;
-        case 4:
-            switch (L) {
-                case 4: f(integral_constant<int, 4>{}, integral_constant<int, 4>{}); return;
-                case 8: f(integral_constant<int, 4>{}, integral_constant<int, 8>{}); return;
-            }
-            break;
-        case 8:
-            if (L == 8) {
-                f(integral_constant<int, 8>{}, integral_constant<int, 8>{});
-                return;
-            }
-            break;
+        case 1: f(std::integral_constant<int, 1>{}); return;
+        case 2: f(std::integral_constant<int, 2>{}); return;
+        case 4: f(std::integral_constant<int, 4>{}); return;
+        case 8: f(std::integral_constant<int, 8>{}); return;
     }
-    throw Error(SPC5CUDA_ERR_FORMAT, "r must be 1, 2, 4 or 8 and lanes >= r");
+    throw Error(SPC5CUDA_ERR_FORMAT, "r must be 1, 2, 4 or 8");
 }
 
 template <class LT, class V, class X, class A, class Y>
-int rows_occupancy(int r, int lanes) {
+int rows_occupancy(int r) {
     int n = 0;
-    dispatch_rl(r, lanes, [&](auto RC, auto LC) {
-        constexpr int R_ = decltype(RC)::value, L_ = decltype(LC)::value;
-        using G = RowGeo<LT, R_, V, L_>;
-        auto kern = k_rows<LT, R_, V, X, A, Y, L_, false>;
+    dispatch_r(r, [&](auto RC) {
+        constexpr int R_ = decltype(RC)::value;
+        using G = RowGeo<LT, R_, V, R_>;
+        auto kern = k_rows<LT, R_, V, X, A, Y, R_>;
         set_smem(kern, G::SMEM);
         SPC5_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, ROWS_THREADS, G::SMEM));
     });
@@ -343,13 +298,13 @@ void launch_rows_impl(const BetaView& m, const X* x, Y* y, cudaStream_t s) {
     if (m.nbr <= 0 || m.nwarps <= 0) return;
     const V* vals = static_cast<const V*>(m.values);
     const int ctas = (m.nwarps + ROWS_WARPS - 1) / ROWS_WARPS;
-    dispatch_rl(m.r, m.lanes, [&](auto RC, auto LC) {
-        constexpr int R_ = decltype(RC)::value, L_ = decltype(LC)::value;
-        using G = RowGeo<LT, R_, V, L_>;
-        auto kern = m.nseg > 0 ? k_rows<LT, R_, V, X, A, Y, L_, true> : k_rows<LT, R_, V, X, A, Y, L_, false>;
+    dispatch_r(m.r, [&](auto RC) {
+        constexpr int R_ = decltype(RC)::value;
+        using G = RowGeo<LT, R_, V, R_>;
+        auto kern = k_rows<LT, R_, V, X, A, Y, R_>;
         set_smem(kern, G::SMEM);
-        kern<<<ctas, ROWS_THREADS, G::SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart,
-                                                 m.nwarps, m.perm, m.nseg, x, y, m.run_if, m.run_if_value);
+        kern<<<ctas, ROWS_THREADS, G::SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart, m.nwarps, x, y,
+                                                 m.run_if, m.run_if_value);
     });
     SPC5_CUDA(cudaGetLastError());
 }
@@ -383,14 +338,13 @@ __global__ void k_blockrow_max(int nbr, const int* __restrict__ brptr, const int
 
 }  // namespace
 
-int rows_warps(int vt, int r, int lanes) {
-    // cached per (device, value type, r, lanes): the drop-in symbols ask on
-    // every call
+int rows_warps(int vt, int r) {
+    // cached per (device, value type, r): the drop-in symbols ask on every call
     static std::mutex mu;
-    static std::map<std::tuple<int, int, int, int>, int> cache;
+    static std::map<std::tuple<int, int, int>, int> cache;
     int dev = 0;
     SPC5_CUDA(cudaGetDevice(&dev));
-    const auto key = std::make_tuple(dev, vt, r, lanes);
+    const auto key = std::make_tuple(dev, vt, r);
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
@@ -398,12 +352,12 @@ int rows_warps(int vt, int r, int lanes) {
     }
     int per_sm;
     if (vt == SPC5CUDA_F64) {
-        per_sm = rows_occupancy<double, double, double, double, double>(r, lanes);
+        per_sm = rows_occupancy<double, double, double, double, double>(r);
     } else if (vt == SPC5CUDA_F32_V8) {
-        per_sm = rows_occupancy<double, float, float, double, double>(r, lanes);
+        per_sm = rows_occupancy<double, float, float, double, double>(r);
     } else {
-        per_sm = std::min(rows_occupancy<float, float, float, float, float>(r, lanes),
-                          rows_occupancy<float, float, float, double, double>(r, lanes));
+        per_sm = std::min(rows_occupancy<float, float, float, float, float>(r),
+                          rows_occupancy<float, float, float, double, double>(r));
     }
     const int n = sm_count() * per_sm * ROWS_WARPS;
     std::lock_guard<std::mutex> lk(mu);
@@ -423,19 +377,6 @@ bool rows_fit(int vt, int r, int max_blocks, int max_values) {
     const long vneed = (long(max_values) + 2 * (16 / vbytes)) * vbytes;
     return hneed <= ROWS_HB && vneed <= ROWS_VB;
 }
-
-long rows_lane_units(int vt, int r, int nblocks, int nvalues) {
-    // a block-row of this size fits `lanes` lanes' share of a chunk (32 / lanes
-    // block-rows per chunk) when the result is <= lanes * ROWS_UNIT
-    const long stride = 4 + r * (vt == SPC5CUDA_F32 ? 2 : 1);
-    const long vbytes = vt == SPC5CUDA_F64 ? 8 : 4;
-    return std::max(long(nblocks) * stride * (ROWS_VB - 32), long(nvalues) * vbytes * (ROWS_HB - 32));
-}
-
-long rows_unit() { return long(ROWS_HB - 32) * long(ROWS_VB - 32) / 32; }
-
-int rows_hb() { return ROWS_HB; }
-int rows_vb() { return ROWS_VB; }
 
 void blockrow_max(int nbr, const int* brptr, const int* valptr, int* max_blocks, int* max_values,
                   cudaStream_t s) {
