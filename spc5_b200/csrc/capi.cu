@@ -105,10 +105,10 @@ namespace {
 // core_SPC5_{r}rVc_Spmv_{double,float} over device arrays without a handle.
 // Per call, all on the stream and without a host round trip: the value
 // offsets of the block-rows (one pass over the headers), the largest
-// block-row, the per-group and per-warp splits; then the row kernel and the
-// group kernel are both enqueued, gated on a device word: the row kernel runs
-// when every block-row fits its staging buffers, the group kernel otherwise.
-// Both give the reference's bits.
+// block-row, the per-group and per-warp splits; then the two instantiations of
+// the row kernel and the group kernel are enqueued, gated on a device word: a
+// row kernel runs when every block-row fits its staging buffers, the group
+// kernel otherwise.  All give the reference's bits.
 template <class T>
 void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* headers,
                const T* values, const T* x, T* y, cudaStream_t s) {
@@ -122,11 +122,11 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     constexpr int vt = sizeof(T) == 8 ? SPC5CUDA_F64 : SPC5CUDA_F32;
     const int nbr = div_up(nbRows, r);
     const int ngroups = spmv_groups(vs_of(vt), r);
-    const int nwarps = rows_warps(vt, r);
+    const int nwarps = rows_warps(vt, r, true);  // one wave of either instantiation, about
     PoolBuf valptr(sizeof(int) * size_t(nbr + 1), s);
     PoolBuf gstart(sizeof(int) * size_t(ngroups + 1), s);
     PoolBuf wstart(sizeof(int) * size_t(nwarps + 1), s);
-    PoolBuf work(sizeof(int) * 4, s);
+    PoolBuf work(sizeof(int) * 5, s);
     {
         PoolBuf tmp(sizeof(int) * size_t(scan_tmp_ints(nbr) + 1), s);
         launch_blockrow_value_counts(mask_bytes_of(vt), r, nbr, rowsSizes, headers, valptr.as<int>(), s);
@@ -134,7 +134,7 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     }
     launch_partition(nbr, rowsSizes, ngroups, gstart.as<int>(), s);
     launch_partition(nbr, rowsSizes, nwarps, wstart.as<int>(), s);
-    launch_rows_fit_flag(vt, r, nbr, rowsSizes, valptr.as<int>(), work.as<int>(), s);
+    launch_rows_fit_flag(vt, r, nbr, rowsSizes, valptr.as<int>(), headers, work.as<int>(), s);
     BetaView v;
     v.r = r;
     v.nrows = int(nbRows);
@@ -149,14 +149,14 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     BetaView vr = v;
     vr.wstart = wstart.as<int>();
     vr.nwarps = nwarps;
+    BetaView vn = vr;
+    vn.narrow = true;
     v.run_if_value = 0;   // group kernel: some block-row does not fit
     vr.run_if_value = 1;  // row kernel: every block-row fits
-    if constexpr (sizeof(T) == 8) {
-        launch_spmv_f64(vr, x, y, s);
-        launch_spmv_f64(v, x, y, s);
-    } else {
-        launch_spmv_f32(vr, x, y, s);
-        launch_spmv_f32(v, x, y, s);
+    vn.run_if_value = 2;  // and the masks are narrow
+    for (const BetaView& one : {vn, vr, v}) {
+        if constexpr (sizeof(T) == 8) launch_spmv_f64(one, x, y, s);
+        else launch_spmv_f32(one, x, y, s);
     }
 }
 

@@ -199,6 +199,7 @@ struct spc5cuda_mat {
     int nwarps = 0;
     int kernel = SPC5CUDA_KERNEL_AUTO;  // SpMV kernel choice (spc5cuda_mat_set_kernel)
     bool rows_ok = false;               // every block-row fits the row kernel's buffers
+    bool rows_narrow = false;           // its narrow instantiation suits the masks
     std::unique_ptr<spc5cuda::SortedPlan> plan;  // rows sorted by size (irregular matrices)
     // the plan holds the only copy of the values (set when the plan is built
     // and serves SpMV): the reference order is rebuilt on demand
@@ -219,6 +220,7 @@ struct spc5cuda_mat {
         if (use_rows()) {
             v.wstart = wstart.as<int>();
             v.nwarps = nwarps;
+            v.narrow = rows_narrow;
         }
         return v;
     }
@@ -277,11 +279,12 @@ struct spc5cuda_mat {
         ngroups = spc5cuda::spmv_groups(vs, r);
         gstart.alloc(sizeof(int) * size_t(ngroups + 1));
         spc5cuda::launch_partition(nbr(), brptr.as<int>(), ngroups, gstart.as<int>(), s);
-        int max_blocks = 0, max_values = 0;
-        spc5cuda::blockrow_max(nbr(), brptr.as<int>(), valptr.as<int>(), &max_blocks, &max_values, s);
-        rows_ok = spc5cuda::rows_fit(value_type, r, max_blocks, max_values);
+        const spc5cuda::RowStats stats = spc5cuda::row_stats(value_type, r, nbr(), brptr.as<int>(), valptr.as<int>(),
+                                                             headers.as<uint8_t>(), s);
+        rows_ok = stats.fits;
+        rows_narrow = stats.narrow;
         if (rows_ok) {
-            nwarps = spc5cuda::rows_warps(value_type, r);
+            nwarps = spc5cuda::rows_warps(value_type, r, rows_narrow);
             wstart.alloc(sizeof(int) * size_t(nwarps + 1));
             spc5cuda::launch_partition(nbr(), brptr.as<int>(), nwarps, wstart.as<int>(), s);
         } else {

@@ -51,6 +51,7 @@ struct BetaView {
     // starts of the per-warp ranges; null selects the group kernel
     const int* wstart = nullptr;
     int nwarps = 0;
+    bool narrow = false;  // row kernel: the instantiation for narrow masks
     // when set, the launch does its work only if *run_if == run_if_value (a
     // device word written by an earlier kernel on the same stream)
     const int* run_if = nullptr;
@@ -68,18 +69,22 @@ void launch_spmv_f64(const BetaView& m, const double* x, double* y, cudaStream_t
 
 // Thread-per-sub-row kernel (spmv_rows.cu): resident warps on this device,
 // whether block-rows of at most max_blocks blocks / max_values values fit its
-// staging buffers, and the largest block-row of a converted matrix
-// (synchronises s).
+// staging buffers, and what a converted matrix asks of it (synchronises s).
 // (vt: the handle's value type, SPC5CUDA_F64 / F32 / F32_V8.)
-int rows_warps(int vt, int r);
+int rows_warps(int vt, int r, bool narrow);
 bool rows_fit(int vt, int r, int max_blocks, int max_values);
-void blockrow_max(int nbr, const int* brptr, const int* valptr, int* max_blocks, int* max_values,
-                  cudaStream_t s);
-// The same test on the device, without a host round trip: work[0] = 1 when
-// every block-row fits the row kernel's buffers, else 0 (work holds 3 ints;
-// work[1], work[2] receive the largest block and value counts).
-void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* valptr, int* work,
-                          cudaStream_t s);
+struct RowStats {
+    bool fits;    // every block-row fits the row kernel's buffers
+    bool narrow;  // most blocks' sub-row masks span few columns
+};
+// (headers may be null: narrow is not asked for.)
+RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
+                   cudaStream_t s);
+// The same on the device, without a host round trip: work[0] = 0 when some
+// block-row does not fit the row kernel's buffers, else 1 for its wide, 2 for
+// its narrow instantiation (work holds 5 ints).
+void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
+                          int* work, cudaStream_t s);
 void launch_rows_f64(const BetaView& m, const double* x, double* y, cudaStream_t s);
 void launch_rows_f32(const BetaView& m, const float* x, float* y, cudaStream_t s);
 void launch_rows_mixed(const BetaView& m, const float* x, double* y, cudaStream_t s);

@@ -4,15 +4,24 @@
 // matrices).
 //
 // Work split: warp w owns the contiguous block-rows [wstart[w], wstart[w+1])
-// (balanced by blocks).  It walks them in chunks of at most 32 / L
-// block-rows (L lanes per block-row, L >= r): the chunk's packed headers and
-// values are copied into the warp's shared-memory buffer with coalesced
-// 16-byte cp.async (rows_stage.cuh), then the L lanes of each block-row work
-// on it from shared memory.  With L = r >= 2 lane s owns sub-row s and all VS
-// columns; otherwise lane q owns the columns q + L k of every sub-row.
-// Either way a lane holds r * VS / L accumulators in registers, a block
-// costs it one header decode and predicated multiply-adds, and the row sums
-// need at most log2(L) shuffles per block-row.
+// (balanced by blocks).  It walks them in chunks of at most 32 / r block-rows:
+// the chunk's packed headers and values are copied into the warp's
+// shared-memory buffer with coalesced 16-byte cp.async (rows_stage.cuh), then
+// lane s of a block-row works on its sub-row s from shared memory, all VS
+// columns, with VS accumulators in registers.
+//
+// Two instantiations.  The wide one tests every column of a block.  The narrow
+// one is for matrices whose sub-row masks span at most NS columns (stencils:
+// 3 of 8 or 16): a lane's masks keep to one window of NS columns from its
+// block-row's first column on (at r = 8, VS = 8 modulo VS), so it tests NS
+// columns per block; a step with a wider mask in some lane runs block by block
+// over all columns.  The window starts at accumulator 0: the row's
+// accumulators are rotated, which the reduce tree (it pairs accumulators VS/2,
+// ..., 1 apart, and addition commutes) does not see.  The wide kernel spent 165
+// warp instructions per step of 8 block-rows on the 27-point stencil and was
+// bound by issue.  Measured on B200, wide before / narrow now: stencil 160^3
+// r = 4 FP64 278 / 201 us, 127^3 r = 8 FP64 234 / 181 us, 140^3 r = 1 FP64 201 /
+// 145 us, 140^3 r = 2 mixed 182 / 135 us, 101^3 r = 1 f32 93 / 46 us.
 //
 // Arithmetic (bit-identical to the reference kernels core_SPC5_{r}rVc_Spmv_*,
 // src/spc5.hpp:2309-2715): accumulator c of sub-row s receives
@@ -44,100 +53,229 @@ constexpr int ROWS_THREADS = rows::THREADS;
 constexpr int ROWS_WARPS = rows::WARPS;
 constexpr int ROWS_CTAS_PER_SM = 16;
 
-template <class LT, int R, class V, int L>
-using RowGeo = rows::Geo<LT, R, V, L>;
+// The narrow kernel runs when at least 7 of 8 sampled blocks are narrow.
+__host__ __device__ inline bool rows_narrow(int narrow, int sampled) {
+    return sampled > 0 && long(narrow) * 8 >= long(sampled) * 7;
+}
 
-// The blocks [b, b_stop) of a staged chunk for the lane that owns sub-row q
-// of its block-row and all VS columns (acc[c / CPL][c % CPL] is column c).
-// Its values in a block are contiguous: after those of the sub-rows below q,
-// one per set bit of its mask, in column order.
-template <class LT, int R, class V, class X, class A, int CPL>
-__device__ __forceinline__ void rows_subrow_blocks(const uint32_t* hw, long h_al, const V* vbuf,
-                                                   const X* __restrict__ x, int q, int& b, int b_stop, int& v,
-                                                   uint64_t pol_x, A (&acc)[R][CPL]) {
-    constexpr int VS = Layout<LT>::VS, MB = Layout<LT>::MASK_BYTES;
-    constexpr int MW = Header<LT, R>::MASK_WORDS, STRIDE = Header<LT, R>::STRIDE;
-    constexpr int FPW = 4 / MB, BITS = 8 * MB;
-    constexpr uint32_t FMASK = MB == 1 ? 0xFFu : 0xFFFFu;
-    // blocks per step (their x loads are issued together): 4 at r = 8 for
-    // double blocks, else 16 / VS (measured on B200: 4 blocks lifted the
-    // power-law r = 8 SpMV by 10% and slowed r = 2 by 9%)
-    constexpr int UT = (R == 8 && VS == 8) ? 4 : (16 / VS > 1 ? 16 / VS : 1);
-    const int wq = q / FPW;
-    const unsigned sh = unsigned(q % FPW) * BITS;
-    uint32_t lowmask[MW];  // mask bits of the sub-rows below q
+// The lane of sub-row q of its block-row: where it stands in the staged chunk.
+struct SubRow {
+    int n;      // blocks left
+    int hoff;   // byte offset of the next block's header in the staged headers
+    int v;      // index of its first value in the staged values
+};
+
+// One staged block as sub-row q sees it: first column, own mask, its values'
+// place (from the block's first value) and the block's value count.
+template <class LT, int R>
+struct Block {
+    static constexpr int MW = Header<LT, R>::MASK_WORDS;
+    int col;
+    uint32_t mw[MW], m;
+};
+
+template <class LT, int R>
+struct SubRowOf {
+    static constexpr int MB = Layout<LT>::MASK_BYTES, MW = Header<LT, R>::MASK_WORDS;
+    static constexpr int FPW = 4 / MB, BITS = 8 * MB;
+    int wq;            // mask word of sub-row q
+    unsigned sh;       // its field in that word
+    uint32_t low[MW];  // mask bits of the sub-rows below q
+    __device__ __forceinline__ explicit SubRowOf(int q) : wq(q / FPW), sh(unsigned(q % FPW) * BITS) {
 #pragma unroll
-    for (int w = 0; w < MW; ++w) lowmask[w] = w < wq ? 0xFFFFFFFFu : (w == wq ? (1u << sh) - 1u : 0u);
-    while (__any_sync(FULL, b < b_stop)) {
-        int col[UT];
-        uint32_t mw[UT][MW];
-        uint32_t mi[UT];
+        for (int w = 0; w < MW; ++w) low[w] = w < wq ? 0xFFFFFFFFu : (w == wq ? (1u << sh) - 1u : 0u);
+    }
+    // the block at header offset off, empty when !ok
+    __device__ __forceinline__ void load(const uint32_t* hw, int off, bool ok, Block<LT, R>& b) const {
+        constexpr uint32_t FMASK = MB == 1 ? 0xFFu : 0xFFFFu;
+        b.col = 0;
 #pragma unroll
-        for (int u = 0; u < UT; ++u) {
-            col[u] = 0;
+        for (int w = 0; w < MW; ++w) b.mw[w] = 0u;
+        if (ok) b.col = rows::decode_staged<LT, R>(hw, off, b.mw);
+        uint32_t word = b.mw[0];
 #pragma unroll
-            for (int w = 0; w < MW; ++w) mw[u][w] = 0u;
-            if (b + u < b_stop) col[u] = rows::decode_staged<LT, R>(hw, long(b + u) * STRIDE - h_al, mw[u]);
-            uint32_t word = mw[u][0];
+        for (int w = 1; w < MW; ++w) word = w == wq ? b.mw[w] : word;
+        b.m = R == 1 ? word : (word >> sh) & FMASK;
+    }
+    __device__ __forceinline__ int before(const Block<LT, R>& b) const {
+        int n = 0;
+        if constexpr (R > 1) {
 #pragma unroll
-            for (int w = 1; w < MW; ++w) word = w == wq ? mw[u][w] : word;
-            mi[u] = (word >> sh) & FMASK;
+            for (int w = 0; w < MW; ++w) n += __popc(b.mw[w] & low[w]);
         }
+        return n;
+    }
+    static __device__ __forceinline__ int values(const Block<LT, R>& b) {
+        int n = 0;
+#pragma unroll
+        for (int w = 0; w < MW; ++w) n += __popc(b.mw[w]);
+        return n;
+    }
+};
+
+// All VS columns of every block, UT blocks per step (their x loads are issued
+// together).
+template <class LT, int R, class V, class X, class A, int UT>
+__device__ __forceinline__ void wide_blocks(const uint32_t* hw, const V* vbuf, const X* __restrict__ x, int q,
+                                            SubRow at, uint64_t pol_x, A (&acc)[Layout<LT>::VS]) {
+    constexpr int VS = Layout<LT>::VS, STRIDE = Header<LT, R>::STRIDE;
+    const SubRowOf<LT, R> me(q);
+    const int steps = (__reduce_max_sync(FULL, at.n) + UT - 1) / UT;
+#pragma unroll 1
+    for (int step = 0; step < steps; ++step) {
+        Block<LT, R> b[UT];
         X xk[UT][VS];
 #pragma unroll
-        for (int u = 0; u < UT; ++u) {
-            const X* xp = x + col[u];
+        for (int u = 0; u < UT; ++u) me.load(hw, at.hoff + u * STRIDE, u < at.n, b[u]);
 #pragma unroll
-            for (int c = 0; c < VS; ++c) xk[u][c] = ((mi[u] >> c) & 1u) ? ld_x(xp + c, pol_x) : X(0);
+        for (int u = 0; u < UT; ++u) {
+            const X* xp = x + b[u].col;
+#pragma unroll
+            for (int c = 0; c < VS; ++c) xk[u][c] = b[u].m & (1u << c) ? ld_x(xp + c, pol_x) : X(0);
         }
 #pragma unroll
         for (int u = 0; u < UT; ++u) {
-            int pre = 0, tot = 0;
-#pragma unroll
-            for (int w = 0; w < MW; ++w) {
-                pre += __popc(mw[u][w] & lowmask[w]);
-                tot += __popc(mw[u][w]);
-            }
-            int idx = v + pre;
+            const V* vp = vbuf + at.v + me.before(b[u]);
 #pragma unroll
             for (int c = 0; c < VS; ++c) {
-                if ((mi[u] >> c) & 1u) {
-                    acc[c / CPL][c % CPL] = fma(A(vbuf[idx]), A(xk[u][c]), acc[c / CPL][c % CPL]);
-                    ++idx;
+                if (b[u].m & (1u << c)) {
+                    acc[c] = fma(A(*vp), A(xk[u][c]), acc[c]);
+                    ++vp;
                 }
             }
-            v += tot;
+            at.v += me.values(b[u]);
         }
-        b += UT;
+        at.n -= UT;
+        at.hoff += UT * STRIDE;
     }
 }
 
-template <class LT, int R, class V, class X, class A, class Y, int L>
-__global__ void __launch_bounds__(ROWS_THREADS)
+// CTAs per SM asked of the compiler: 6 (80 registers; the narrow kernel at 7 and
+// 72 ran the r = 8 stencil 127^3 7% slower), 5 where 16 double
+// accumulators (the float layout in mixed precision), 4 where 4 wide blocks of
+// double x per step need more.
+template <class LT, int R, class X, class A>
+constexpr int row_ctas(bool narrow) {
+    constexpr int VS = Layout<LT>::VS;
+    return VS * sizeof(A) > 64 ? 5 : (!narrow && R == 8 && VS == 8 && sizeof(X) == 8 ? 4 : 6);
+}
+
+// A window of NS columns, from the first column of the sub-row's first
+// non-empty mask on: accumulator a is column (rho + a) mod VS.
+constexpr int NS = 3;
+template <class LT, int R, class V, class X, class A>
+__device__ __forceinline__ void narrow_blocks(const uint32_t* hw, const V* vbuf, const X* __restrict__ x, int q,
+                                              SubRow at, uint64_t pol_x, A (&acc)[Layout<LT>::VS]) {
+    constexpr int VS = Layout<LT>::VS, STRIDE = Header<LT, R>::STRIDE;
+    constexpr uint32_t VSMASK = (1u << VS) - 1u;
+    constexpr bool WRAP = R == VS;  // the window may run over the last column into the next block
+    // blocks per step: a 27-point stencil's row has 9 at r <= 4 (2 / 3 / 4 blocks
+    // measured on B200: 160^3 r = 4 253 / 240 / 249 us, 101^3 r = 1 f32 52 / 48 / 50)
+    constexpr int UT = 3;
+    const SubRowOf<LT, R> me(q);
+    int rho = 0;
+    // the window's columns (bit[a]), the columns outside it (all of them until
+    // the lane has met its first mask; at r = 1 a block starts at its first
+    // column), and x there
+    uint32_t bit[NS], outside;
+    const X* xw[NS];
+    auto window = [&]() {
+        outside = VSMASK;
+#pragma unroll
+        for (int a = 0; a < NS; ++a) {
+            const int c = WRAP ? (rho + a) & (VS - 1) : rho + a;
+            bit[a] = 1u << c;
+            outside &= ~bit[a];
+            xw[a] = x + c;
+        }
+    };
+    window();
+    if constexpr (R > 1) outside = VSMASK;
+    const int steps = (__reduce_max_sync(FULL, at.n) + UT - 1) / UT;
+#pragma unroll 1
+    for (int step = 0; step < steps; ++step) {
+        Block<LT, R> b[UT];
+        uint32_t some = 0u;
+#pragma unroll
+        for (int u = 0; u < UT; ++u) {
+            me.load(hw, at.hoff + u * STRIDE, u < at.n, b[u]);
+            some |= b[u].m;
+        }
+        if (__any_sync(FULL, (some & outside) != 0u)) {
+            bool wide = true;
+            if constexpr (R > 1) {
+                if (some && outside == VSMASK) {  // the lane's first masks
+                    uint32_t first = b[UT - 1].m;
+#pragma unroll
+                    for (int u = UT - 2; u >= 0; --u) first = b[u].m ? b[u].m : first;
+                    rho = __ffs(first) - 1;
+                    window();
+                }
+                wide = __any_sync(FULL, (some & outside) != 0u);
+            }
+            if (wide) {
+                // a wide mask: the accumulators back at their columns, and the
+                // rest of the chunk over all columns
+                if constexpr (R > 1) {
+#pragma unroll
+                    for (int d = 1; d < VS; d <<= 1) {
+                        A t[VS];
+#pragma unroll
+                        for (int c = 0; c < VS; ++c) t[c] = acc[c];
+#pragma unroll
+                        for (int c = 0; c < VS; ++c) acc[c] = (rho & d) ? t[(c - d) & (VS - 1)] : t[c];
+                    }
+                }
+                wide_blocks<LT, R, V, X, A, 1>(hw, vbuf, x, q, at, pol_x, acc);
+                return;
+            }
+        }
+        X xk[UT][NS];
+#pragma unroll
+        for (int u = 0; u < UT; ++u) {
+#pragma unroll
+            for (int a = 0; a < NS; ++a) {
+                xk[u][a] = b[u].m & bit[a] ? ld_x(xw[a] + b[u].col, pol_x) : X(0);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UT; ++u) {
+            // values are in column order: those of the window's columns
+            // past the last one (its wrapped part) come first
+            const V* v0 = vbuf + at.v + me.before(b[u]);
+            const V* vp = v0;
+            if constexpr (WRAP) vp += __popc(b[u].m & ((1u << rho) - 1u));
+#pragma unroll
+            for (int a = 0; a < NS; ++a) {
+                if (WRAP && a > 0 && rho == VS - a) vp = v0;
+                if (b[u].m & bit[a]) {
+                    acc[a] = fma(A(*vp), A(xk[u][a]), acc[a]);
+                    ++vp;
+                }
+            }
+            at.v += me.values(b[u]);
+        }
+        at.n -= UT;
+        at.hoff += UT * STRIDE;
+    }
+}
+
+template <class LT, int R, class V, class X, class A, class Y, bool NARROW>
+__global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, X, A>(NARROW))
     k_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
-           const V* __restrict__ values, const int* __restrict__ valptr,
-           const int* __restrict__ wstart, int nwarps, const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
+           const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart, int nwarps,
+           const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
     // a launch gated on a device word (see BetaView::run_if)
     if (run_if && __ldg(run_if) != run_if_value) return;
-    using G = RowGeo<LT, R, V, L>;
-    constexpr int VS = G::VS, MB = G::MB, MW = G::MW, SPW = G::SPW;
-    constexpr int FPW = 4 / MB;  // mask fields per 32-bit word
-    constexpr int BITS = 8 * MB;
-    constexpr uint32_t FMASK = MB == 1 ? 0xFFu : 0xFFFFu;
+    using G = rows::Geo<LT, R, V, R>;
+    constexpr int VS = G::VS;
     constexpr bool Y_ATOMIC = sizeof(Y) == 8;  // red.add.f64 is y + s rounded once
-    constexpr int CPL = VS / L;  // columns per lane
-    // L = r >= 2: lane q owns sub-row q for all VS columns instead (the same
-    // R * CPL = VS accumulators, held per column: acc[c / CPL][c % CPL]).  A
-    // column lane pays the offset arithmetic of every mask field per block; a
-    // sub-row lane finds its values contiguous, after the masks below its own.
-    constexpr bool TRANS = R >= 2 && L == R;
     extern __shared__ __align__(16) unsigned char smem[];
-
     const int lane = threadIdx.x & 31;
     const int wi = threadIdx.x >> 5;
     const int warp = blockIdx.x * ROWS_WARPS + wi;
-    const int slot = lane / L;  // block-row of the chunk
-    const int q = lane % L;     // column class: this lane owns columns c = q + L k
+    const int slot = lane / R;  // block-row of the chunk
+    const int q = lane % R;     // sub-row
 
     int r_begin = 0, r_stop = 0;
     if (warp < nwarps) {
@@ -146,121 +284,39 @@ __global__ void __launch_bounds__(ROWS_THREADS)
     }
     const uint64_t pol_x = l2_evict_last_policy();
 
-    A acc[R][CPL];
-    auto zero = [&]() {
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-            for (int k = 0; k < CPL; ++k) acc[i][k] = A(0);
-    };
-    // ---- row sums: the _mm512_reduce_add tree (distance VS/2, ..., 1).
-    // Levels of distance >= L pair columns of the same class inside the
-    // lane; the last log2(L) levels pair the lanes of the block-row.  Then
-    // y[brow * R + q] += sum of sub-row q (warp-uniform call).
-    auto flush = [&](bool mine, int brow) {
-        A res = A(0);
-        if constexpr (TRANS) {
-            // the whole tree inside the lane: column c in acc[c / CPL][c % CPL]
-#pragma unroll
-            for (int d = VS / 2; d >= 1; d >>= 1) {
-#pragma unroll
-                for (int c = 0; c < d; ++c)
-                    acc[c / CPL][c % CPL] = acc[c / CPL][c % CPL] + acc[(c + d) / CPL][(c + d) % CPL];
-            }
-            res = acc[0][0];
-        } else {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-#pragma unroll
-                for (int d = CPL / 2; d >= 1; d >>= 1) {
-#pragma unroll
-                    for (int k = 0; k < d; ++k) acc[i][k] = acc[i][k] + acc[i][k + d];
-                }
-                A sum = acc[i][0];
-#pragma unroll
-                for (int d = L / 2; d >= 1; d >>= 1) sum = sum + __shfl_xor_sync(FULL, sum, d);
-                if (i == q) res = sum;
-            }
-        }
-        if (mine && q < R) {
-            const long yrow = long(brow) * R + q;
-            if (yrow < nrows) {
-                if constexpr (Y_ATOMIC) atomicAdd(y + yrow, Y(res));
-                else y[yrow] = y[yrow] + Y(res);
-            }
-        }
-    };
-
     // ---- the blocks of block-row r0 + slot of a staged chunk
     auto compute = [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
-        // blocks per step: the x loads of all of them are issued before the
-        // FMAs, which still run block by block (the chain order is kept)
-        constexpr int U = (16 / CPL) < 1 ? 1 : ((16 / CPL) > 8 ? 8 : 16 / CPL);
         const int src = slot > 0 ? slot - 1 : 0;
         const int b_prev = __shfl_sync(FULL, ch.b_hi, src);
         const int v_prev = __shfl_sync(FULL, ch.v_hi, src);
         const int b_mine = __shfl_sync(FULL, ch.b_hi, slot);
         const bool mine = slot < ch.nrow;
-        int b = mine ? (slot > 0 ? b_prev : ch.b_lo) : 0;
-        const int b_stop = mine ? b_mine : 0;
-        int v = (mine ? (slot > 0 ? v_prev : ch.v_lo) : 0) - ch.v_al;  // buffer index of the block's values
+        const int b = slot > 0 ? b_prev : ch.b_lo;
+        SubRow at;
+        at.n = mine ? b_mine - b : 0;
+        at.hoff = int(long(b) * G::STRIDE - ch.h_al);
+        at.v = (slot > 0 ? v_prev : ch.v_lo) - ch.v_al;
 
-        zero();
-        if constexpr (TRANS) {
-            rows_subrow_blocks<LT, R, V, X, A, CPL>(hw, ch.h_al, vbuf, x, q, b, b_stop, v, pol_x, acc);
-        } else {
-            while (__any_sync(FULL, b < b_stop)) {
-                int col[U];
-                uint32_t mw[U][MW];
+        A acc[VS];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    col[u] = 0;
+        for (int c = 0; c < VS; ++c) acc[c] = A(0);
+        if constexpr (NARROW) narrow_blocks<LT, R, V, X, A>(hw, vbuf, x, q, at, pol_x, acc);
+        else wide_blocks<LT, R, V, X, A, (R == 8 && VS == 8) ? 4 : (16 / VS > 1 ? 16 / VS : 1)>(hw, vbuf, x, q, at, pol_x, acc);
+        // ---- row sum: the _mm512_reduce_add tree (distance VS/2, ..., 1)
 #pragma unroll
-                    for (int w = 0; w < MW; ++w) mw[u][w] = 0u;
-                    if (b + u < b_stop) col[u] = rows::decode_staged<LT, R>(hw, long(b + u) * G::STRIDE - ch.h_al, mw[u]);
-                }
-                // x of this lane's columns where some sub-row has a value
-                X xk[U][CPL];
+        for (int d = VS / 2; d >= 1; d >>= 1) {
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint32_t uni = rows::mask_union<LT, R>(mw[u]);
-                    const X* xp = x + col[u] + q;
-#pragma unroll
-                    for (int k = 0; k < CPL; ++k)
-                        xk[u][k] = ((uni >> (q + L * k)) & 1u) ? ld_x(xp + L * k, pol_x) : X(0);
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    uint32_t pre[MW];
-                    const int tot = rows::subrow_prefix<LT, R>(mw[u], pre);
-#pragma unroll
-                    for (int k = 0; k < CPL; ++k) {
-                        const int c = q + L * k;
-                        const uint32_t below = (1u << c) - 1u;
-#pragma unroll
-                        for (int w = 0; w < MW; ++w) {
-                            // field i: buffer offset of sub-row i's value in column c
-                            const uint32_t off = rows::column_offsets<LT, R>(mw[u][w], pre[w], below);
-#pragma unroll
-                            for (int f = 0; f < FPW; ++f) {
-                                const int i = w * FPW + f;
-                                if (i < R && ((mw[u][w] >> (f * BITS + c)) & 1u)) {
-                                    const int idx = v + int((off >> (f * BITS)) & FMASK);
-                                    acc[i][k] = fma(A(vbuf[idx]), A(xk[u][k]), acc[i][k]);
-                                }
-                            }
-                        }
-                    }
-                    v += tot;
-                }
-                b += U;
-            }
+            for (int c = 0; c < d; ++c) acc[c] = acc[c] + acc[c + d];
         }
-        flush(mine, ch.r0 + slot);
+        const long yrow = long(ch.r0 + slot) * R + q;
+        if (mine && yrow < nrows) {
+            if constexpr (Y_ATOMIC) atomicAdd(y + yrow, Y(acc[0]));
+            else y[yrow] = y[yrow] + Y(acc[0]);
+        }
     };
 
     unsigned char* wbuf = smem + wi * G::BUF_BYTES;
-    rows::walk<LT, R, V, L>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
+    rows::walk<LT, R, V, R>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
 }
 
 template <class K>
@@ -281,12 +337,12 @@ void dispatch_r(int r, F&& f) {
 }
 
 template <class LT, class V, class X, class A, class Y>
-int rows_occupancy(int r) {
+int rows_occupancy(int r, bool narrow) {
     int n = 0;
     dispatch_r(r, [&](auto RC) {
         constexpr int R_ = decltype(RC)::value;
-        using G = RowGeo<LT, R_, V, R_>;
-        auto kern = k_rows<LT, R_, V, X, A, Y, R_>;
+        using G = rows::Geo<LT, R_, V, R_>;
+        auto kern = narrow ? k_rows<LT, R_, V, X, A, Y, true> : k_rows<LT, R_, V, X, A, Y, false>;
         set_smem(kern, G::SMEM);
         SPC5_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, ROWS_THREADS, G::SMEM));
     });
@@ -300,8 +356,8 @@ void launch_rows_impl(const BetaView& m, const X* x, Y* y, cudaStream_t s) {
     const int ctas = (m.nwarps + ROWS_WARPS - 1) / ROWS_WARPS;
     dispatch_r(m.r, [&](auto RC) {
         constexpr int R_ = decltype(RC)::value;
-        using G = RowGeo<LT, R_, V, R_>;
-        auto kern = k_rows<LT, R_, V, X, A, Y, R_>;
+        using G = rows::Geo<LT, R_, V, R_>;
+        auto kern = m.narrow ? k_rows<LT, R_, V, X, A, Y, true> : k_rows<LT, R_, V, X, A, Y, false>;
         set_smem(kern, G::SMEM);
         kern<<<ctas, ROWS_THREADS, G::SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart, m.nwarps, x, y,
                                                  m.run_if, m.run_if_value);
@@ -309,13 +365,51 @@ void launch_rows_impl(const BetaView& m, const X* x, Y* y, cudaStream_t s) {
     SPC5_CUDA(cudaGetLastError());
 }
 
-// flag[0] = 1 when a block-row of maxes[0] blocks and maxes[1] values fits
-// the staging buffers (the test of rows_fit, on the device), else 0.
-__global__ void k_fit_flag(const int* __restrict__ maxes, int stride, int vbytes, int hb, int vb,
+// flag[0] = 0 when a block-row of stats[0] blocks and stats[1] values does not
+// fit the staging buffers (the test of rows_fit, on the device), else 1 for the
+// wide row kernel, 2 for the narrow one (stats[2] of stats[3] sampled blocks).
+__global__ void k_fit_flag(const int* __restrict__ stats, int stride, int vbytes, int hb, int vb,
                            int* __restrict__ flag) {
-    const long hneed = long(maxes[0]) * stride + 32;
-    const long vneed = (long(maxes[1]) + 2 * (16 / vbytes)) * vbytes;
-    flag[0] = (hneed <= hb && vneed <= vb) ? 1 : 0;
+    const long hneed = long(stats[0]) * stride + 32;
+    const long vneed = (long(stats[1]) + 2 * (16 / vbytes)) * vbytes;
+    flag[0] = (hneed <= hb && vneed <= vb) ? (rows_narrow(stats[2], stats[3]) ? 2 : 1) : 0;
+}
+
+// Of at most SAMPLED blocks spread over the matrix: how many, and how many
+// whose every sub-row mask spans at most NS columns.  At r = VS the narrow
+// kernel's steps of 3 blocks pay for themselves only on block-rows of several
+// steps (measured on B200, FP64, wide / narrow us: 27-point stencil 127^3, 18
+// blocks per block-row, 234 / 181; 5-point Poisson 900^2, 4 blocks, 29.4 / 31.5).
+constexpr int SAMPLED = 1 << 15;
+template <class LT, int R>
+__global__ void __launch_bounds__(256) k_narrow_sample(int nbr, const int* __restrict__ brptr,
+                                                       const uint8_t* __restrict__ headers, int* __restrict__ out) {
+    const long nblocks = brptr[nbr];
+    const long step = max(1L, nblocks / SAMPLED);
+    const long i = (long(blockIdx.x) * blockDim.x + threadIdx.x) * step;
+    const bool in = i < nblocks && i / step < SAMPLED;
+    bool narrow = in && (R < Layout<LT>::VS || nblocks >= 6L * nbr);
+    if (in) {
+        uint32_t mw[Header<LT, R>::MASK_WORDS];
+        load_header<LT, R>(headers, i, mw);
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+            const uint32_t m = mask_of<LT, R>(mw, s);
+            narrow = narrow && (m == 0u || (m >> (__ffs(m) - 1)) < (1u << NS));
+        }
+    }
+    const unsigned n = __popc(__ballot_sync(FULL, narrow)), all = __popc(__ballot_sync(FULL, in));
+    if ((threadIdx.x & 31) == 0 && all) {
+        atomicAdd(out, int(n));
+        atomicAdd(out + 1, int(all));
+    }
+}
+
+template <class LT>
+void narrow_sample(int r, int nbr, const int* brptr, const uint8_t* headers, int* out, cudaStream_t s) {
+    dispatch_r(r, [&](auto RC) {
+        k_narrow_sample<LT, decltype(RC)::value><<<SAMPLED / 256, 256, 0, s>>>(nbr, brptr, headers, out);
+    });
 }
 
 // Largest block count and value count of any block-row.
@@ -338,13 +432,13 @@ __global__ void k_blockrow_max(int nbr, const int* __restrict__ brptr, const int
 
 }  // namespace
 
-int rows_warps(int vt, int r) {
-    // cached per (device, value type, r): the drop-in symbols ask on every call
+int rows_warps(int vt, int r, bool narrow) {
+    // cached per (device, value type, r, instantiation): the drop-in symbols ask on every call
     static std::mutex mu;
-    static std::map<std::tuple<int, int, int>, int> cache;
+    static std::map<std::tuple<int, int, int, bool>, int> cache;
     int dev = 0;
     SPC5_CUDA(cudaGetDevice(&dev));
-    const auto key = std::make_tuple(dev, vt, r);
+    const auto key = std::make_tuple(dev, vt, r, narrow);
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
@@ -352,12 +446,12 @@ int rows_warps(int vt, int r) {
     }
     int per_sm;
     if (vt == SPC5CUDA_F64) {
-        per_sm = rows_occupancy<double, double, double, double, double>(r);
+        per_sm = rows_occupancy<double, double, double, double, double>(r, narrow);
     } else if (vt == SPC5CUDA_F32_V8) {
-        per_sm = rows_occupancy<double, float, float, double, double>(r);
+        per_sm = rows_occupancy<double, float, float, double, double>(r, narrow);
     } else {
-        per_sm = std::min(rows_occupancy<float, float, float, float, float>(r),
-                          rows_occupancy<float, float, float, double, double>(r));
+        per_sm = std::min(rows_occupancy<float, float, float, float, float>(r, narrow),
+                          rows_occupancy<float, float, float, double, double>(r, narrow));
     }
     const int n = sm_count() * per_sm * ROWS_WARPS;
     std::lock_guard<std::mutex> lk(mu);
@@ -378,34 +472,41 @@ bool rows_fit(int vt, int r, int max_blocks, int max_values) {
     return hneed <= ROWS_HB && vneed <= ROWS_VB;
 }
 
-void blockrow_max(int nbr, const int* brptr, const int* valptr, int* max_blocks, int* max_values,
-                  cudaStream_t s) {
-    int* d = nullptr;
-    SPC5_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d), 2 * sizeof(int), s));
-    SPC5_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof(int), s));
-    if (nbr > 0) {
-        const int threads = 256;
-        const int blocks = std::max(1, std::min(div_up(nbr, threads), sm_count() * 4));
-        k_blockrow_max<<<blocks, threads, 0, s>>>(nbr, brptr, valptr, d);
-        SPC5_CUDA(cudaGetLastError());
+namespace {
+
+// stats[0], stats[1]: the largest block and value counts of any block-row;
+// stats[2], stats[3]: narrow and all sampled blocks (headers may be null: none).
+void enqueue_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers, int* stats,
+                   cudaStream_t s) {
+    SPC5_CUDA(cudaMemsetAsync(stats, 0, 4 * sizeof(int), s));
+    if (nbr <= 0) return;
+    const int threads = 256;
+    const int blocks = std::max(1, std::min(div_up(nbr, threads), sm_count() * 4));
+    k_blockrow_max<<<blocks, threads, 0, s>>>(nbr, brptr, valptr, stats);
+    if (headers) {
+        if (vt == SPC5CUDA_F32) narrow_sample<float>(r, nbr, brptr, headers, stats + 2, s);
+        else narrow_sample<double>(r, nbr, brptr, headers, stats + 2, s);
     }
-    int h[2] = {0, 0};
-    SPC5_CUDA(cudaMemcpyAsync(h, d, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    SPC5_CUDA(cudaFreeAsync(d, s));
-    SPC5_CUDA(cudaStreamSynchronize(s));
-    *max_blocks = h[0];
-    *max_values = h[1];
+    SPC5_CUDA(cudaGetLastError());
 }
 
-void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* valptr, int* work,
-                          cudaStream_t s) {
-    SPC5_CUDA(cudaMemsetAsync(work, 0, 3 * sizeof(int), s));
-    if (nbr > 0) {
-        const int threads = 256;
-        const int blocks = std::max(1, std::min(div_up(nbr, threads), sm_count() * 4));
-        k_blockrow_max<<<blocks, threads, 0, s>>>(nbr, brptr, valptr, work + 1);
-        SPC5_CUDA(cudaGetLastError());
-    }
+}  // namespace
+
+RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
+                   cudaStream_t s) {
+    int* d = nullptr;
+    SPC5_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d), 4 * sizeof(int), s));
+    enqueue_stats(vt, r, nbr, brptr, valptr, headers, d, s);
+    int h[4] = {0, 0, 0, 0};
+    SPC5_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
+    SPC5_CUDA(cudaFreeAsync(d, s));
+    SPC5_CUDA(cudaStreamSynchronize(s));
+    return RowStats{rows_fit(vt, r, h[0], h[1]), rows_narrow(h[2], h[3])};
+}
+
+void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
+                          int* work, cudaStream_t s) {
+    enqueue_stats(vt, r, nbr, brptr, valptr, headers, work + 1, s);
     const int stride = 4 + r * (vt == SPC5CUDA_F32 ? 2 : 1);
     const int vbytes = vt == SPC5CUDA_F64 ? 8 : 4;
     k_fit_flag<<<1, 1, 0, s>>>(work + 1, stride, vbytes, ROWS_HB, ROWS_VB, work);

@@ -61,9 +61,7 @@ int plan_regime(const spc5cuda_mat* m, int r, const int* brptr, cudaStream_t s) 
     const int nbr = div_up(m->nrows, r);
     DevBuf valptr(sizeof(int) * size_t(nbr + 1), s);
     launch_valptr_from_csr(r, m->nrows, m->rowptr.as<int>(), valptr.as<int>(), s);
-    int max_blocks = 0, max_values = 0;
-    blockrow_max(nbr, brptr, valptr.as<int>(), &max_blocks, &max_values, s);
-    return rows_fit(m->value_type, r, max_blocks, max_values) ? 0 : 1;
+    return row_stats(m->value_type, r, nbr, brptr, valptr.as<int>(), nullptr, s).fits ? 0 : 1;
 }
 
 // A trial run: a temporary handle holding a copy of the CSR matrix is
