@@ -150,14 +150,18 @@ __device__ __forceinline__ void wide_blocks(const uint32_t* hw, const V* vbuf, c
     }
 }
 
-// CTAs per SM asked of the compiler: 6 (80 registers; the narrow kernel at 7 and
-// 72 ran the r = 8 stencil 127^3 7% slower), 5 where 16 double
-// accumulators (the float layout in mixed precision), 4 where 4 wide blocks of
-// double x per step need more.
+// CTAs per SM asked of the compiler.  Wide: 6 (80 registers), 4 where 4 blocks of
+// double x per step need more.  Narrow: 7 (72 registers: the 5-point Poisson
+// 512^2 at r = 2 then takes two chunks per warp instead of three, 8.3 against
+// 9.4 us on the device; 160^3 at r = 4 197 against 203 us), 6 at r = 8, whose
+// window wraps (127^3: 7 was 7% slower).  5 where 16 double accumulators (the
+// float layout in mixed precision) need the registers.
 template <class LT, int R, class X, class A>
 constexpr int row_ctas(bool narrow) {
     constexpr int VS = Layout<LT>::VS;
-    return VS * sizeof(A) > 64 ? 5 : (!narrow && R == 8 && VS == 8 && sizeof(X) == 8 ? 4 : 6);
+    if (VS * sizeof(A) > 64) return 5;
+    if (narrow) return R < 8 ? 7 : 6;
+    return R == 8 && VS == 8 && sizeof(X) == 8 ? 4 : 6;
 }
 
 // A window of NS columns, from the first column of the sub-row's first
