@@ -2,12 +2,15 @@
 // sides, in one CUDA graph.
 //
 // Every matrix is cut into jobs of about kJobBlocks blocks along block-row
-// boundaries; each pass of kc right-hand sides (kc a power of two, at most
-// the register budget of its r) is a separate job.  Jobs are grouped by
+// boundaries (128 / 256 / 512 / 1024 / 2048 blocks measured on B200 on 64 banded
+// matrices: 1360 / 1180 / 1220 / 1470 / 2210 us; larger jobs leave the last wave
+// to few warps); each pass of kc right-hand sides is a separate job.  Jobs are
+// grouped by
 // (value kind, r, kc, kernel): one launch of the batched SpMM kernel per class
 // walks its job list with a fixed grid.  Matrices whose every block-row fits
 // the row kernels' staging buffers (and that did not ask for the group
-// kernel) run the staged SpMM, one warp per job; the others the group SpMM.
+// kernel) run the staged SpMM or SpMV, one warp per job; the others the group
+// SpMM.
 // The class launches are captured as parallel branches of one graph, so small
 // matrices of different classes share the GPU; spc5cuda_batch_launch replays
 // the graph.
@@ -22,7 +25,10 @@
 
 namespace spc5cuda {
 namespace {
-constexpr int kJobBlocks = 2048;
+constexpr int kJobBlocks = 256;
+// How a class of jobs runs: the group SpMM, the staged SpMM by lists or by
+// columns, the row SpMV.
+enum How { GROUP, LISTS, COLUMNS, SPMV_WIDE, SPMV_NARROW };
 }  // namespace
 }  // namespace spc5cuda
 
@@ -55,7 +61,7 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
         try {
             std::vector<BatchMat> hm(static_cast<size_t>(n));
             // class (kind, r, kc, staged) -> jobs
-            std::map<std::tuple<int, int, int, bool>, std::vector<BatchJob>> classes;
+            std::map<std::tuple<int, int, int, int>, std::vector<BatchJob>> classes;
             for (int i = 0; i < n; ++i) {
                 const spc5cuda_mat* m = mats[i];
                 require(m && m->r != 0, SPC5CUDA_ERR_FORMAT, "batch matrices must be converted");
@@ -80,7 +86,7 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
                 b.xcs = 1;
                 b.ycs = 1;
                 b.nrows = m->nrows;
-                b.pad = 0;
+                b.k = k[i];
                 if (m->nrows == 0 || k[i] == 0) continue;
                 // block-row cuts every ~kJobBlocks blocks
                 const int nbr = m->nbr();
@@ -99,9 +105,21 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
                 int kofs = 0;
                 while (kofs < k[i]) {
                     const bool staged = m->spmm_view().wstart != nullptr;
-                    const int kc = staged ? spmm_rows_kc(vs_of(m->value_type), m->r, k[i] - kofs)
-                                          : batch_kc(m->r, k[i] - kofs);
-                    auto& list = classes[std::make_tuple(kind, m->r, kc, staged)];
+                    const int left = k[i] - kofs, vs = vs_of(m->value_type);
+                    int kc, how = GROUP;
+                    if (!staged) {
+                        kc = batch_kc(m->r, left);
+                    } else if (k[i] == 1 && ldx[i] == 1 && ldy[i] == 1) {
+                        kc = 1;
+                        how = m->rows_narrow ? SPMV_NARROW : SPMV_WIDE;
+                    } else if (spmm_columns(vs, m->r, m->full_blocks(), left)) {
+                        kc = spmm_cols_kc(vs, m->r, left);
+                        how = COLUMNS;
+                    } else {
+                        kc = spmm_rows_kc(left);
+                        how = LISTS;
+                    }
+                    auto& list = classes[std::make_tuple(kind, m->r, kc, how)];
                     for (auto& pc : pieces) list.push_back(BatchJob{i, pc.first, pc.second, kofs});
                     kofs += kc;
                 }
@@ -139,16 +157,19 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
             const int sms = sm_count();
             for (auto& kv : classes) {
                 const int kind = std::get<0>(kv.first), r = std::get<1>(kv.first), kc = std::get<2>(kv.first);
-                const bool staged = std::get<3>(kv.first);
+                const int how = std::get<3>(kv.first);
                 const int vs = (kind == 0 || kind == 3) ? 8 : 16;
                 const int njobs = int(kv.second.size());
                 const int ctas = std::max(1, std::min(div_up(long(njobs) * vs, 128), sms * 16));
                 SPC5_CUDA(cudaStreamWaitEvent(br[c], fork, 0));
-                if (staged)
-                    launch_batch_rows(kind, r, kc, bt->mats.as<BatchMat>(), bt->jobs[c].as<BatchJob>(), njobs,
-                                      br[c]);
+                const BatchMat* mats = bt->mats.as<BatchMat>();
+                const BatchJob* list = bt->jobs[c].as<BatchJob>();
+                if (how == COLUMNS)
+                    launch_batch_cols(kind, r, kc, mats, list, njobs, br[c]);
+                else if (how != GROUP)
+                    launch_batch_rows(kind, r, kc, how == SPMV_NARROW, mats, list, njobs, br[c]);
                 else
-                    launch_batch(kind, r, kc, bt->mats.as<BatchMat>(), bt->jobs[c].as<BatchJob>(), njobs,
+                    launch_batch(kind, r, kc, mats, list, njobs,
                                  ctas, br[c]);
                 SPC5_CUDA(cudaEventRecord(done[c], br[c]));
                 SPC5_CUDA(cudaStreamWaitEvent(cap, done[c], 0));

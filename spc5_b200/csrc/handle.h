@@ -217,6 +217,7 @@ struct spc5cuda_mat {
         v.valptr = valptr.as<int>();
         v.gstart = gstart.as<int>();
         v.ngroups = ngroups;
+        v.full_blocks = full_blocks();
         if (use_rows()) {
             v.wstart = wstart.as<int>();
             v.nwarps = nwarps;
@@ -224,6 +225,7 @@ struct spc5cuda_mat {
         }
         return v;
     }
+    bool full_blocks() const { return nnz >= 2L * r * nblocks; }
     // The view of the SpMM kernels: the per-warp ranges of the staged kernel
     // whenever every block-row fits its buffers, unless the group kernel was
     // requested.
@@ -234,6 +236,7 @@ struct spc5cuda_mat {
         if (rows_ok && nwarps > 0 && kernel != SPC5CUDA_KERNEL_GROUPS) {
             v.wstart = wstart.as<int>();
             v.nwarps = nwarps;
+            v.narrow = rows_narrow;
         }
         return v;
     }

@@ -52,6 +52,7 @@ struct BetaView {
     const int* wstart = nullptr;
     int nwarps = 0;
     bool narrow = false;  // row kernel: the instantiation for narrow masks
+    bool full_blocks = false;  // at least two values per sub-row and block on average
     // when set, the launch does its work only if *run_if == run_if_value (a
     // device word written by an earlier kernel on the same stream)
     const int* run_if = nullptr;
@@ -85,6 +86,8 @@ RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, 
 // its narrow instantiation (work holds 5 ints).
 void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
                           int* work, cudaStream_t s);
+// The row SpMV of a kind (below).
+void launch_rows_kind(int kind, const BetaView& m, const void* x, void* y, cudaStream_t s);
 void launch_rows_f64(const BetaView& m, const double* x, double* y, cudaStream_t s);
 void launch_rows_f32(const BetaView& m, const float* x, float* y, cudaStream_t s);
 void launch_rows_mixed(const BetaView& m, const float* x, double* y, cudaStream_t s);
@@ -131,7 +134,7 @@ struct BatchMat {
     long xcs;       // stride between right-hand sides (1: row-major)
     long ycs;
     int nrows;
-    int pad;
+    int k;          // right-hand sides
 };
 struct BatchJob {
     int mat;      // index into the BatchMat array
@@ -145,18 +148,29 @@ int batch_kc(int r, int k);
 // 8-column layout (F32_V8 matrices)
 void launch_batch(int kind, int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs,
                   int ctas, cudaStream_t s);
-// Right-hand sides per pass of the staged SpMM for VS columns per block,
-// rows-per-block r and k right-hand sides left.
-int spmm_rows_kc(int vs, int r, int k);
-// Most right-hand sides per pass of the staged SpMM with `lanes` lanes per
-// block-row: r x (vs / lanes columns per lane) x kc accumulators stay at
-// most 32, kc at most 16.
+// Right-hand sides per pass of the staged SpMM with k left: 2, 4, 8 or 16 (the
+// last pass may have fewer).
+int spmm_rows_kc(int k);
+// Whether a pass with k right-hand sides left runs with a lane per column
+// (spmm_cols.cu) instead: few right-hand sides on blocks of many rows.
+// full_blocks: at least two values per sub-row and block on average.
+bool spmm_columns(int vs, int r, bool full_blocks, int k);
+// Right-hand sides of such a pass (a power of two), and its launch for a kind.
+int spmm_cols_kc(int vs, int r, int k);
+void launch_spmm_cols(int kind, const BetaView& m, int kc, const void* x, long ldx, long xcs, void* y, long ldy,
+                      long ycs, cudaStream_t s);
+void launch_batch_cols(int kind, int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs,
+                       cudaStream_t s);
+// Most right-hand sides of such a pass: r x (vs / lanes columns per lane) x kc
+// accumulators stay at most 32, kc at most 8.
 constexpr int mm_kc_limit(int vs, int r, int lanes) {
-    return 32 / (r * (vs / lanes)) > 16 ? 16 : 32 / (r * (vs / lanes));
+    return 32 / (r * (vs / lanes)) > 8 ? 8 : 32 / (r * (vs / lanes));
 }
 // The same for matrices whose block-rows fit the row kernels' buffers
-// (spmm_rows.cu): one warp per job at a time; kc from spmm_rows_kc.
-void launch_batch_rows(int kind, int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs,
+// (spmm_rows.cu): one warp per job at a time; kc from spmm_rows_kc, or 1 for
+// jobs of one right-hand side with contiguous x and y, which run the row SpMV's
+// wide or narrow form.
+void launch_batch_rows(int kind, int r, int kc, bool narrow, const BatchMat* mats, const BatchJob* jobs, int njobs,
                        cudaStream_t s);
 
 }  // namespace spc5cuda

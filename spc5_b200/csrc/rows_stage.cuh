@@ -6,9 +6,7 @@
 // and values are copied into the warp's shared-memory buffer with coalesced
 // 16-byte cp.async (matrix data streamed with an L2 evict-first policy, the
 // data after the chunk prefetched into L2), then the caller's compute step
-// reads every block of the chunk from shared memory.  The helpers below
-// decode a staged header and locate the value of (sub-row, column) in a block
-// -- the expand-load offsets of the reference vector kernels.
+// reads every block of the chunk from shared memory (decode_staged below).
 #pragma once
 
 #include <algorithm>
@@ -26,11 +24,6 @@ constexpr int WARPS = THREADS / 32;
 // small for the stencil).
 constexpr int HB = 1536;  // header bytes of one warp's staging buffer
 constexpr int VB = 6144;  // value bytes of one warp's staging buffer
-// The multi-RHS kernels are limited by registers to 4 CTAs per SM, so they
-// stage larger chunks (every block-row that fits the buffers above fits
-// these).
-constexpr int MM_HB = 2048;
-constexpr int MM_VB = 8192;
 constexpr unsigned FULL = 0xffffffffu;
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
@@ -187,60 +180,6 @@ __device__ __forceinline__ int decode_staged(const uint32_t* hw, long off,
         const unsigned sh = unsigned(off & 3) * 8u;
         mw[0] = __funnelshift_r(lw[1], lw[2], sh) & ((1u << (8 * H::MASK_BYTES_TOTAL)) - 1u);
         return int(__funnelshift_r(lw[0], lw[1], sh));
-    }
-}
-
-// Union of the sub-row masks (bit c: some sub-row has a value in column c).
-template <class LT, int R>
-__device__ __forceinline__ uint32_t mask_union(const uint32_t (&mw)[Header<LT, R>::MASK_WORDS]) {
-    uint32_t uni = 0;
-#pragma unroll
-    for (int w = 0; w < Header<LT, R>::MASK_WORDS; ++w) uni |= mw[w];
-    if constexpr (Layout<LT>::MASK_BYTES == 1) return (uni | (uni >> 16)) | ((uni | (uni >> 16)) >> 8);
-    else return uni | (uni >> 16);
-}
-
-// Per mask word: exclusive prefix of the sub-row value counts, one field per
-// sub-row (pre); returns the block's value count.
-template <class LT, int R>
-__device__ __forceinline__ int subrow_prefix(const uint32_t (&mw)[Header<LT, R>::MASK_WORDS],
-                                             uint32_t (&pre)[Header<LT, R>::MASK_WORDS]) {
-    uint32_t carry = 0;
-#pragma unroll
-    for (int w = 0; w < Header<LT, R>::MASK_WORDS; ++w) {
-        uint32_t cnt = mw[w] - ((mw[w] >> 1) & 0x55555555u);
-        cnt = (cnt & 0x33333333u) + ((cnt >> 2) & 0x33333333u);
-        cnt = (cnt + (cnt >> 4)) & 0x0F0F0F0Fu;
-        if constexpr (Layout<LT>::MASK_BYTES == 1) {
-            pre[w] = cnt * 0x01010100u + carry * 0x01010101u;
-            carry += (cnt * 0x01010101u) >> 24;
-        } else {
-            cnt = (cnt + (cnt >> 8)) & 0x001F001Fu;
-            pre[w] = (cnt << 16) + carry * 0x00010001u;
-            carry += (cnt + (cnt >> 16)) & 0xFFFFu;
-        }
-    }
-    return int(carry);
-}
-
-// Field f of the result: offset, from the block's first value, of the value
-// of sub-row (w * fields per word + f) in the column whose lower columns are
-// `below`, for mask word w with prefix pre_w.
-template <class LT, int R>
-__device__ __forceinline__ uint32_t column_offsets(uint32_t mw_w, uint32_t pre_w, uint32_t below) {
-    if constexpr (R == 1) {
-        return uint32_t(__popc(mw_w & below));
-    } else if constexpr (Layout<LT>::MASK_BYTES == 1) {
-        uint32_t t = mw_w & (below * 0x01010101u);
-        t = t - ((t >> 1) & 0x55555555u);
-        t = (t & 0x33333333u) + ((t >> 2) & 0x33333333u);
-        return pre_w + ((t + (t >> 4)) & 0x0F0F0F0Fu);
-    } else {
-        uint32_t t = mw_w & (below * 0x00010001u);
-        t = t - ((t >> 1) & 0x55555555u);
-        t = (t & 0x33333333u) + ((t >> 2) & 0x33333333u);
-        t = (t + (t >> 4)) & 0x0F0F0F0Fu;
-        return pre_w + ((t + (t >> 8)) & 0x001F001Fu);
     }
 }
 

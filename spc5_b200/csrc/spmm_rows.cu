@@ -1,28 +1,36 @@
 // spmm_rows.cu -- staged multi-RHS SpMM, Y += A X, for matrices whose every
 // block-row fits the row kernels' staging buffers (rows_stage.cuh).
 //
-// A warp walks its block-rows in chunks staged into shared memory; each
-// block-row of a chunk is served by L lanes (mm_lanes), and lane q owns the
-// columns q + L k of every block for all R sub-rows and KC right-hand sides
-// (R * VS / L * KC accumulators, at most 32).  Per block a lane decodes the
-// staged header once, loads its KC x values per column (only where some
-// sub-row has a value in that column: blocks at the right edge may reach
-// past the last column), reads each of its values once from shared memory
-// and issues KC multiply-adds with it.
+// A warp walks its block-rows in chunks of 32 sub-rows staged into shared
+// memory.  One lane per sub-row first lists the sub-row's values in chain order
+// -- column class 0 of its blocks in block order, then class 1, ... -- each
+// with its x index and its place in the staged values (two walks over the
+// staged headers: count, place).  Then KC / 2 lanes serve one sub-row, two
+// neighbouring right-hand sides each, 64 / KC sub-rows at a time: per value a
+// lane reads the list entry and the value (the same for the sub-row's lanes),
+// loads its two x (16 or 8 bytes at once where X allows) and does two
+// multiply-adds; where a chain ends it leaves the results in shared memory.
+//
+// What bounds it: instructions.  With a lane per column (before) each lane
+// tested every sub-row's mask per block and issued KC multiply-adds for each,
+// of which a matrix with 1 to 4 values per block uses a tenth: 16 instructions
+// per value and 8 right-hand sides, now 9 to 10.  Measured on B200, before / now
+// (us, FP64): banded n = 200,000, 21 values per row, r = 4, k = 8 140 / 76; r = 1, k
+// = 16 330 / 137; r = 2, k = 4 100 / 57.  Where a lane per column is still the
+// faster one (few right-hand sides on blocks of many rows) it stays:
+// spmm_cols.cu.
 //
 // Arithmetic per right-hand side j is the SpMV's (src/spc5.hpp:2309-2715):
-// accumulator (i, j) of column c receives fma(value, x[col + c][j], acc) for
-// every block in order whose mask i has bit c; the row sum is the
-// _mm512_reduce_add tree over the VS columns (XOR distances VS/2, ..., 1: in
-// the lane, then across the L lanes); then
-// Y[row][j] += sum (one rounding: red.add.f64 for double Y, load-add-store for
-// float Y, exactly as the SpMV kernels).  Column j of the result is therefore
-// bit-identical to an SpMV with column j of X.
+// the chain of (sub-row, column class c) receives fma(value, x[col + c][j],
+// acc) for every block in order whose mask has bit c; the row sum is the
+// _mm512_reduce_add tree over the VS chains (+0 for a class without values);
+// then Y[row][j] += sum.  Column j of the result is therefore bit-identical to
+// an SpMV with column j of X.
 #include <algorithm>
 
 #include "common.cuh"
 #include "kernels.h"
-#include "rows_stage.cuh"
+#include "rows_blocks.cuh"
 
 namespace spc5cuda {
 
@@ -30,213 +38,277 @@ namespace {
 
 using rows::FULL;
 
-// Lanes per block-row of the staged SpMM: one column per lane for double
-// blocks (8 columns); for float blocks (16 columns) two per lane, except at
-// r = 8 where one column per lane keeps four right-hand sides per pass.
-template <class LT, int R>
-constexpr int mm_lanes() {
-    return (Layout<LT>::VS == 16 && R == 8) ? 16 : 8;
+constexpr uint32_t LAST = 1u << 31;  // list entry: the last one of its chain (x indices are below 2^31)
+constexpr int MM_CTAS = 6;  // of 2 warps: the shared memory of 12 to 13 warps per SM
+constexpr int MM_WARPS = 2;  // per CTA: finer steps of shared memory than 4
+constexpr int MM_THREADS = MM_WARPS * 32;
+
+// One warp's shared memory: the staged headers (later the chain results, one
+// column per lane), the staged values, the list.
+template <class LT, int R, class V, class A>
+struct MMGeo {
+    static constexpr int VS = Layout<LT>::VS;
+    static constexpr int CHAIN = VS * 32 * 2 * int(sizeof(A));
+    static constexpr int HB = CHAIN > rows::HB ? CHAIN : rows::HB;
+    static constexpr int VB = rows::VB;
+    static constexpr int VALUES = VB / int(sizeof(V));
+    static constexpr int WARP = HB + VB + VALUES * 8;
+    static constexpr int SMEM = MM_WARPS * WARP;
+};
+
+// Two neighbouring elements as one vector.
+template <class T>
+struct __align__(2 * sizeof(T)) Two {
+    T a, b;
+};
+
+// x of two right-hand sides: one vector load (vec: unit stride, aligned) or two.
+__device__ __forceinline__ Two<double> ld_two(const double* p) {
+    const double2 t = __ldg(reinterpret_cast<const double2*>(p));
+    return {t.x, t.y};
+}
+__device__ __forceinline__ Two<float> ld_two(const float* p) {
+    const float2 t = __ldg(reinterpret_cast<const float2*>(p));
+    return {t.x, t.y};
 }
 
-// Y += A X over block-rows [r_begin, r_stop) of one matrix for right-hand
-// sides [0, KC) of xm / ym (already offset to the pass's first one).
+// A list entry in shared memory (on != 0; predicated without a branch), and LAST
+// set in one.
+__device__ __forceinline__ void st_entry_if(uint32_t saddr, uint32_t x, uint32_t v, uint32_t on) {
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q st.shared.v2.u32 [%0], {%1, %2}; }" ::"r"(saddr), "r"(x),
+                 "r"(v), "r"(on)
+                 : "memory");
+}
+__device__ __forceinline__ void mark_last(uint32_t saddr) {
+    uint32_t x;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(saddr) : "memory");
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(saddr), "r"(x | LAST) : "memory");
+}
+
+// Y += A X over block-rows [r_begin, r_stop) of one matrix for the kc <= KC
+// right-hand sides of xm / ym (already offset to the pass's first one).
 template <class LT, int R, int KC, class V, class X, class A, class Y>
 __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brptr,
                                          const uint8_t* __restrict__ headers, const V* __restrict__ values,
-                                         const int* __restrict__ valptr, int r_begin, int r_stop,
-                                         const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym,
-                                         long ldy, long ycs, unsigned char* wbuf) {
-    constexpr int VS = Layout<LT>::VS;
-    constexpr int L = mm_lanes<LT, R>();  // lanes per block-row
-    constexpr int CPL = VS / L;                // columns per lane: q + L k
-    constexpr int LOGL = L == 16 ? 4 : (L == 8 ? 3 : (L == 4 ? 2 : (L == 2 ? 1 : 0)));
-    using G = rows::Geo<LT, R, V, L, rows::MM_HB, rows::MM_VB>;
-    constexpr int MB = G::MB, MW = G::MW;
-    constexpr int FPW = 4 / MB;  // mask fields per 32-bit word
-    constexpr int BITS = 8 * MB;
-    constexpr uint32_t FMASK = MB == 1 ? 0xFFu : 0xFFFFu;
-    constexpr bool Y_ATOMIC = sizeof(Y) == 8;
-    static_assert(R * CPL * KC <= 32, "accumulators");
-    // blocks per step: their x loads are issued before the FMAs, which still
-    // run block by block (the chain order is kept)
-    constexpr int XW = CPL * KC;  // x values of one block
-    constexpr int U = XW >= 8 ? 1 : 8 / XW;
+                                         const int* __restrict__ valptr, int r_begin, int r_stop, int kc,
+                                         const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym, long ldy,
+                                         long ycs, unsigned char* wbuf) {
+    using G = MMGeo<LT, R, V, A>;
+    constexpr int VS = G::VS, STRIDE = Header<LT, R>::STRIDE;
+    constexpr int LPS = KC / 2;    // lanes per sub-row
+    constexpr int PAR = 32 / LPS;  // sub-rows at a time
+    constexpr int U = 8;           // list entries at a time (4 / 6 / 8: r = 4, k = 8 90 / 82 / 80 us)
     const int lane = threadIdx.x & 31;
-    const int slot = lane / L;  // block-row of the chunk
-    const int q = lane % L;     // this lane's columns: q + L k
-    const uint64_t pol_x = l2_evict_last_policy();
-
-    A acc[R][CPL][KC];
-    auto zero = [&]() {
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-            for (int k = 0; k < CPL; ++k)
-#pragma unroll
-                for (int j = 0; j < KC; ++j) acc[i][k][j] = A(0);
-    };
-
-    // ---- row sums: the _mm512_reduce_add tree (distance VS/2, ..., 1).
-    // Levels of distance >= L pair columns of one lane.  The last log2(L)
-    // levels pair the lanes of the block-row as a reduce-scatter of the
-    // N = R KC sums: at distance d the lane with bit d set keeps the odd
-    // entries and its partner the even ones, each adding the partner's
-    // copy (the same pairs as the tree, so the same bits), until one sum
-    // per entry is left; then the plain butterfly.  Lane q ends with the
-    // entries t L + rev(q) (rev: q's log2(L) bits reversed), or, when
-    // N < L, entry rev(q) mod N in the lanes whose low bits are zero.
-    // Entries are ordered so that one store covers neighbouring
-    // addresses: (i, j) at i KC + j for row-major Y (ycs == 1), at j R + i
-    // otherwise (the R rows of consecutive block-rows are adjacent).  Then
-    // Y[brow R + i][j] += sum (warp-uniform call).
-    auto flush = [&](bool mine, int brow) {
-        constexpr int N = R * KC;
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-#pragma unroll
-            for (int j = 0; j < KC; ++j) {
-#pragma unroll
-                for (int d = CPL / 2; d >= 1; d >>= 1) {
-#pragma unroll
-                    for (int k = 0; k < d; ++k) acc[i][k][j] = acc[i][k][j] + acc[i][k + d][j];
-                }
-            }
-        }
-        const bool row_major = ycs == 1;
-        A sv[N];
-#pragma unroll
-        for (int e = 0; e < N; ++e) sv[e] = row_major ? acc[e / KC][0][e % KC] : acc[e % R][0][e / R];
-#pragma unroll
-        for (int lev = 0; lev < LOGL; ++lev) {
-            const int d = L >> (lev + 1);
-            const int n = N >> lev;  // entries still held
-            const bool hi = (q & d) != 0;
-            if (n >= 2) {
-#pragma unroll
-                for (int t = 0; t < n / 2; ++t) {
-                    const A keep = hi ? sv[2 * t + 1] : sv[2 * t];
-                    const A send = hi ? sv[2 * t] : sv[2 * t + 1];
-                    sv[t] = keep + __shfl_xor_sync(FULL, send, d);
-                }
-            } else {
-                sv[0] = sv[0] + __shfl_xor_sync(FULL, sv[0], d);
-            }
-        }
-        const int rq = LOGL ? int(__brev(unsigned(q)) >> (32 - LOGL)) : 0;
-        constexpr int PER = N >= L ? N / L : 1;
-        const bool writer = mine && (N >= L || (q & (L / N - 1)) == 0);
-        const long row0 = long(brow) * R;
-#pragma unroll
-        for (int t = 0; t < PER; ++t) {
-            const int e = N >= L ? t * L + rq : (rq & (N - 1));
-            const int i = row_major ? e / KC : e % R;
-            const int j = row_major ? e % KC : e / R;
-            const long yrow = row0 + i;
-            if (writer && yrow < nrows) {
-                Y* dst = ym + yrow * ldy + long(j) * ycs;
-                if constexpr (Y_ATOMIC) atomicAdd(dst, Y(sv[t]));
-                else *dst = *dst + Y(sv[t]);
-            }
-        }
-    };
+    const int q = lane % R;
+    const int h = lane / LPS, j = 2 * (lane % LPS);
+    const bool both = j + 1 < kc;
+    const bool vec = xcs == 1 && ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(xm) % (2 * sizeof(X))) == 0;
+    Two<A>* chain = reinterpret_cast<Two<A>*>(wbuf) + lane;
+    // list entry: x index (and LAST), byte offset of the value in the staged values
+    unsigned char* list = wbuf + G::HB + G::VB;
+    const rows::SubRowOf<LT, R> me(q);
+    const X* xj = xm + long(j) * xcs;
+    Y* yj = ym + long(j) * ycs;
 
     auto compute = [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
-        const int src = slot > 0 ? slot - 1 : 0;
-        const int b_prev = __shfl_sync(FULL, ch.b_hi, src);
-        const int v_prev = __shfl_sync(FULL, ch.v_hi, src);
-        const int b_mine = __shfl_sync(FULL, ch.b_hi, slot);
-        const bool mine = slot < ch.nrow;
-        int b = mine ? (slot > 0 ? b_prev : ch.b_lo) : 0;
-        const int b_stop = mine ? b_mine : 0;
-        int v = (mine ? (slot > 0 ? v_prev : ch.v_lo) : 0) - ch.v_al;
-
-        zero();
-        while (__any_sync(FULL, b < b_stop)) {
-            int col[U];
-            uint32_t mw[U][MW];
+        // ---- the sub-row's values per column class
+        const rows::SubRow at = rows::sub_row_at<LT, R>(ch, lane);
+        const unsigned char* vb = reinterpret_cast<const unsigned char*>(vbuf);
+        int cnt[VS];
+        uint32_t chains = 0u;
+        if (__any_sync(FULL, at.n > 255)) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                col[u] = 0;
+            for (int c = 0; c < VS; ++c) cnt[c] = 0;
+            for (int k = 0; k < at.n; ++k) {
+                rows::Block<LT, R> b;
+                me.load(hw, at.hoff + k * STRIDE, true, b);
+                chains |= b.m;
 #pragma unroll
-                for (int w = 0; w < MW; ++w) mw[u][w] = 0u;
-                if (b + u < b_stop) col[u] = rows::decode_staged<LT, R>(hw, long(b + u) * G::STRIDE - ch.h_al, mw[u]);
+                for (int c = 0; c < VS; ++c) cnt[c] += int((b.m >> c) & 1u);
             }
-            // x of this lane's columns where some sub-row has a value
-            X xk[U][CPL][KC];
+        } else {  // four counts to a word
+            uint32_t sum[VS / 4];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const uint32_t uni = rows::mask_union<LT, R>(mw[u]);
+            for (int w = 0; w < VS / 4; ++w) sum[w] = 0u;
+            for (int k = 0; k < at.n; ++k) {
+                rows::Block<LT, R> b;
+                me.load(hw, at.hoff + k * STRIDE, true, b);
+                chains |= b.m;
 #pragma unroll
-                for (int k = 0; k < CPL; ++k) {
-                    const bool has = (uni >> (q + L * k)) & 1u;
-                    const X* xr = xm + long(col[u] + q + L * k) * ldx;
+                for (int w = 0; w < VS / 4; ++w) sum[w] += (((b.m >> (4 * w)) & 0xFu) * 0x00204081u) & 0x01010101u;
+            }
 #pragma unroll
-                    for (int j = 0; j < KC; ++j) xk[u][k][j] = has ? ld_x(xr + long(j) * xcs, pol_x) : X(0);
+            for (int c = 0; c < VS; ++c) cnt[c] = int((sum[c / 4] >> (8 * (c % 4))) & 0xFFu);
+        }
+        int len = 0;
+#pragma unroll
+        for (int c = 0; c < VS; ++c) {
+            const int n = cnt[c];
+            cnt[c] = 8 * len;  // from here on: byte offset of the class's next place
+            len += n;
+        }
+        int first = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(FULL, first, d);
+            if (lane >= d) first += t;
+        }
+        first = 8 * (first - len);
+        // ---- the list
+        {
+            const uint32_t l = uint32_t(__cvta_generic_to_shared(list)) + unsigned(first);
+#pragma unroll
+            for (int c = 0; c < VS; ++c) cnt[c] += int(l);
+            int v = at.v * int(sizeof(V));
+            for (int k = 0; k < at.n; ++k) {
+                rows::Block<LT, R> b;
+                me.load(hw, at.hoff + k * STRIDE, true, b);
+                int w = v + me.before(b) * int(sizeof(V));
+#pragma unroll
+                for (int c = 0; c < VS; ++c) {
+                    const uint32_t on = b.m & (1u << c);
+                    st_entry_if(uint32_t(cnt[c]), uint32_t(b.col + c), uint32_t(w), on);
+                    cnt[c] += on ? 8 : 0;
+                    w += on ? int(sizeof(V)) : 0;
                 }
+                v += me.values(b) * int(sizeof(V));
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                uint32_t pre[MW];
-                const int tot = rows::subrow_prefix<LT, R>(mw[u], pre);
+            for (int c = 0; c < VS; ++c)
+                if (chains & (1u << c)) mark_last(uint32_t(cnt[c]) - 8u);
+        }
+        __syncwarp();  // the list is complete, the headers are done with
+
+        // ---- KC lanes per sub-row
+        const long row0 = long(ch.r0) * R;
+        const int live = int(std::min(long(ch.nrow) * R, nrows - row0));
+        for (int i0 = 0; i0 < live; i0 += PAR) {
+            const int i = i0 + h;
+            const uint2* at0 = reinterpret_cast<const uint2*>(list + __shfl_sync(FULL, first, i));
+            const int n = __shfl_sync(FULL, len, i);
+            const uint32_t mask = __shfl_sync(FULL, chains, i);
+            const bool mine = i < live && j < kc;
+            const int stop = mine ? n : 0;
+            A acc0 = A(0), acc1 = A(0);
+            Two<A>* slot = chain;
+            for (int k = 0; k < stop; k += U) {
+                uint32_t e[U];
+                V v[U];
+                Two<X> x[U];
 #pragma unroll
-                for (int k = 0; k < CPL; ++k) {
-                    const int c = q + L * k;
-                    const uint32_t below = (1u << c) - 1u;
+                for (int u = 0; u < U; ++u) {
+                    e[u] = 0u;
+                    if (k + u < stop) {
+                        const uint2 t = at0[k + u];
+                        e[u] = t.x;
+                        v[u] = *reinterpret_cast<const V*>(vb + t.y);
+                    }
+                }
+                if (vec && both) {
 #pragma unroll
-                    for (int w = 0; w < MW; ++w) {
-                        const uint32_t off = rows::column_offsets<LT, R>(mw[u][w], pre[w], below);
+                    for (int u = 0; u < U; ++u)
+                        if (k + u < stop) x[u] = ld_two(xj + long(e[u] & ~LAST) * ldx);
+                } else {
 #pragma unroll
-                        for (int f = 0; f < FPW; ++f) {
-                            const int i = w * FPW + f;
-                            if (i < R && ((mw[u][w] >> (f * BITS + c)) & 1u)) {
-                                const A e = A(vbuf[v + int((off >> (f * BITS)) & FMASK)]);
-#pragma unroll
-                                for (int j = 0; j < KC; ++j) acc[i][k][j] = fma(e, A(xk[u][k][j]), acc[i][k][j]);
-                            }
+                    for (int u = 0; u < U; ++u) {
+                        if (k + u < stop) {
+                            const X* xp = xj + long(e[u] & ~LAST) * ldx;
+                            x[u].a = __ldg(xp);
+                            x[u].b = both ? __ldg(xp + xcs) : X(0);
                         }
                     }
                 }
-                v += tot;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (k + u < stop) {
+                        acc0 = fma(A(v[u]), A(x[u].a), acc0);
+                        acc1 = fma(A(v[u]), A(x[u].b), acc1);
+                        if (e[u] & LAST) {
+                            *slot = Two<A>{acc0, acc1};
+                            slot += 32;
+                            acc0 = acc1 = A(0);
+                        }
+                    }
+                }
             }
-            b += U;
+            if (mine) {
+                const Two<A>* from = chain;
+                A a0[VS], a1[VS];
+#pragma unroll
+                for (int c = 0; c < VS; ++c) {
+                    Two<A> t{A(0), A(0)};
+                    if (mask & (1u << c)) {
+                        t = *from;
+                        from += 32;
+                    }
+                    a0[c] = t.a;
+                    a1[c] = t.b;
+                }
+                Y* yp = yj + (row0 + i) * ldy;
+                rows::add_to(yp, Y(rows::reduce_tree<A, VS>(a0)));
+                if (both) rows::add_to(yp + ycs, Y(rows::reduce_tree<A, VS>(a1)));
+            }
         }
-        flush(mine, ch.r0 + slot);
     };
-    rows::walk<LT, R, V, L, rows::MM_HB, rows::MM_VB>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
+    rows::walk<LT, R, V, R, G::HB, G::VB>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
 }
 
 // One matrix: warp w owns block-rows [wstart[w], wstart[w + 1]).
 template <class LT, int R, int KC, class V, class X, class A, class Y>
-__global__ void __launch_bounds__(rows::THREADS)
+__global__ void __launch_bounds__(MM_THREADS, MM_CTAS)
     k_spmm_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
                 const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart,
-                int nwarps, const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym, long ldy, long ycs) {
-    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), rows::MM_HB, rows::MM_VB>;
+                int nwarps, int kc, const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym, long ldy,
+                long ycs) {
+    using G = MMGeo<LT, R, V, A>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
-    const int warp = blockIdx.x * rows::WARPS + wi;
+    const int warp = blockIdx.x * MM_WARPS + wi;
     if (warp >= nwarps) return;  // warp-uniform
-    const int r_begin = __ldg(wstart + warp), r_stop = __ldg(wstart + warp + 1);
-    mm_range<LT, R, KC, V, X, A, Y>(nrows, brptr, headers, values, valptr, r_begin, r_stop, xm, ldx, xcs, ym, ldy, ycs,
-                                    smem + wi * G::BUF_BYTES);
+    mm_range<LT, R, KC, V, X, A, Y>(nrows, brptr, headers, values, valptr, __ldg(wstart + warp),
+                                    __ldg(wstart + warp + 1), kc, xm, ldx, xcs, ym, ldy, ycs, smem + wi * G::WARP);
 }
 
 // Batched: warps walk the job list with the grid's warp count as stride; job
-// j is block-rows [r_begin, r_end) of mats[j.mat] for right-hand sides
-// [kofs, kofs + KC).  X and Y of a batch are row-major (xcs = ycs = 1).
+// j is block-rows [r_begin, r_end) of mats[j.mat] for the right-hand sides
+// [kofs, kofs + kc).  X and Y of a batch are row-major (xcs = ycs = 1).
 template <class LT, int R, int KC, class V, class X, class A, class Y>
-__global__ void __launch_bounds__(rows::THREADS)
+__global__ void __launch_bounds__(MM_THREADS, MM_CTAS)
     k_spmm_rows_batch(const BatchMat* __restrict__ mats, const BatchJob* __restrict__ jobs, int njobs) {
-    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), rows::MM_HB, rows::MM_VB>;
+    using G = MMGeo<LT, R, V, A>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
-    const int nw = gridDim.x * rows::WARPS;
-    for (int j = blockIdx.x * rows::WARPS + wi; j < njobs; j += nw) {  // warp-uniform
+    const int nw = gridDim.x * MM_WARPS;
+    for (int j = blockIdx.x * MM_WARPS + wi; j < njobs; j += nw) {  // warp-uniform
         const BatchJob job = jobs[j];
         const BatchMat& m = mats[job.mat];
         mm_range<LT, R, KC, V, X, A, Y>(m.nrows, m.brptr, m.headers, static_cast<const V*>(m.values), m.valptr,
-                                        job.r_begin, job.r_end, static_cast<const X*>(m.x) + job.kofs, m.ldx, 1L,
-                                        static_cast<Y*>(m.y) + job.kofs, m.ldy, 1L, smem + wi * G::BUF_BYTES);
+                                        job.r_begin, job.r_end, m.k - job.kofs, static_cast<const X*>(m.x) + job.kofs,
+                                        m.ldx, 1L, static_cast<Y*>(m.y) + job.kofs, m.ldy, 1L, smem + wi * G::WARP);
+    }
+}
+
+// The jobs of one right-hand side with contiguous x and y: the row SpMV's
+// chunks.
+template <class LT, int R, class V, class X, class A, class Y, bool NARROW>
+__global__ void __launch_bounds__(rows::THREADS, 5)
+    k_spmv_rows_batch(const BatchMat* __restrict__ mats, const BatchJob* __restrict__ jobs, int njobs) {
+    using G = rows::Geo<LT, R, V, R>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int wi = threadIdx.x >> 5;
+    const int nw = gridDim.x * rows::WARPS;
+    const uint64_t pol_x = l2_evict_last_policy();
+    for (int j = blockIdx.x * rows::WARPS + wi; j < njobs; j += nw) {  // warp-uniform
+        const BatchJob job = jobs[j];
+        const BatchMat& m = mats[job.mat];
+        const int nrows = m.nrows;
+        const X* x = static_cast<const X*>(m.x);
+        Y* y = static_cast<Y*>(m.y);
+        rows::walk<LT, R, V, R>(m.brptr, m.headers, static_cast<const V*>(m.values), m.valptr, job.r_begin, job.r_end,
+                                smem + wi * G::BUF_BYTES,
+                                [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
+                                    rows::chunk_spmv<LT, R, V, X, A, Y, NARROW>(ch, hw, vbuf, x, y, nrows, pol_x);
+                                });
     }
 }
 
@@ -245,112 +317,140 @@ void set_smem(K kernel, int bytes) {
     SPC5_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
-// Calls f(integral_constant<R>, integral_constant<KC>) for r in {1, 2, 4, 8}
-// and kc a power of two up to mm_kc_limit of the kernel's lanes.
-template <class LT, class F>
-void dispatch_rkc(int r, int kc, F&& f) {
+// Calls f(integral_constant<R>) for r in {1, 2, 4, 8}.
+template <class F>
+void dispatch_r(int r, F&& f) {
     using std::integral_constant;
-    auto with_r = [&](auto RC) {
-        constexpr int R_ = decltype(RC)::value;
-        constexpr int KMAX = mm_kc_limit(Layout<LT>::VS, R_, mm_lanes<LT, R_>());
-        switch (kc) {
-            case 1: f(RC, integral_constant<int, 1>{}); return true;
-            case 2: if constexpr (KMAX >= 2) { f(RC, integral_constant<int, 2>{}); return true; } break;
-            case 4: if constexpr (KMAX >= 4) { f(RC, integral_constant<int, 4>{}); return true; } break;
-            case 8: if constexpr (KMAX >= 8) { f(RC, integral_constant<int, 8>{}); return true; } break;
-            case 16: if constexpr (KMAX >= 16) { f(RC, integral_constant<int, 16>{}); return true; } break;
-        }
-        return false;
-    };
-    bool done = false;
     switch (r) {
-        case 1: done = with_r(integral_constant<int, 1>{}); break;
-        case 2: done = with_r(integral_constant<int, 2>{}); break;
-        case 4: done = with_r(integral_constant<int, 4>{}); break;
-        case 8: done = with_r(integral_constant<int, 8>{}); break;
+        case 1: f(integral_constant<int, 1>{}); return;
+        case 2: f(integral_constant<int, 2>{}); return;
+        case 4: f(integral_constant<int, 4>{}); return;
+        case 8: f(integral_constant<int, 8>{}); return;
     }
-    if (!done) throw Error(SPC5CUDA_ERR_INVALID, "unsupported (r, right-hand sides per pass)");
+    throw Error(SPC5CUDA_ERR_FORMAT, "r must be 1, 2, 4 or 8");
 }
 
-template <class LT, class V, class X, class A, class Y>
+// Calls f(integral_constant<R>, integral_constant<KC>) for kc in {2, 4, 8, 16}.
+template <class F>
+void dispatch_rkc(int r, int kc, F&& f) {
+    using std::integral_constant;
+    dispatch_r(r, [&](auto RC) {
+        switch (kc) {
+            case 2: f(RC, integral_constant<int, 2>{}); return;
+            case 4: f(RC, integral_constant<int, 4>{}); return;
+            case 8: f(RC, integral_constant<int, 8>{}); return;
+            case 16: f(RC, integral_constant<int, 16>{}); return;
+        }
+        throw Error(SPC5CUDA_ERR_INVALID, "right-hand sides per pass");
+    });
+}
+
+template <int KIND, class LT, class V, class X, class A, class Y>
 void spmm_rows_impl(const BetaView& m, int k, const X* x, long ldx, long xcs, Y* y, long ldy, long ycs,
                     cudaStream_t s) {
     if (m.nbr <= 0 || k <= 0 || m.nwarps <= 0) return;
-    const int ctas = (m.nwarps + rows::WARPS - 1) / rows::WARPS;
+    const int ctas = (m.nwarps + MM_WARPS - 1) / MM_WARPS;
     const V* vals = static_cast<const V*>(m.values);
     for (int k0 = 0; k0 < k;) {
-        const int kc = spmm_rows_kc(Layout<LT>::VS, m.r, k - k0);
-        dispatch_rkc<LT>(m.r, kc, [&](auto RC, auto KCC) {
+        const X* xp = x + long(k0) * xcs;
+        Y* yp = y + long(k0) * ycs;
+        if (k - k0 == 1 && ldx == 1 && ldy == 1) {  // one right-hand side, contiguous: the SpMV
+            launch_rows_kind(KIND, m, xp, yp, s);
+            return;
+        }
+        if (spmm_columns(Layout<LT>::VS, m.r, m.full_blocks, k - k0)) {
+            const int kc = spmm_cols_kc(Layout<LT>::VS, m.r, k - k0);
+            launch_spmm_cols(KIND, m, kc, xp, ldx, xcs, yp, ldy, ycs, s);
+            k0 += kc;
+            continue;
+        }
+        const int kc = spmm_rows_kc(k - k0);
+        dispatch_rkc(m.r, kc, [&](auto RC, auto KCC) {
             constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-            constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), rows::MM_HB, rows::MM_VB>::SMEM;
+            constexpr int SMEM = MMGeo<LT, R_, V, A>::SMEM;
             auto kern = k_spmm_rows<LT, R_, KC_, V, X, A, Y>;
             set_smem(kern, SMEM);
-            kern<<<ctas, rows::THREADS, SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart,
-                                                   m.nwarps, x + long(k0) * xcs, ldx, xcs, y + long(k0) * ycs, ldy,
-                                                   ycs);
+            kern<<<ctas, MM_THREADS, SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart, m.nwarps,
+                                                   std::min(k - k0, KC_), xp, ldx, xcs, yp, ldy, ycs);
         });
         k0 += kc;
     }
     SPC5_CUDA(cudaGetLastError());
 }
 
+template <class K>
+void launch_jobs(K kern, int threads, int smem, const BatchMat* mats, const BatchJob* jobs, int njobs, cudaStream_t s) {
+    set_smem(kern, smem);
+    int per_sm = 0;
+    SPC5_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+    const int grid = std::max(1, std::min(div_up(njobs, threads / 32), sm_count() * std::max(1, per_sm)));
+    kern<<<grid, threads, smem, s>>>(mats, jobs, njobs);
+}
+
 template <class LT, class V, class X, class A, class Y>
-void batch_rows_impl(int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs, int ctas,
+void batch_rows_impl(int r, int kc, bool narrow, const BatchMat* mats, const BatchJob* jobs, int njobs,
                      cudaStream_t s) {
-    dispatch_rkc<LT>(r, kc, [&](auto RC, auto KCC) {
+    if (kc == 1) {
+        dispatch_r(r, [&](auto RC) {
+            constexpr int R_ = decltype(RC)::value, SMEM = rows::Geo<LT, R_, V, R_>::SMEM;
+            if (narrow) launch_jobs(k_spmv_rows_batch<LT, R_, V, X, A, Y, true>, rows::THREADS, SMEM, mats, jobs, njobs, s);
+            else launch_jobs(k_spmv_rows_batch<LT, R_, V, X, A, Y, false>, rows::THREADS, SMEM, mats, jobs, njobs, s);
+        });
+        return;
+    }
+    dispatch_rkc(r, kc, [&](auto RC, auto KCC) {
         constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), rows::MM_HB, rows::MM_VB>::SMEM;
-        auto kern = k_spmm_rows_batch<LT, R_, KC_, V, X, A, Y>;
-        set_smem(kern, SMEM);
-        int per_sm = 0;
-        SPC5_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, rows::THREADS, SMEM));
-        const int grid = std::max(1, std::min(ctas, sm_count() * std::max(1, per_sm)));
-        kern<<<grid, rows::THREADS, SMEM, s>>>(mats, jobs, njobs);
+        launch_jobs(k_spmm_rows_batch<LT, R_, KC_, V, X, A, Y>, MM_THREADS, MMGeo<LT, R_, V, A>::SMEM, mats, jobs, njobs, s);
     });
 }
 
 }  // namespace
 
-int spmm_rows_kc(int vs, int r, int k) {
-    const int lanes = (vs == 16 && r == 8) ? 16 : 8;
-    const int kmax = mm_kc_limit(vs, r, lanes);
-    int kc = 1;
-    while (kc * 2 <= k && kc * 2 <= kmax) kc *= 2;
-    return kc;
+// Measured on B200 (us, columns / lists; 27-point stencil 64^3, fill 3 per
+// sub-row and block at r = 4, 1.5 at r = 8; banded n = 100,000, fill 1 and 0.9):
+//   r = 8, FP64: k = 2 47 / 59 and 30 / 39, k = 3 90 / 92 and 55 / 53, k = 4 72 /
+//     78 and 49 / 45, k = 8 (two passes of columns) 149 / 96 and 96 / 61;
+//   r = 4, FP64: k = 2 42 / 55 and 31 / 29, k = 4 49 / 72 and 43 / 34, k = 8 98 /
+//     107 and 84 / 45, k = 12 (two passes of columns) 145 / 172;
+//   float layout, r = 4: k = 2 55 / 55 and 32 / 35, k = 3 111 / 86 and 61 / 49, k =
+//     4 67 / 74 and 41 / 43, k = 5 126 / 135, k = 8 137 / 112 and 81 / 55; r = 8: k = 4 65 / 82 and
+//     43 / 49, k = 8 133 / 119 and 84 / 61;
+//   r = 1 and 2: lists (r = 2, k = 4 81 / 74 and 58 / 34).
+bool spmm_columns(int vs, int r, bool full_blocks, int k) {
+    if (vs == 16) return r >= 4 && k <= 5 && k != 3;
+    if (r == 8) return k <= 4;
+    return r == 4 && full_blocks && k <= 12;
 }
+
+int spmm_rows_kc(int k) { return k > 8 ? 16 : (k > 4 ? 8 : (k > 2 ? 4 : 2)); }
 
 void launch_spmm_rows_f64(const BetaView& m, int k, const double* x, long ldx, long xcs, double* y, long ldy,
                           long ycs, cudaStream_t s) {
-    spmm_rows_impl<double, double, double, double, double>(m, k, x, ldx, xcs, y, ldy, ycs, s);
+    spmm_rows_impl<0, double, double, double, double, double>(m, k, x, ldx, xcs, y, ldy, ycs, s);
 }
 
 void launch_spmm_rows_f32(const BetaView& m, int k, const float* x, long ldx, long xcs, float* y, long ldy,
                           long ycs, cudaStream_t s) {
-    spmm_rows_impl<float, float, float, float, float>(m, k, x, ldx, xcs, y, ldy, ycs, s);
+    spmm_rows_impl<1, float, float, float, float, float>(m, k, x, ldx, xcs, y, ldy, ycs, s);
 }
 
 void launch_spmm_rows_mixed(const BetaView& m, int k, const float* x, long ldx, long xcs, double* y, long ldy,
                             long ycs, cudaStream_t s) {
-    spmm_rows_impl<float, float, float, double, double>(m, k, x, ldx, xcs, y, ldy, ycs, s);
+    spmm_rows_impl<2, float, float, float, double, double>(m, k, x, ldx, xcs, y, ldy, ycs, s);
 }
 
 void launch_spmm_rows_mixed8(const BetaView& m, int k, const float* x, long ldx, long xcs, double* y, long ldy,
                              long ycs, cudaStream_t s) {
-    spmm_rows_impl<double, float, float, double, double>(m, k, x, ldx, xcs, y, ldy, ycs, s);
+    spmm_rows_impl<3, double, float, float, double, double>(m, k, x, ldx, xcs, y, ldy, ycs, s);
 }
 
-void launch_batch_rows(int kind, int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs,
+void launch_batch_rows(int kind, int r, int kc, bool narrow, const BatchMat* mats, const BatchJob* jobs, int njobs,
                        cudaStream_t s) {
     if (njobs <= 0) return;
-    const int ctas = div_up(njobs, rows::WARPS);
-    if (kind == 0)
-        batch_rows_impl<double, double, double, double, double>(r, kc, mats, jobs, njobs, ctas, s);
-    else if (kind == 1)
-        batch_rows_impl<float, float, float, float, float>(r, kc, mats, jobs, njobs, ctas, s);
-    else if (kind == 2)
-        batch_rows_impl<float, float, float, double, double>(r, kc, mats, jobs, njobs, ctas, s);
-    else
-        batch_rows_impl<double, float, float, double, double>(r, kc, mats, jobs, njobs, ctas, s);
+    if (kind == 0) batch_rows_impl<double, double, double, double, double>(r, kc, narrow, mats, jobs, njobs, s);
+    else if (kind == 1) batch_rows_impl<float, float, float, float, float>(r, kc, narrow, mats, jobs, njobs, s);
+    else if (kind == 2) batch_rows_impl<float, float, float, double, double>(r, kc, narrow, mats, jobs, njobs, s);
+    else batch_rows_impl<double, float, float, double, double>(r, kc, narrow, mats, jobs, njobs, s);
     SPC5_CUDA(cudaGetLastError());
 }
 

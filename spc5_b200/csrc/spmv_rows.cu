@@ -42,13 +42,13 @@
 
 #include "common.cuh"
 #include "kernels.h"
-#include "rows_stage.cuh"
+#include "rows_blocks.cuh"
 
 namespace spc5cuda {
 
 namespace {
 
-using rows::FULL;
+using namespace rows;
 constexpr int ROWS_THREADS = rows::THREADS;
 constexpr int ROWS_WARPS = rows::WARPS;
 constexpr int ROWS_CTAS_PER_SM = 16;
@@ -56,98 +56,6 @@ constexpr int ROWS_CTAS_PER_SM = 16;
 // The narrow kernel runs when at least 7 of 8 sampled blocks are narrow.
 __host__ __device__ inline bool rows_narrow(int narrow, int sampled) {
     return sampled > 0 && long(narrow) * 8 >= long(sampled) * 7;
-}
-
-// The lane of sub-row q of its block-row: where it stands in the staged chunk.
-struct SubRow {
-    int n;      // blocks left
-    int hoff;   // byte offset of the next block's header in the staged headers
-    int v;      // index of its first value in the staged values
-};
-
-// One staged block as sub-row q sees it: first column, own mask, its values'
-// place (from the block's first value) and the block's value count.
-template <class LT, int R>
-struct Block {
-    static constexpr int MW = Header<LT, R>::MASK_WORDS;
-    int col;
-    uint32_t mw[MW], m;
-};
-
-template <class LT, int R>
-struct SubRowOf {
-    static constexpr int MB = Layout<LT>::MASK_BYTES, MW = Header<LT, R>::MASK_WORDS;
-    static constexpr int FPW = 4 / MB, BITS = 8 * MB;
-    int wq;            // mask word of sub-row q
-    unsigned sh;       // its field in that word
-    uint32_t low[MW];  // mask bits of the sub-rows below q
-    __device__ __forceinline__ explicit SubRowOf(int q) : wq(q / FPW), sh(unsigned(q % FPW) * BITS) {
-#pragma unroll
-        for (int w = 0; w < MW; ++w) low[w] = w < wq ? 0xFFFFFFFFu : (w == wq ? (1u << sh) - 1u : 0u);
-    }
-    // the block at header offset off, empty when !ok
-    __device__ __forceinline__ void load(const uint32_t* hw, int off, bool ok, Block<LT, R>& b) const {
-        constexpr uint32_t FMASK = MB == 1 ? 0xFFu : 0xFFFFu;
-        b.col = 0;
-#pragma unroll
-        for (int w = 0; w < MW; ++w) b.mw[w] = 0u;
-        if (ok) b.col = rows::decode_staged<LT, R>(hw, off, b.mw);
-        uint32_t word = b.mw[0];
-#pragma unroll
-        for (int w = 1; w < MW; ++w) word = w == wq ? b.mw[w] : word;
-        b.m = R == 1 ? word : (word >> sh) & FMASK;
-    }
-    __device__ __forceinline__ int before(const Block<LT, R>& b) const {
-        int n = 0;
-        if constexpr (R > 1) {
-#pragma unroll
-            for (int w = 0; w < MW; ++w) n += __popc(b.mw[w] & low[w]);
-        }
-        return n;
-    }
-    static __device__ __forceinline__ int values(const Block<LT, R>& b) {
-        int n = 0;
-#pragma unroll
-        for (int w = 0; w < MW; ++w) n += __popc(b.mw[w]);
-        return n;
-    }
-};
-
-// All VS columns of every block, UT blocks per step (their x loads are issued
-// together).
-template <class LT, int R, class V, class X, class A, int UT>
-__device__ __forceinline__ void wide_blocks(const uint32_t* hw, const V* vbuf, const X* __restrict__ x, int q,
-                                            SubRow at, uint64_t pol_x, A (&acc)[Layout<LT>::VS]) {
-    constexpr int VS = Layout<LT>::VS, STRIDE = Header<LT, R>::STRIDE;
-    const SubRowOf<LT, R> me(q);
-    const int steps = (__reduce_max_sync(FULL, at.n) + UT - 1) / UT;
-#pragma unroll 1
-    for (int step = 0; step < steps; ++step) {
-        Block<LT, R> b[UT];
-        X xk[UT][VS];
-#pragma unroll
-        for (int u = 0; u < UT; ++u) me.load(hw, at.hoff + u * STRIDE, u < at.n, b[u]);
-#pragma unroll
-        for (int u = 0; u < UT; ++u) {
-            const X* xp = x + b[u].col;
-#pragma unroll
-            for (int c = 0; c < VS; ++c) xk[u][c] = b[u].m & (1u << c) ? ld_x(xp + c, pol_x) : X(0);
-        }
-#pragma unroll
-        for (int u = 0; u < UT; ++u) {
-            const V* vp = vbuf + at.v + me.before(b[u]);
-#pragma unroll
-            for (int c = 0; c < VS; ++c) {
-                if (b[u].m & (1u << c)) {
-                    acc[c] = fma(A(*vp), A(xk[u][c]), acc[c]);
-                    ++vp;
-                }
-            }
-            at.v += me.values(b[u]);
-        }
-        at.n -= UT;
-        at.hoff += UT * STRIDE;
-    }
 }
 
 // CTAs per SM asked of the compiler.  Wide: 6 (80 registers), 4 where 4 blocks of
@@ -164,106 +72,6 @@ constexpr int row_ctas(bool narrow) {
     return R == 8 && VS == 8 && sizeof(X) == 8 ? 4 : 6;
 }
 
-// A window of NS columns, from the first column of the sub-row's first
-// non-empty mask on: accumulator a is column (rho + a) mod VS.
-constexpr int NS = 3;
-template <class LT, int R, class V, class X, class A>
-__device__ __forceinline__ void narrow_blocks(const uint32_t* hw, const V* vbuf, const X* __restrict__ x, int q,
-                                              SubRow at, uint64_t pol_x, A (&acc)[Layout<LT>::VS]) {
-    constexpr int VS = Layout<LT>::VS, STRIDE = Header<LT, R>::STRIDE;
-    constexpr uint32_t VSMASK = (1u << VS) - 1u;
-    constexpr bool WRAP = R == VS;  // the window may run over the last column into the next block
-    // blocks per step: a 27-point stencil's row has 9 at r <= 4 (2 / 3 / 4 blocks
-    // measured on B200: 160^3 r = 4 253 / 240 / 249 us, 101^3 r = 1 f32 52 / 48 / 50)
-    constexpr int UT = 3;
-    const SubRowOf<LT, R> me(q);
-    int rho = 0;
-    // the window's columns (bit[a]), the columns outside it (all of them until
-    // the lane has met its first mask; at r = 1 a block starts at its first
-    // column), and x there
-    uint32_t bit[NS], outside;
-    const X* xw[NS];
-    auto window = [&]() {
-        outside = VSMASK;
-#pragma unroll
-        for (int a = 0; a < NS; ++a) {
-            const int c = WRAP ? (rho + a) & (VS - 1) : rho + a;
-            bit[a] = 1u << c;
-            outside &= ~bit[a];
-            xw[a] = x + c;
-        }
-    };
-    window();
-    if constexpr (R > 1) outside = VSMASK;
-    const int steps = (__reduce_max_sync(FULL, at.n) + UT - 1) / UT;
-#pragma unroll 1
-    for (int step = 0; step < steps; ++step) {
-        Block<LT, R> b[UT];
-        uint32_t some = 0u;
-#pragma unroll
-        for (int u = 0; u < UT; ++u) {
-            me.load(hw, at.hoff + u * STRIDE, u < at.n, b[u]);
-            some |= b[u].m;
-        }
-        if (__any_sync(FULL, (some & outside) != 0u)) {
-            bool wide = true;
-            if constexpr (R > 1) {
-                if (some && outside == VSMASK) {  // the lane's first masks
-                    uint32_t first = b[UT - 1].m;
-#pragma unroll
-                    for (int u = UT - 2; u >= 0; --u) first = b[u].m ? b[u].m : first;
-                    rho = __ffs(first) - 1;
-                    window();
-                }
-                wide = __any_sync(FULL, (some & outside) != 0u);
-            }
-            if (wide) {
-                // a wide mask: the accumulators back at their columns, and the
-                // rest of the chunk over all columns
-                if constexpr (R > 1) {
-#pragma unroll
-                    for (int d = 1; d < VS; d <<= 1) {
-                        A t[VS];
-#pragma unroll
-                        for (int c = 0; c < VS; ++c) t[c] = acc[c];
-#pragma unroll
-                        for (int c = 0; c < VS; ++c) acc[c] = (rho & d) ? t[(c - d) & (VS - 1)] : t[c];
-                    }
-                }
-                wide_blocks<LT, R, V, X, A, 1>(hw, vbuf, x, q, at, pol_x, acc);
-                return;
-            }
-        }
-        X xk[UT][NS];
-#pragma unroll
-        for (int u = 0; u < UT; ++u) {
-#pragma unroll
-            for (int a = 0; a < NS; ++a) {
-                xk[u][a] = b[u].m & bit[a] ? ld_x(xw[a] + b[u].col, pol_x) : X(0);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < UT; ++u) {
-            // values are in column order: those of the window's columns
-            // past the last one (its wrapped part) come first
-            const V* v0 = vbuf + at.v + me.before(b[u]);
-            const V* vp = v0;
-            if constexpr (WRAP) vp += __popc(b[u].m & ((1u << rho) - 1u));
-#pragma unroll
-            for (int a = 0; a < NS; ++a) {
-                if (WRAP && a > 0 && rho == VS - a) vp = v0;
-                if (b[u].m & bit[a]) {
-                    acc[a] = fma(A(*vp), A(xk[u][a]), acc[a]);
-                    ++vp;
-                }
-            }
-            at.v += me.values(b[u]);
-        }
-        at.n -= UT;
-        at.hoff += UT * STRIDE;
-    }
-}
-
 template <class LT, int R, class V, class X, class A, class Y, bool NARROW>
 __global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, X, A>(NARROW))
     k_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
@@ -272,15 +80,9 @@ __global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, X, A>(NARROW))
     // a launch gated on a device word (see BetaView::run_if)
     if (run_if && __ldg(run_if) != run_if_value) return;
     using G = rows::Geo<LT, R, V, R>;
-    constexpr int VS = G::VS;
-    constexpr bool Y_ATOMIC = sizeof(Y) == 8;  // red.add.f64 is y + s rounded once
     extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31;
     const int wi = threadIdx.x >> 5;
     const int warp = blockIdx.x * ROWS_WARPS + wi;
-    const int slot = lane / R;  // block-row of the chunk
-    const int q = lane % R;     // sub-row
-
     int r_begin = 0, r_stop = 0;
     if (warp < nwarps) {
         r_begin = __ldg(wstart + warp);
@@ -288,39 +90,11 @@ __global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, X, A>(NARROW))
     }
     const uint64_t pol_x = l2_evict_last_policy();
 
-    // ---- the blocks of block-row r0 + slot of a staged chunk
-    auto compute = [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
-        const int src = slot > 0 ? slot - 1 : 0;
-        const int b_prev = __shfl_sync(FULL, ch.b_hi, src);
-        const int v_prev = __shfl_sync(FULL, ch.v_hi, src);
-        const int b_mine = __shfl_sync(FULL, ch.b_hi, slot);
-        const bool mine = slot < ch.nrow;
-        const int b = slot > 0 ? b_prev : ch.b_lo;
-        SubRow at;
-        at.n = mine ? b_mine - b : 0;
-        at.hoff = int(long(b) * G::STRIDE - ch.h_al);
-        at.v = (slot > 0 ? v_prev : ch.v_lo) - ch.v_al;
-
-        A acc[VS];
-#pragma unroll
-        for (int c = 0; c < VS; ++c) acc[c] = A(0);
-        if constexpr (NARROW) narrow_blocks<LT, R, V, X, A>(hw, vbuf, x, q, at, pol_x, acc);
-        else wide_blocks<LT, R, V, X, A, (R == 8 && VS == 8) ? 4 : (16 / VS > 1 ? 16 / VS : 1)>(hw, vbuf, x, q, at, pol_x, acc);
-        // ---- row sum: the _mm512_reduce_add tree (distance VS/2, ..., 1)
-#pragma unroll
-        for (int d = VS / 2; d >= 1; d >>= 1) {
-#pragma unroll
-            for (int c = 0; c < d; ++c) acc[c] = acc[c] + acc[c + d];
-        }
-        const long yrow = long(ch.r0 + slot) * R + q;
-        if (mine && yrow < nrows) {
-            if constexpr (Y_ATOMIC) atomicAdd(y + yrow, Y(acc[0]));
-            else y[yrow] = y[yrow] + Y(acc[0]);
-        }
-    };
-
     unsigned char* wbuf = smem + wi * G::BUF_BYTES;
-    rows::walk<LT, R, V, R>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
+    rows::walk<LT, R, V, R>(brptr, headers, values, valptr, r_begin, r_stop, wbuf,
+                            [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
+                                chunk_spmv<LT, R, V, X, A, Y, NARROW>(ch, hw, vbuf, x, y, nrows, pol_x);
+                            });
 }
 
 template <class K>
@@ -515,6 +289,15 @@ void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* v
     const int vbytes = vt == SPC5CUDA_F64 ? 8 : 4;
     k_fit_flag<<<1, 1, 0, s>>>(work + 1, stride, vbytes, ROWS_HB, ROWS_VB, work);
     SPC5_CUDA(cudaGetLastError());
+}
+
+void launch_rows_kind(int kind, const BetaView& m, const void* x, void* y, cudaStream_t s) {
+    switch (kind) {
+        case 0: launch_rows_f64(m, static_cast<const double*>(x), static_cast<double*>(y), s); return;
+        case 1: launch_rows_f32(m, static_cast<const float*>(x), static_cast<float*>(y), s); return;
+        case 2: launch_rows_mixed(m, static_cast<const float*>(x), static_cast<double*>(y), s); return;
+        default: launch_rows_mixed8(m, static_cast<const float*>(x), static_cast<double*>(y), s); return;
+    }
 }
 
 void launch_rows_f64(const BetaView& m, const double* x, double* y, cudaStream_t s) {
