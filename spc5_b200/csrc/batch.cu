@@ -112,7 +112,7 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
                     } else if (k[i] == 1 && ldx[i] == 1 && ldy[i] == 1) {
                         kc = 1;
                         how = m->rows_narrow ? SPMV_NARROW : SPMV_WIDE;
-                    } else if (spmm_columns(vs, m->r, m->full_blocks(), left)) {
+                    } else if (spmm_columns(vs, value_bytes_of(m->value_type), m->r, m->full_blocks(), left)) {
                         kc = spmm_cols_kc(vs, m->r, left);
                         how = COLUMNS;
                     } else {

@@ -154,7 +154,7 @@ int spmm_rows_kc(int k);
 // Whether a pass with k right-hand sides left runs with a lane per column
 // (spmm_cols.cu) instead: few right-hand sides on blocks of many rows.
 // full_blocks: at least two values per sub-row and block on average.
-bool spmm_columns(int vs, int r, bool full_blocks, int k);
+bool spmm_columns(int vs, int value_bytes, int r, bool full_blocks, int k);
 // Right-hand sides of such a pass (a power of two), and its launch for a kind.
 int spmm_cols_kc(int vs, int r, int k);
 void launch_spmm_cols(int kind, const BetaView& m, int kc, const void* x, long ldx, long xcs, void* y, long ldy,

@@ -249,10 +249,10 @@ __device__ __forceinline__ void chunk_spmv(const Chunk& ch, const uint32_t* hw, 
     if constexpr (NARROW)
         narrow_blocks<LT, R, V, X, A>(hw, vbuf, x, lane % R, at, pol_x, acc);
     else
-        // blocks per step: 4 at r = 8 for double blocks, else 16 / VS (measured
-        // on B200: 4 blocks lifted r = 8 by 10% and slowed r = 2 by 9%)
-        wide_blocks<LT, R, V, X, A, (R == 8 && VS == 8) ? 4 : (16 / VS > 1 ? 16 / VS : 1)>(hw, vbuf, x, lane % R, at,
-                                                                                         pol_x, acc);
+        // 16 columns per step (r = 8, FP64, 2 blocks and 6 CTAs per SM against 4 and
+        // 4 on B200: banded 150,000 44 / 42 us, 5-point Poisson 700^2 19.2 / 21.1;
+        // mixed, banded 200,000 14.2 / 19.1)
+        wide_blocks<LT, R, V, X, A, (16 / VS > 1 ? 16 / VS : 1)>(hw, vbuf, x, lane % R, at, pol_x, acc);
     const A sum = reduce_tree<A, VS>(acc);
     const long yrow = long(ch.r0) * R + lane;  // sub-row `lane` of the chunk
     if (lane / R < ch.nrow && yrow < nrows) add_to(y + yrow, Y(sum));

@@ -358,7 +358,7 @@ void spmm_rows_impl(const BetaView& m, int k, const X* x, long ldx, long xcs, Y*
             launch_rows_kind(KIND, m, xp, yp, s);
             return;
         }
-        if (spmm_columns(Layout<LT>::VS, m.r, m.full_blocks, k - k0)) {
+        if (spmm_columns(Layout<LT>::VS, int(sizeof(V)), m.r, m.full_blocks, k - k0)) {
             const int kc = spmm_cols_kc(Layout<LT>::VS, m.r, k - k0);
             launch_spmm_cols(KIND, m, kc, xp, ldx, xcs, yp, ldy, ycs, s);
             k0 += kc;
@@ -416,10 +416,12 @@ void batch_rows_impl(int r, int kc, bool narrow, const BatchMat* mats, const Bat
 //     4 67 / 74 and 41 / 43, k = 5 126 / 135, k = 8 137 / 112 and 81 / 55; r = 8: k = 4 65 / 82 and
 //     43 / 49, k = 8 133 / 119 and 84 / 61;
 //   r = 1 and 2: lists (r = 2, k = 4 81 / 74 and 58 / 34).
-bool spmm_columns(int vs, int r, bool full_blocks, int k) {
+//   8 columns of float values (mixed): as FP64, but the columns' x are half as
+//     wide: r = 4, fill 3, k = 16 166 / 183; r = 8, k = 5 135 / 153.
+bool spmm_columns(int vs, int value_bytes, int r, bool full_blocks, int k) {
     if (vs == 16) return r >= 4 && k <= 5 && k != 3;
-    if (r == 8) return k <= 4;
-    return r == 4 && full_blocks && k <= 12;
+    if (r == 8) return k <= (value_bytes == 4 ? 5 : 4);
+    return r == 4 && full_blocks && k <= (value_bytes == 4 ? 16 : 12);
 }
 
 int spmm_rows_kc(int k) { return k > 8 ? 16 : (k > 4 ? 8 : (k > 2 ? 4 : 2)); }

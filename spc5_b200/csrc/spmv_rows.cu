@@ -58,22 +58,20 @@ __host__ __device__ inline bool rows_narrow(int narrow, int sampled) {
     return sampled > 0 && long(narrow) * 8 >= long(sampled) * 7;
 }
 
-// CTAs per SM asked of the compiler.  Wide: 6 (80 registers), 4 where 4 blocks of
-// double x per step need more.  Narrow: 7 (72 registers: the 5-point Poisson
+// CTAs per SM asked of the compiler.  Wide: 6 (80 registers).  Narrow: 7 (72 registers: the 5-point Poisson
 // 512^2 at r = 2 then takes two chunks per warp instead of three, 8.3 against
 // 9.4 us on the device; 160^3 at r = 4 197 against 203 us), 6 at r = 8, whose
 // window wraps (127^3: 7 was 7% slower).  5 where 16 double accumulators (the
 // float layout in mixed precision) need the registers.
-template <class LT, int R, class X, class A>
+template <class LT, int R, class A>
 constexpr int row_ctas(bool narrow) {
     constexpr int VS = Layout<LT>::VS;
     if (VS * sizeof(A) > 64) return 5;
-    if (narrow) return R < 8 ? 7 : 6;
-    return R == 8 && VS == 8 && sizeof(X) == 8 ? 4 : 6;
+    return narrow && R < 8 ? 7 : 6;
 }
 
 template <class LT, int R, class V, class X, class A, class Y, bool NARROW>
-__global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, X, A>(NARROW))
+__global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, A>(NARROW))
     k_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
            const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart, int nwarps,
            const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
