@@ -59,6 +59,14 @@ inline int div_up(long a, long b) { return int((a + b - 1) / b); }
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// CTAs of a kernel that one SM holds (at least 1).
+template <class K>
+int resident_ctas(K kern, int threads, int smem) {
+    int n = 0;
+    SPC5_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, size_t(smem)));
+    return n > 0 ? n : 1;
+}
+
 // ---------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------

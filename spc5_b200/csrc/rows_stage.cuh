@@ -22,6 +22,16 @@ constexpr int WARPS = THREADS / 32;
 // (measured on B200: 10 KB buffers, 5 per SM, were 3% slower on the
 // power-law matrix and 10% on the 27-point stencil; 5 KB chunks were too
 // small for the stencil).
+// First block-row of warp w of W: the boundaries wstart of a partition made for
+// nwarps warps (the SpMV's), interpolated for a kernel that keeps W resident.
+// The row counts are int, so the product stays in 64 bits.
+__device__ __forceinline__ int part_start(const int* __restrict__ wstart, int nwarps, int w, int W) {
+    const long at = long(w) * nwarps;
+    const int p = int(at / W), f = int(at % W);
+    const int a = __ldg(wstart + p);
+    return f == 0 ? a : a + int(long(__ldg(wstart + p + 1) - a) * f / W);
+}
+
 constexpr int HB = 1536;  // header bytes of one warp's staging buffer
 constexpr int VB = 6144;  // value bytes of one warp's staging buffer
 constexpr unsigned FULL = 0xffffffffu;

@@ -34,8 +34,17 @@ using rows::FULL;
 
 // Registers limit this kernel to 4 CTAs per SM, so it stages larger chunks than
 // the SpMV (every block-row that fits the SpMV's buffers fits these).
-constexpr int COLS_HB = 2048;
-constexpr int COLS_VB = 8192;
+// One or two right-hand sides leave room for the SpMV's own chunks and 5 or 6
+// CTAs, except with double values at r = 8 (stencil 64^3, k = 2 on a B200: mixed
+// 77 us at 4 CTAs and larger chunks / 67 so, r = 4 46 / 38; FP64, r = 8 55 / 73).
+template <class V, int R, int KC>
+constexpr bool cols_small = KC <= 2 && (R < 8 || sizeof(V) == 4);
+template <class V, int R, int KC>
+constexpr int cols_hb = cols_small<V, R, KC> ? rows::HB : 2048;
+template <class V, int R, int KC>
+constexpr int cols_vb = cols_small<V, R, KC> ? rows::VB : 8192;
+template <class V, int R, int KC>
+constexpr int cols_ctas(int acc_bytes) { return cols_small<V, R, KC> ? (acc_bytes > 64 ? 5 : 6) : 1; }
 
 // Union of the sub-row masks (bit c: some sub-row has a value in column c).
 template <class LT, int R>
@@ -111,7 +120,7 @@ __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brpt
     constexpr int L = mm_lanes<LT, R>();  // lanes per block-row
     constexpr int CPL = VS / L;                // columns per lane: q + L k
     constexpr int LOGL = L == 16 ? 4 : (L == 8 ? 3 : (L == 4 ? 2 : (L == 2 ? 1 : 0)));
-    using G = rows::Geo<LT, R, V, L, COLS_HB, COLS_VB>;
+    using G = rows::Geo<LT, R, V, L, cols_hb<V, R, KC>, cols_vb<V, R, KC>>;
     constexpr int MB = G::MB, MW = G::MW;
     constexpr int FPW = 4 / MB;  // mask fields per 32-bit word
     constexpr int BITS = 8 * MB;
@@ -263,21 +272,24 @@ __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brpt
         }
         flush(mine, ch.r0 + slot);
     };
-    rows::walk<LT, R, V, L, COLS_HB, COLS_VB>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
+    rows::walk<LT, R, V, L, cols_hb<V, R, KC>, cols_vb<V, R, KC>>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
 }
 
-// One matrix: warp w owns block-rows [wstart[w], wstart[w + 1]).
+// One matrix: the grid's warps, one resident wave, share its block-rows
+// (part_start).  The SpMV's partition is for 5 to 7 CTAs per SM, of which 3 or 4
+// fit here: stencil 64^3, r = 8, on a B200 FP64 k = 4 74 us, now 60; k = 2 55 / 45;
+// mixed k = 5 148 / 121.
 template <class LT, int R, int KC, class V, class X, class A, class Y>
-__global__ void __launch_bounds__(rows::THREADS)
+__global__ void __launch_bounds__(rows::THREADS, cols_ctas<V, R, KC>(Layout<LT>::VS * int(sizeof(A))))
     k_spmm_cols(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
                 const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart,
                 int nwarps, const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym, long ldy, long ycs) {
-    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), COLS_HB, COLS_VB>;
+    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), cols_hb<V, R, KC>, cols_vb<V, R, KC>>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
     const int warp = blockIdx.x * rows::WARPS + wi;
-    if (warp >= nwarps) return;  // warp-uniform
-    const int r_begin = __ldg(wstart + warp), r_stop = __ldg(wstart + warp + 1);
+    const int W = gridDim.x * rows::WARPS;
+    const int r_begin = rows::part_start(wstart, nwarps, warp, W), r_stop = rows::part_start(wstart, nwarps, warp + 1, W);
     mm_range<LT, R, KC, V, X, A, Y>(nrows, brptr, headers, values, valptr, r_begin, r_stop, xm, ldx, xcs, ym, ldy, ycs,
                                     smem + wi * G::BUF_BYTES);
 }
@@ -286,9 +298,9 @@ __global__ void __launch_bounds__(rows::THREADS)
 // j is block-rows [r_begin, r_end) of mats[j.mat] for right-hand sides
 // [kofs, kofs + KC).  X and Y of a batch are row-major (xcs = ycs = 1).
 template <class LT, int R, int KC, class V, class X, class A, class Y>
-__global__ void __launch_bounds__(rows::THREADS)
+__global__ void __launch_bounds__(rows::THREADS, cols_ctas<V, R, KC>(Layout<LT>::VS * int(sizeof(A))))
     k_spmm_cols_batch(const BatchMat* __restrict__ mats, const BatchJob* __restrict__ jobs, int njobs) {
-    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), COLS_HB, COLS_VB>;
+    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), cols_hb<V, R, KC>, cols_vb<V, R, KC>>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
     const int nw = gridDim.x * rows::WARPS;
@@ -333,12 +345,13 @@ void dispatch_rkc(int r, int kc, F&& f) {
 template <class LT, class V, class X, class A, class Y>
 void cols_pass(const BetaView& m, int kc, const void* x, long ldx, long xcs, void* y, long ldy, long ycs,
                cudaStream_t s) {
-    const int ctas = (m.nwarps + rows::WARPS - 1) / rows::WARPS;
     dispatch_rkc<LT>(m.r, kc, [&](auto RC, auto KCC) {
         constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), COLS_HB, COLS_VB>::SMEM;
+        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), cols_hb<V, R_, KC_>, cols_vb<V, R_, KC_>>::SMEM;
         auto kern = k_spmm_cols<LT, R_, KC_, V, X, A, Y>;
         set_smem(kern, SMEM);
+        static const int per_sm = resident_ctas(kern, rows::THREADS, SMEM);
+        const int ctas = std::min((m.nwarps + rows::WARPS - 1) / rows::WARPS, sm_count() * per_sm);
         kern<<<ctas, rows::THREADS, SMEM, s>>>(m.nrows, m.brptr, m.headers, static_cast<const V*>(m.values), m.valptr,
                                                m.wstart, m.nwarps, static_cast<const X*>(x), ldx, xcs,
                                                static_cast<Y*>(y), ldy, ycs);
@@ -350,7 +363,7 @@ template <class LT, class V, class X, class A, class Y>
 void cols_batch(int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs, cudaStream_t s) {
     dispatch_rkc<LT>(r, kc, [&](auto RC, auto KCC) {
         constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), COLS_HB, COLS_VB>::SMEM;
+        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), cols_hb<V, R_, KC_>, cols_vb<V, R_, KC_>>::SMEM;
         auto kern = k_spmm_cols_batch<LT, R_, KC_, V, X, A, Y>;
         set_smem(kern, SMEM);
         int per_sm = 0;

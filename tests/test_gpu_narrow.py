@@ -73,3 +73,28 @@ def test_narrow_masks_equal_oracle(cuda, tag, r):
             S.core_spmv(r, csr.nrows, dev(ob), dev(oh), dev(ov), dev(x), y)
             torch.cuda.synchronize()
             assert y.cpu().numpy().tobytes() == yo.tobytes(), (csr.name, "drop-in")
+
+
+@pytest.mark.parametrize("tag", ["f64", "f32", "mixed"])
+@pytest.mark.parametrize("r", [1, 4, 8])
+def test_spmm_waves_equal_spmv(cuda, tag, r):
+    """Parts of several block-rows, long and short, whose boundaries the SpMM
+    kernels interpolate: every column is the SpMV's, bit for bit."""
+    dt = np.float64 if tag == "f64" else np.float32
+    yt = torch.float64 if tag != "f32" else torch.float32
+    csr = strewn(40003, 1009, 9)
+    m = S.csr_matrix(csr.rowptr, csr.colidx, csr.values.astype(dt), csr.ncols)
+    S.CSR_to_SPC5(m, S.FORMAT_OF_R[r])
+    assert m.kernel == S.KERNEL_ROWS
+    spmv, spmm = (S.SPC5_Spmv_mixed, S.SPC5_Spmm_mixed) if tag == "mixed" else (S.SPC5_Spmv, S.SPC5_Spmm)
+    rng = np.random.default_rng(2)
+    x = dev(rng.uniform(-1, 1, (csr.ncols, 7)).astype(dt))
+    want = torch.zeros(csr.nrows, 7, dtype=yt, device="cuda")
+    for j in range(7):
+        y = torch.zeros(csr.nrows, dtype=yt, device="cuda")
+        spmv(m, x[:, j].contiguous(), y)
+        want[:, j] = y
+    for k in (2, 3, 5, 7):
+        got = torch.zeros(csr.nrows, k, dtype=yt, device="cuda")
+        spmm(m, x[:, :k].contiguous(), got)
+        assert torch.equal(got, want[:, :k])
