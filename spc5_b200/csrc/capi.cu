@@ -76,28 +76,48 @@ void spc5cuda::valptr_from_headers(int mask_bytes, int r, int nbr, const int* br
     exclusive_scan_i32(valptr, valptr, nbr, tmp.as<int>(), s);
 }
 
-// The library's own stream-ordered memory pool on the current device: the
-// per-call scratch of the drop-in symbols comes from it, and it keeps freed memory for the next call (release threshold:
-// never), so repeated calls do not go back to the driver.  One pool per
-// device for the process lifetime.
-cudaMemPool_t spc5cuda::scratch_pool() {
+// One pool and one allocation stream per device for the process lifetime.
+namespace {
+struct DeviceMemory {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+    void* anchor = nullptr;  // keeps the memory mapped that wait_device() takes and frees
+};
+
+const DeviceMemory& device_memory() {
     static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
+    static DeviceMemory mem[64];
+    constexpr uint64_t keep = uint64_t(4) << 30;
     int dev = 0;
     SPC5_CUDA(cudaGetDevice(&dev));
     require(dev >= 0 && dev < 64, SPC5CUDA_ERR_UNSUPPORTED, "device index");
     std::lock_guard<std::mutex> lk(mu);
-    if (!pools[dev]) {
-        cudaMemPoolProps props;
-        std::memset(&props, 0, sizeof(props));
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        SPC5_CUDA(cudaMemPoolCreate(&pools[dev], &props));
-        uint64_t keep = UINT64_MAX;
-        SPC5_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+    DeviceMemory& m = mem[dev];
+    if (!m.stream) {
+        if (!m.pool) {
+            cudaMemPoolProps props;
+            std::memset(&props, 0, sizeof(props));
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            SPC5_CUDA(cudaMemPoolCreate(&m.pool, &props));
+            uint64_t bytes = keep;
+            SPC5_CUDA(cudaMemPoolSetAttribute(m.pool, cudaMemPoolAttrReleaseThreshold, &bytes));
+        }
+        if (!m.anchor) SPC5_CUDA(cudaMalloc(&m.anchor, 16));
+        SPC5_CUDA(cudaStreamCreateWithFlags(&m.stream, cudaStreamNonBlocking));
     }
-    return pools[dev];
+    return m;
+}
+}  // namespace
+
+cudaMemPool_t spc5cuda::scratch_pool() { return device_memory().pool; }
+cudaStream_t spc5cuda::alloc_stream() { return device_memory().stream; }
+
+void spc5cuda::wait_device() {
+    void* p = nullptr;
+    if (cudaMalloc(&p, 16) == cudaSuccess) cudaFree(p);
+    else cudaDeviceSynchronize();
 }
 
 namespace {
@@ -382,21 +402,18 @@ spc5cuda_status spc5cuda_convert(spc5cuda_mat* m, int format, void* stream) {
         const size_t stride = 4 + size_t(r) * mask_bytes_of(m->value_type);
         Owned headers, values, valptr;
         headers.alloc(stride * size_t(nb));
-        values.alloc(size_t(value_bytes_of(m->value_type)) * size_t(m->nnz));
+        // at r = 1 the block order is the CSR order: the values stay where they are
+        if (r > 1) values.alloc(size_t(value_bytes_of(m->value_type)) * size_t(m->nnz));
         valptr.alloc(sizeof(int) * size_t(nbr + 1));
         launch_emit(vs_of(m->value_type), r, m->nrows, m->rowptr.as<int>(), m->colidx.as<int>(),
                     m->values.p, value_bytes_of(m->value_type), brptr.as<int>(),
                     headers.as<uint8_t>(), values.p, s);
         launch_valptr_from_csr(r, m->nrows, m->rowptr.as<int>(), valptr.as<int>(), s);
         SPC5_CUDA(cudaStreamSynchronize(s));
-        std::swap(m->brptr.p, brptr.p);
-        std::swap(m->brptr.bytes, brptr.bytes);
-        std::swap(m->headers.p, headers.p);
-        std::swap(m->headers.bytes, headers.bytes);
-        std::swap(m->values.p, values.p);
-        std::swap(m->values.bytes, values.bytes);
-        std::swap(m->valptr.p, valptr.p);
-        std::swap(m->valptr.bytes, valptr.bytes);
+        m->brptr = std::move(brptr);
+        m->headers = std::move(headers);
+        if (r > 1) m->values = std::move(values);
+        m->valptr = std::move(valptr);
         m->rowptr.release();
         m->colidx.release();
         m->r = r;

@@ -10,9 +10,11 @@
 //   pass 2  headers + values of block-row br at brptr[br] and at the CSR
 //           value offset rowptr[br*r]                    (k_emit)
 // Inside a block-row the greedy is a sequential chain (the next block starts
-// at the smallest unconsumed column of the r sub-rows), so one thread walks
-// one block-row; block-rows are independent and run in parallel.  Values are
-// copied bit for bit, so the arrays equal the reference's exactly.
+// at the smallest unconsumed column of the r sub-rows); block-rows are
+// independent.  At r = 1 a warp resolves 32 entries at a time (row_windows); at
+// r > 1 one lane walks a short block-row and a warp a long one.  Values are
+// copied bit for bit (at r = 1 they stay where they are), so the arrays equal
+// the reference's exactly.
 #include <climits>
 
 #include "common.cuh"
@@ -142,30 +144,47 @@ void exclusive_scan_i32(const int* in, int* out, long n, int* tmp, cudaStream_t 
 
 namespace {
 
-__global__ void k_validate_csr(int nrows, int ncols, long nnz, const int* __restrict__ rowptr,
-                               const int* __restrict__ colidx, int* __restrict__ flag) {
-    const long stride = long(gridDim.x) * blockDim.x;
+// Threads per CTA of the kernels that give a warp 32 rows: few, so that a CTA
+// does not wait long for the warp with the most entries.
+constexpr int ROW_THREADS = 64;
+
+// One warp per 32 rows: their entries are one range, read 32 at a time.  A
+// column must exceed the one before it unless an entry starts a row.  (One
+// thread per row before: 600 us on a power-law matrix of 15M entries, bound by
+// its longest rows; now 116 us on a B200.)
+__global__ void __launch_bounds__(ROW_THREADS) k_validate_csr(int nrows, int ncols, long nnz,
+                                                      const int* __restrict__ rowptr,
+                                                      const int* __restrict__ colidx, int* __restrict__ flag) {
+    const int lane = threadIdx.x & 31;
+    const long warps = long(gridDim.x) * blockDim.x / 32;
     const long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
     if (tid == 0 && (rowptr[0] != 0 || long(rowptr[nrows]) != nnz)) atomicMax(flag, 1);
-    for (long i = tid; i < nrows; i += stride) {
-        const int a = rowptr[i], b = rowptr[i + 1];
-        if (b < a || a < 0 || long(b) > nnz) {
-            atomicMax(flag, 1);
+    for (long r0 = tid / 32 * 32; r0 < nrows; r0 += warps * 32) {  // warp-uniform
+        const long row = r0 + lane;
+        const bool in = row < nrows;
+        const int a = in ? rowptr[row] : 0, b = in ? rowptr[row + 1] : 0;
+        const bool bad = in && (b < a || a < 0 || long(b) > nnz);
+        if (__any_sync(0xffffffffu, bad)) {  // the range cannot be trusted
+            if (bad) atomicMax(flag, 1);
             continue;
         }
-        int prev = -1;
-        for (int k = a; k < b; ++k) {
-            const int c = colidx[k];
-            if (c < 0 || c >= ncols) {
-                atomicMax(flag, 2);
-                break;
+        const int last = int(min(long(31), nrows - 1 - r0));
+        const long k0 = __shfl_sync(0xffffffffu, a, 0), k1 = __shfl_sync(0xffffffffu, b, last);
+        int worst = 0, before = -1;  // before: the last column of the previous 32
+        int ahead = k0 + lane < k1 ? colidx[k0 + lane] : 0;
+        for (long k = k0; k < k1; k += 32) {
+            const int c = ahead;
+            ahead = k + 32 + lane < k1 ? colidx[k + 32 + lane] : 0;
+            const unsigned starts = __reduce_or_sync(0xffffffffu, in && a >= k && a - k < 32 ? 1u << (a - k) : 0u);
+            int prev = __shfl_up_sync(0xffffffffu, c, 1);
+            if (lane == 0) prev = before;
+            if (k + lane < k1) {
+                if (c < 0 || c >= ncols) worst = max(worst, 2);
+                else if (!((starts >> lane) & 1u) && c <= prev) worst = max(worst, 3);
             }
-            if (c <= prev) {
-                atomicMax(flag, 3);
-                break;
-            }
-            prev = c;
+            before = __shfl_sync(0xffffffffu, c, 31);
         }
+        if (worst) atomicMax(flag, worst);
     }
 }
 
@@ -174,9 +193,7 @@ __global__ void k_validate_csr(int nrows, int ncols, long nnz, const int* __rest
 void launch_validate_csr(int nrows, int ncols, long nnz, const int* rowptr, const int* colidx,
                          int* d_flag, cudaStream_t s) {
     SPC5_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
-    const int threads = 256;
-    const int blocks = nrows > 0 ? std::min(div_up(nrows, threads), sm_count() * 8) : 1;
-    k_validate_csr<<<blocks, threads, 0, s>>>(nrows, ncols, nnz, rowptr, colidx, d_flag);
+    k_validate_csr<<<std::max(1, div_up(nrows, ROW_THREADS)), ROW_THREADS, 0, s>>>(nrows, ncols, nnz, rowptr, colidx, d_flag);
     SPC5_CUDA(cudaGetLastError());
 }
 
@@ -186,45 +203,102 @@ void launch_validate_csr(int nrows, int ncols, long nnz, const int* rowptr, cons
 
 namespace {
 
+// A block-row of more than LONG_ENTRIES entries is walked by its whole warp
+// (long_blocks), a shorter one by its own lane.  Headers and values on a B200,
+// by lanes / by warps: stencil 100^3, r = 4 (108 entries) 1328 us / 361, r = 2 (54)
+// 1216 / 622; Poisson 64^2, r = 8 (40, with few warps to share them) 26 / 79.
+constexpr int LONG_ENTRIES = 48;
+
+// The greedy over block-row br by one warp: L = 32 / R lanes per sub-row hold
+// its next L columns.  Calls block(index, first column) per block, and per
+// step put(sub-row's entry, bit, lane takes part) for the entries that go to
+// that block; the lanes of a sub-row advance together.
+template <int VS, int R, class B, class P>
+__device__ __forceinline__ void long_blocks(int nrows, long br, const int* __restrict__ rowptr,
+                                            const int* __restrict__ colidx, B&& block, P&& put) {
+    constexpr int L = 32 / R;
+    constexpr unsigned LMASK = (1u << L) - 1u;
+    const int lane = threadIdx.x & 31;
+    const int s = lane / L, t = lane % L;
+    const long row = br * R + s;
+    int head = row < nrows ? rowptr[row] : 0;
+    const int end = row < nrows ? rowptr[row + 1] : 0;
+    int c = t < end - head ? __ldg(colidx + head + t) : INT_MAX;
+    for (int n = 0;; ++n) {
+        const int idx = __reduce_min_sync(0xffffffffu, c);  // a sub-row's columns ascend: its lane 0 has its least
+        if (idx == INT_MAX) break;
+        block(n, idx);
+        for (;;) {
+            const bool take = c != INT_MAX && c - idx < VS;
+            const unsigned all = __ballot_sync(0xffffffffu, take);
+            if (all == 0u) break;
+            const int k = __popc((all >> (s * L)) & LMASK);  // a prefix of the sub-row's lanes
+            put(head + t, c - idx, take, s);
+            if (k > 0) {
+                head += k;
+                c = t < end - head ? __ldg(colidx + head + t) : INT_MAX;
+            }
+        }
+    }
+}
+
 template <int VS, int R>
 __global__ void __launch_bounds__(256) k_blockrow_counts(int nrows, int nbr,
                                                          const int* __restrict__ rowptr,
                                                          const int* __restrict__ colidx,
                                                          int* __restrict__ counts) {
-    for (long br = long(blockIdx.x) * blockDim.x + threadIdx.x; br < nbr;
-         br += long(gridDim.x) * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (long b0 = (long(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; b0 < nbr;
+         b0 += long(gridDim.x) * blockDim.x) {  // warp-uniform
+        const long br = b0 + lane;
         const long row0 = br * R;
         int head[R], end[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const bool ok = row0 + i < nrows;
+            const bool ok = br < nbr && row0 + i < nrows;
             head[i] = ok ? rowptr[row0 + i] : 0;
             end[i] = ok ? rowptr[row0 + i + 1] : 0;
         }
-        int cnt = 0;
-        for (;;) {
-            bool have = false;
-            int idx = INT_MAX;
+        int entries = 0;
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                if (head[i] < end[i]) {
-                    have = true;
-                    idx = min(idx, __ldg(colidx + head[i]));
+        for (int i = 0; i < R; ++i) entries += end[i] - head[i];
+        const bool by_warp = entries > LONG_ENTRIES;
+        int cnt = 0;
+        if (!by_warp) {
+            for (;;) {
+                bool have = false;
+                int idx = INT_MAX;
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    if (head[i] < end[i]) {
+                        have = true;
+                        idx = min(idx, __ldg(colidx + head[i]));
+                    }
+                }
+                if (!have) break;
+                ++cnt;
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    // columns inside a row ascend, so col >= idx: col < idx + VS
+                    // is col - idx < VS without the int overflow of idx + VS
+                    while (head[i] < end[i] && __ldg(colidx + head[i]) - idx < VS) ++head[i];
                 }
             }
-            if (!have) break;
-            ++cnt;
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                // columns inside a row ascend, so col >= idx: col < idx + VS
-                // is col - idx < VS without the int overflow of idx + VS
-                while (head[i] < end[i] && __ldg(colidx + head[i]) - idx < VS) ++head[i];
-            }
         }
-        counts[br] = cnt;
+        unsigned todo = __ballot_sync(0xffffffffu, by_warp);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            int n = 0;
+            long_blocks<VS, R>(nrows, b0 + l, rowptr, colidx, [&](int k, int) { n = k + 1; },
+                               [](int, int, bool, int) {});
+            if (lane == l) cnt = n;
+        }
+        if (br < nbr) counts[br] = cnt;
     }
 }
 
+// Headers of every block-row, and its values in block order.
 template <int VS, int R, class V>
 __global__ void __launch_bounds__(256) k_emit(int nrows, int nbr, const int* __restrict__ rowptr,
                                               const int* __restrict__ colidx,
@@ -233,47 +307,221 @@ __global__ void __launch_bounds__(256) k_emit(int nrows, int nbr, const int* __r
                                               uint8_t* __restrict__ headers, V* __restrict__ vout) {
     constexpr int MB = VS == 8 ? 1 : 2;
     constexpr int STRIDE = 4 + R * MB;
-    for (long br = long(blockIdx.x) * blockDim.x + threadIdx.x; br < nbr;
-         br += long(gridDim.x) * blockDim.x) {
+    constexpr int L = 32 / R;
+    const int lane = threadIdx.x & 31;
+    for (long b0 = (long(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; b0 < nbr;
+         b0 += long(gridDim.x) * blockDim.x) {  // warp-uniform
+        const long br = b0 + lane;
         const long row0 = br * R;
         int head[R], end[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const bool ok = row0 + i < nrows;
+            const bool ok = br < nbr && row0 + i < nrows;
             head[i] = ok ? rowptr[row0 + i] : 0;
             end[i] = ok ? rowptr[row0 + i + 1] : 0;
         }
-        long vo = rowptr[row0];
-        uint8_t* h = headers + long(brptr[br]) * STRIDE;
-        for (;;) {
-            bool have = false;
-            int idx = INT_MAX;
+        int entries = 0;
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                if (head[i] < end[i]) {
-                    have = true;
-                    idx = min(idx, __ldg(colidx + head[i]));
-                }
-            }
-            if (!have) break;
-            h[0] = uint8_t(idx);
-            h[1] = uint8_t(idx >> 8);
-            h[2] = uint8_t(idx >> 16);
-            h[3] = uint8_t(idx >> 24);
+        for (int i = 0; i < R; ++i) entries += end[i] - head[i];
+        const bool by_warp = entries > LONG_ENTRIES;
+        if (!by_warp && entries > 0) {
+            long vo = head[0];
+            uint8_t* h = headers + long(brptr[br]) * STRIDE;
+            for (;;) {
+                bool have = false;
+                int idx = INT_MAX;
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                uint32_t m = 0;
-                while (head[i] < end[i]) {
-                    const int d = __ldg(colidx + head[i]) - idx;
-                    if (d >= VS) break;
-                    vout[vo++] = vin[head[i]];
-                    m |= 1u << d;
-                    ++head[i];
+                for (int i = 0; i < R; ++i) {
+                    if (head[i] < end[i]) {
+                        have = true;
+                        idx = min(idx, __ldg(colidx + head[i]));
+                    }
                 }
-                h[4 + i * MB] = uint8_t(m);
-                if (MB == 2) h[5 + i * MB] = uint8_t(m >> 8);
+                if (!have) break;
+                h[0] = uint8_t(idx);
+                h[1] = uint8_t(idx >> 8);
+                h[2] = uint8_t(idx >> 16);
+                h[3] = uint8_t(idx >> 24);
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    uint32_t m = 0;
+                    while (head[i] < end[i]) {
+                        const int d = __ldg(colidx + head[i]) - idx;
+                        if (d >= VS) break;
+                        vout[vo++] = vin[head[i]];
+                        m |= 1u << d;
+                        ++head[i];
+                    }
+                    h[4 + i * MB] = uint8_t(m);
+                    if (MB == 2) h[5 + i * MB] = uint8_t(m >> 8);
+                }
+                h += STRIDE;
             }
-            h += STRIDE;
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, by_warp);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            const long b = b0 + l;
+            uint8_t* h = headers + long(brptr[b]) * STRIDE;
+            // a block's masks are complete when the next block begins; the
+            // values of its sub-rows follow one another
+            const int s = lane / L;
+            long vo = rowptr[b * R];  // the block's first value
+            uint32_t mask = 0u;       // of the lane's sub-row
+            int first = 0;            // the sub-row's first entry in this block
+            auto close = [&]() {
+                if (lane % L == 0) {
+                    h[4 + s * MB] = uint8_t(mask);
+                    if (MB == 2) h[5 + s * MB] = uint8_t(mask >> 8);
+                }
+                // values of the sub-rows up to this one, of the whole block
+                const int n = __popc(mask);
+                int upto = n;
+#pragma unroll
+                for (int d = L; d < 32; d <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, upto, d);
+                    if (lane >= d) upto += u;
+                }
+                for (int k = lane % L; k < n; k += L) vout[vo + upto - n + k] = vin[first + k];
+                vo += __shfl_sync(0xffffffffu, upto, 31);
+                h += STRIDE;
+                mask = 0u;
+            };
+            bool open = false;
+            long_blocks<VS, R>(nrows, b, rowptr, colidx,
+                               [&](int, int idx) {
+                                   if (open) close();
+                                   open = true;
+                                   if (lane < 4) h[lane] = uint8_t(uint32_t(idx) >> (8 * lane));
+                               },
+                               [&](int entry, int d, bool take, int) {
+                                   // the sub-row's lanes agree on its mask; its first entry
+                                   // is the one its lane 0 takes first
+                                   const int e0 = __shfl_sync(0xffffffffu, entry, lane / L * L);
+                                   if (mask == 0u) first = e0;
+                                   uint32_t m = take ? 1u << d : 0u;
+#pragma unroll
+                                   for (int x = L / 2; x >= 1; x >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, x);
+                                   mask |= m;
+                               });
+            if (open) close();
+        }
+    }
+}
+
+// r = 1: a warp takes 32 rows, whose entries are one range, 32 at a time.
+// Every row's first entry starts a block; from there block starts follow from
+// one another, entry p's next block being at the first entry of the row past
+// column + VS.  All 32 successors are found at once, and the starts reachable
+// from the window's (its first entry, the rows' first ones, entries VS or more
+// past the one before) by doubling.  A
+// window ends before its last block unless nothing follows, so that its blocks
+// are complete.  Calls put(window's first entry, its blocks, the starts, the
+// lane's column, one past the entries of the block that the lane's entry would
+// start).
+//
+// One lane per row (and a warp per long row) was bound by the chain of one
+// row's loads: power-law, 1M rows, 15M entries, counts 538 us and headers
+// 910 us on a B200; now 191 and 238.
+template <int VS, class P>
+__device__ __forceinline__ void row_windows(int a, int b, bool in, long k0, long k1, const int* __restrict__ colidx,
+                                            P&& put) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    // columns of entries [q, q + 32), the next 32 and the 32 after those
+    long q = k0;
+    auto load = [&](long at) { return at + lane < k1 ? __ldg(colidx + at + lane) : 0; };
+    int c0 = load(q), c1 = load(q + 32), c2 = load(q + 64);
+    for (long k = k0; k < k1;) {
+        const int n = int(min(32L, k1 - k));
+        if (k - q >= 32) {
+            q += 32;
+            c0 = c1;
+            c1 = c2;
+            c2 = load(q + 64);
+        }
+        const int off = int(k - q) + lane;
+        const int lo = __shfl_sync(FULL, c0, off & 31), hi = __shfl_sync(FULL, c1, off & 31);
+        const int c = off < 32 ? lo : hi;
+        const unsigned row_starts = __reduce_or_sync(FULL, in && a < b && a >= k && a - k < n ? 1u << (a - k) : 0u);
+        const unsigned above = lane == 31 ? 0u : row_starts & (FULL << (lane + 1));
+        const int row_end = above ? __ffs(above) - 1 : n;  // of the lane's row, in this window
+        int last = lane;                                   // the block's last entry
+#pragma unroll
+        for (int d = VS / 2; d >= 1; d >>= 1) {
+            const int cc = __shfl_sync(FULL, c, (last + d) & 31);
+            if (last + d < row_end && cc - c < VS) last += d;
+        }
+        const int before = __shfl_up_sync(FULL, c, 1);
+        unsigned starts = row_starts | 1u | __ballot_sync(FULL, lane > 0 && lane < row_end && c - before >= VS);
+        int jump = last + 1;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const unsigned more =
+                starts | __reduce_or_sync(FULL, ((starts >> lane) & 1u) && jump < n ? 1u << jump : 0u);
+            if (more == starts) break;  // closed under this many steps and so under all
+            starts = more;
+            const int next = __shfl_sync(FULL, jump, jump & 31);
+            jump = jump < n ? next : 32;
+        }
+        int used = n;
+        if (k + n < k1) {  // a full window: its last start is not its first
+            used = 31 - __clz(starts);
+            starts ^= 1u << used;
+        }
+        put(k, starts, c, last + 1);
+        k += used;
+    }
+}
+
+__device__ __forceinline__ unsigned bits_below(long n) {
+    return n <= 0 ? 0u : (n >= 32 ? 0xffffffffu : (1u << int(n)) - 1u);
+}
+
+// EMIT: the headers at brptr, else the blocks per row.
+template <int VS, bool EMIT>
+__global__ void __launch_bounds__(ROW_THREADS) k_rows1(int nrows, const int* __restrict__ rowptr,
+                                               const int* __restrict__ colidx, const int* __restrict__ brptr,
+                                               int* __restrict__ counts, uint8_t* __restrict__ headers) {
+    constexpr int MB = VS == 8 ? 1 : 2;
+    constexpr int STRIDE = 4 + MB;
+    const int lane = threadIdx.x & 31;
+    const long warps = long(gridDim.x) * blockDim.x / 32;
+    for (long r0 = (long(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; r0 < nrows; r0 += warps * 32) {
+        const long row = r0 + lane;
+        const bool in = row < nrows;
+        const int a = in ? rowptr[row] : 0, b = in ? rowptr[row + 1] : 0;
+        const int last = int(min(31L, nrows - 1 - r0));
+        const long k0 = __shfl_sync(0xffffffffu, a, 0), k1 = __shfl_sync(0xffffffffu, b, last);
+        if constexpr (EMIT) {
+            long at = brptr[r0];
+            row_windows<VS>(a, b, in, k0, k1, colidx, [&](long, unsigned starts, int c, int end) {
+                const bool mine = (starts >> lane) & 1u;
+                const int len = mine ? end - lane : 0;
+                const int longest = __reduce_max_sync(0xffffffffu, len);
+                uint32_t m = 1u;
+                for (int d = 1; d < longest; ++d) {
+                    const int cc = __shfl_down_sync(0xffffffffu, c, d);
+                    if (d < len) m |= 1u << (cc - c);
+                }
+                if (mine) {
+                    uint8_t* h = headers + (at + __popc(starts & bits_below(lane))) * STRIDE;
+                    h[0] = uint8_t(c);
+                    h[1] = uint8_t(c >> 8);
+                    h[2] = uint8_t(c >> 16);
+                    h[3] = uint8_t(c >> 24);
+                    h[4] = uint8_t(m);
+                    if (MB == 2) h[5] = uint8_t(m >> 8);
+                }
+                at += __popc(starts);
+            });
+        } else {
+            int cnt = 0;
+            row_windows<VS>(a, b, in, k0, k1, colidx, [&](long k, unsigned starts, int, int) {
+                cnt += __popc(starts & bits_below(b - k) & ~bits_below(a - k));
+            });
+            if (in) counts[row] = cnt;
         }
     }
 }
@@ -308,7 +556,10 @@ void counts_r(int nrows, const int* rowptr, const int* colidx, int* counts, cuda
     const int nbr = div_up(nrows, R);
     const int threads = 256;
     const int blocks = std::max(1, std::min(div_up(nbr, threads), sm_count() * 16));
-    k_blockrow_counts<VS, R><<<blocks, threads, 0, s>>>(nrows, nbr, rowptr, colidx, counts);
+    if constexpr (R == 1)
+        k_rows1<VS, false><<<div_up(nrows, ROW_THREADS), ROW_THREADS, 0, s>>>(nrows, rowptr, colidx, nullptr, counts, nullptr);
+    else
+        k_blockrow_counts<VS, R><<<blocks, threads, 0, s>>>(nrows, nbr, rowptr, colidx, counts);
 }
 
 template <int VS, int R, class V>
@@ -317,9 +568,11 @@ void emit_r(int nrows, const int* rowptr, const int* colidx, const void* vin, co
     const int nbr = div_up(nrows, R);
     const int threads = 256;
     const int blocks = std::max(1, std::min(div_up(nbr, threads), sm_count() * 16));
-    k_emit<VS, R, V><<<blocks, threads, 0, s>>>(nrows, nbr, rowptr, colidx,
-                                               static_cast<const V*>(vin), brptr, headers,
-                                               static_cast<V*>(vout));
+    if constexpr (R == 1)
+        k_rows1<VS, true><<<div_up(nrows, ROW_THREADS), ROW_THREADS, 0, s>>>(nrows, rowptr, colidx, brptr, nullptr, headers);
+    else
+        k_emit<VS, R, V><<<blocks, threads, 0, s>>>(nrows, nbr, rowptr, colidx, static_cast<const V*>(vin), brptr,
+                                                    headers, static_cast<V*>(vout));
 }
 
 }  // namespace

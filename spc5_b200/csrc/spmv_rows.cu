@@ -41,7 +41,7 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "kernels.h"
+#include "handle.h"
 #include "rows_blocks.cuh"
 
 namespace spc5cuda {
@@ -270,12 +270,10 @@ void enqueue_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, 
 
 RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
                    cudaStream_t s) {
-    int* d = nullptr;
-    SPC5_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d), 4 * sizeof(int), s));
-    enqueue_stats(vt, r, nbr, brptr, valptr, headers, d, s);
+    PoolBuf d(4 * sizeof(int), s);
+    enqueue_stats(vt, r, nbr, brptr, valptr, headers, d.as<int>(), s);
     int h[4] = {0, 0, 0, 0};
-    SPC5_CUDA(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
-    SPC5_CUDA(cudaFreeAsync(d, s));
+    SPC5_CUDA(cudaMemcpyAsync(h, d.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     SPC5_CUDA(cudaStreamSynchronize(s));
     return RowStats{rows_fit(vt, r, h[0], h[1]), rows_narrow(h[2], h[3])};
 }
