@@ -413,8 +413,12 @@ void build_sorted_plan(spc5cuda_mat* m, cudaStream_t s) {
     SPC5_CUDA(cudaStreamSynchronize(s));
     m->plan = std::move(plan);
     // the streams serve every SpMV now: the reference-order values are put
-    // back together when a call needs them (restore_values)
-    if (m->use_plan()) {
+    // back together when a call needs them (restore_values), if the rows hold
+    // all of them (the caller's arrays may hold more: values of the rows past
+    // the last one of a block-row that is not full, or past the masks')
+    long held = m->plan->long_values;
+    for (int n = 0; n <= SHORT_VALUES; ++n) held += long(n) * m->plan->short_rows[n];
+    if (m->use_plan() && held == m->nnz) {
         m->values.release();
         m->values_dropped = true;
     }

@@ -123,3 +123,22 @@ def test_streams_in_order_and_captured(cuda, k):
         g.replay()
     torch.cuda.synchronize()
     assert got().tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("r", [2, 8])
+def test_values_outside_the_rows_are_kept(cuda, r):
+    """Arrays of the caller's own whose last block-row has values in the rows
+    past nrows: the product leaves them out, the arrays still hold them."""
+    n = 40 * r
+    csr = rows_matrix([3] * n, 1, 8)
+    ob, oh, ov = oracle.csr_to_beta(r, csr.rowptr, csr.colidx, csr.values)
+    m = S.beta_matrix(r, n - 1, csr.ncols, ob, oh, ov)
+    m.set_kernel(S.KERNEL_SORTED)
+    gb, gh, gv = m.arrays()
+    assert np.array_equal(gb, ob) and np.array_equal(gh, oh) and gv.tobytes() == ov.tobytes()
+    x = M.x_vector(csr.ncols, 3)
+    y = dev(np.zeros(n - 1))
+    S.SPC5_Spmv(m, dev(x), y)
+    torch.cuda.synchronize()
+    yo = oracle.beta_spmv_f64(r, n, ob, oh, ov, x, np.zeros(n))[:n - 1]
+    assert y.cpu().numpy().tobytes() == yo.tobytes()
