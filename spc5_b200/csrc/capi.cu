@@ -123,12 +123,11 @@ void spc5cuda::wait_device() {
 namespace {
 
 // core_SPC5_{r}rVc_Spmv_{double,float} over device arrays without a handle.
-// Per call, all on the stream and without a host round trip: the value
-// offsets of the block-rows (one pass over the headers), the largest
-// block-row, the per-group and per-warp splits; then the two instantiations of
-// the row kernel and the group kernel are enqueued, gated on a device word: a
-// row kernel runs when every block-row fits its staging buffers, the group
-// kernel otherwise.  All give the reference's bits.
+// Per call, all on the stream and without a host round trip: what the kernels
+// must know about the arrays (core_prep.cu); then the two instantiations of the
+// row kernel and the group kernel are enqueued, gated on a device word: a row
+// kernel runs when every block-row fits its staging buffers, the group kernel
+// otherwise.  All give the reference's bits.
 template <class T>
 void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* headers,
                const T* values, const T* x, T* y, cudaStream_t s) {
@@ -143,18 +142,10 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     const int nbr = div_up(nbRows, r);
     const int ngroups = spmv_groups(vs_of(vt), r);
     const int nwarps = rows_warps(vt, r, true);  // one wave of either instantiation, about
-    PoolBuf valptr(sizeof(int) * size_t(nbr + 1), s);
-    PoolBuf gstart(sizeof(int) * size_t(ngroups + 1), s);
-    PoolBuf wstart(sizeof(int) * size_t(nwarps + 1), s);
-    PoolBuf work(sizeof(int) * 5, s);
-    {
-        PoolBuf tmp(sizeof(int) * size_t(scan_tmp_ints(nbr) + 1), s);
-        launch_blockrow_value_counts(mask_bytes_of(vt), r, nbr, rowsSizes, headers, valptr.as<int>(), s);
-        exclusive_scan_i32(valptr.as<int>(), valptr.as<int>(), nbr, tmp.as<int>(), s);
-    }
-    launch_partition(nbr, rowsSizes, ngroups, gstart.as<int>(), s);
-    launch_partition(nbr, rowsSizes, nwarps, wstart.as<int>(), s);
-    launch_rows_fit_flag(vt, r, nbr, rowsSizes, valptr.as<int>(), headers, work.as<int>(), s);
+    const CoreScratch at = core_scratch(nbr, ngroups, nwarps);
+    PoolBuf scratch(at.bytes, s);
+    unsigned char* mem = scratch.as<unsigned char>();
+    launch_core_prep(vt, r, nbr, rowsSizes, headers, ngroups, nwarps, at, mem, s);
     BetaView v;
     v.r = r;
     v.nrows = int(nbRows);
@@ -162,15 +153,17 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     v.brptr = rowsSizes;
     v.headers = headers;
     v.values = values;
-    v.valptr = valptr.as<int>();
-    v.gstart = gstart.as<int>();
+    v.valptr = reinterpret_cast<int*>(mem + at.valptr);
+    v.gstart = reinterpret_cast<int*>(mem + at.gstart);
     v.ngroups = ngroups;
-    v.run_if = work.as<int>();
+    v.run_if = reinterpret_cast<int*>(mem + at.flag);
+    v.follows = true;
     BetaView vr = v;
-    vr.wstart = wstart.as<int>();
+    vr.wstart = reinterpret_cast<int*>(mem + at.wstart);
     vr.nwarps = nwarps;
     BetaView vn = vr;
     vn.narrow = true;
+    vn.follows = false;  // the splits are complete before any of the three begins
     v.run_if_value = 0;   // group kernel: some block-row does not fit
     vr.run_if_value = 1;  // row kernel: every block-row fits
     vn.run_if_value = 2;  // and the masks are narrow

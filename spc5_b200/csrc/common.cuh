@@ -67,9 +67,52 @@ int resident_ctas(K kern, int threads, int smem) {
     return n > 0 ? n : 1;
 }
 
+// Lets kern use bytes of dynamic shared memory (48 KB need no leave).
+template <class K>
+void set_smem(K kern, int bytes) {
+    if (bytes > 48 * 1024)
+        SPC5_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
+// Launches kern.  follows: it may become resident before the previous launch on
+// s ends, as soon as every CTA of that one has run launch_dependents or ended;
+// it orders itself by griddepcontrol.wait.
+template <class... P, class... Q>
+void launch_after(void (*kern)(P...), dim3 grid, int threads, int smem, bool follows, cudaStream_t s, Q... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = size_t(smem);
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = follows ? 1 : 0;
+    SPC5_CUDA(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+}
+
 // ---------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------
+
+// The split of nbr block-rows (nblocks blocks) into n parts of about the same
+// number of blocks, as far as block-row row (0 .. nbr) decides it: part p
+// begins at the first block-row whose first block lies in
+// [p nblocks / n, (p + 1) nblocks / n); start[n] = nbr.
+__device__ __forceinline__ void split_at(int row, int nbr, const int* __restrict__ brptr, long nblocks, int n,
+                                         int* __restrict__ start) {
+    // part of a block-row (nbr -> n); the parts in (part(row - 1), part(row)] begin at row
+    auto part = [&](int q) -> long {
+        if (q >= nbr) return n;
+        if (nblocks == 0) return 0;
+        const long p = (long(brptr[q]) * n) / nblocks;
+        return p < n ? p : n - 1;
+    };
+    const long hi = part(row);
+    const long lo = row == 0 ? -1 : part(row - 1);
+    for (long p = lo + 1; p <= hi && p <= n; ++p) start[p] = row;
+}
 
 // Decode the packed header of block b: returns the column and the mask bytes
 // as little-endian 32-bit words (mask byte j in bits 8*(j%4) of mw[j/4]).

@@ -294,7 +294,7 @@ struct spc5cuda_mat {
         gstart.alloc(sizeof(int) * size_t(ngroups + 1));
         spc5cuda::launch_partition(nbr(), brptr.as<int>(), ngroups, gstart.as<int>(), s);
         const spc5cuda::RowStats stats = spc5cuda::row_stats(value_type, r, nbr(), brptr.as<int>(), valptr.as<int>(),
-                                                             headers.as<uint8_t>(), s);
+                                                             headers.as<uint8_t>(), nblocks, s);
         rows_ok = stats.fits;
         rows_narrow = stats.narrow;
         if (rows_ok) {

@@ -61,6 +61,7 @@ struct BetaView {
 
 // Number of VS-lane groups the SpMV kernels launch on the current device
 // for rows-per-block r: one wave of resident CTAs.
+    bool follows = false;  // may become resident before the launch before it ends (run_if launches wait for it)
 int spmv_groups(int vs, int r);
 
 // gstart[0..ngroups] = block-row ranges holding ~nblocks/ngroups blocks each.
@@ -73,19 +74,24 @@ void launch_spmv_f64(const BetaView& m, const double* x, double* y, cudaStream_t
 // staging buffers, and what a converted matrix asks of it (synchronises s).
 // (vt: the handle's value type, SPC5CUDA_F64 / F32 / F32_V8.)
 int rows_warps(int vt, int r, bool narrow);
-bool rows_fit(int vt, int r, int max_blocks, int max_values);
 struct RowStats {
     bool fits;    // every block-row fits the row kernel's buffers
     bool narrow;  // most blocks' sub-row masks span few columns
 };
 // (headers may be null: narrow is not asked for.)
 RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
-                   cudaStream_t s);
-// The same on the device, without a host round trip: work[0] = 0 when some
+                   long nblocks, cudaStream_t s);
+// What the drop-in symbols find out about bare arrays, without a host round
+// trip (core_prep.cu): byte offsets in a 256-byte aligned scratch block of
+// valptr, gstart and wstart (as in BetaView) and of flag = 0 when some
 // block-row does not fit the row kernel's buffers, else 1 for its wide, 2 for
-// its narrow instantiation (work holds 5 ints).
-void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
-                          int* work, cudaStream_t s);
+// its narrow instantiation.
+struct CoreScratch {
+    size_t valptr, stats, before, gstart, wstart, flag, bytes;
+};
+CoreScratch core_scratch(int nbr, int ngroups, int nwarps);
+void launch_core_prep(int value_type, int r, int nbr, const int* brptr, const uint8_t* headers, int ngroups, int nwarps,
+                      const CoreScratch& c, unsigned char* mem, cudaStream_t s);
 // The row SpMV of a kind (below).
 void launch_rows_kind(int kind, const BetaView& m, const void* x, void* y, cudaStream_t s);
 void launch_rows_f64(const BetaView& m, const double* x, double* y, cudaStream_t s);

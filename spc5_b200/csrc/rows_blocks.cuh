@@ -104,6 +104,23 @@ __device__ __forceinline__ void wide_blocks(const uint32_t* hw, const V* vbuf, c
 // A window of NS columns, from the first column of the sub-row's first
 // non-empty mask on: accumulator a is column (rho + a) mod VS.
 constexpr int NS = 3;
+
+// Whether every block-row alone fits a warp's staging buffers, alignment included.
+__host__ __device__ inline bool fit(int vt, int r, int max_blocks, int max_values) {
+    const int stride = 4 + r * (vt == SPC5CUDA_F32 ? 2 : 1);
+    const int vbytes = vt == SPC5CUDA_F64 ? 8 : 4;
+    return long(max_blocks) * stride + 32 <= HB && (long(max_values) + 2 * (16 / vbytes)) * vbytes <= VB;
+}
+
+// Whether the narrow kernel runs: at least 7 of 8 of the blocks looked at keep
+// every sub-row mask within NS columns.  At r = VS its steps of 3 blocks pay for
+// themselves only on block-rows of several steps (measured on B200, FP64, wide /
+// narrow us: 27-point stencil 127^3, 18 blocks per block-row, 234 / 181; 5-point
+// Poisson 900^2, 4 blocks, 29.4 / 31.5).
+__host__ __device__ inline bool narrow(int vt, int r, int nbr, long nblocks, int narrow_blocks, int looked_at) {
+    const int vs = vt == SPC5CUDA_F32 ? 16 : 8;
+    return looked_at > 0 && long(narrow_blocks) * 8 >= long(looked_at) * 7 && (r < vs || nblocks >= 6L * nbr);
+}
 template <class LT, int R, class V, class X, class A>
 __device__ __forceinline__ void narrow_blocks(const uint32_t* hw, const V* vbuf, const X* __restrict__ x, int q,
                                               SubRow at, uint64_t pol_x, A (&acc)[Layout<LT>::VS]) {

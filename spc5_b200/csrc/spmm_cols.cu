@@ -313,11 +313,6 @@ __global__ void __launch_bounds__(rows::THREADS, cols_ctas<V, R, KC>(Layout<LT>:
     }
 }
 
-template <class K>
-void set_smem(K kernel, int bytes) {
-    SPC5_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-}
-
 // Calls f(integral_constant<R>, integral_constant<KC>) for r in {4, 8}
 // and kc a power of two up to mm_kc_limit of the kernel's lanes.
 template <class LT, class F>

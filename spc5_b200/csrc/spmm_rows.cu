@@ -315,11 +315,6 @@ __global__ void __launch_bounds__(rows::THREADS, 5)
     }
 }
 
-template <class K>
-void set_smem(K kernel, int bytes) {
-    SPC5_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-}
-
 // Calls f(integral_constant<R>) for r in {1, 2, 4, 8}.
 template <class F>
 void dispatch_r(int r, F&& f) {

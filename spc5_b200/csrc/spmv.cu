@@ -198,8 +198,12 @@ __global__ void __launch_bounds__(128)
            const int* __restrict__ gstart, int ngroups,
            const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
     // a launch gated on a device word: the drop-in symbols enqueue the row
-    // kernel and this one, and exactly one of them does the work
-    if (run_if && __ldg(run_if) != run_if_value) return;
+    // kernels and this one, and exactly one of them does the work; each is
+    // resident early and waits for the one before it
+    if (run_if) {
+        asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+        if (__ldg(run_if) != run_if_value) return;
+    }
     using G = Geo<LT, R, V, A>;
     using F = Fields<G::MB>;
     constexpr int VS = G::VS, MW = G::MW, NW = G::NW, PW = F::PER_WORD;
@@ -471,27 +475,11 @@ __global__ void __launch_bounds__(128)
     if (__any_sync(FULL, ns > 0)) reduce_batch(ns > 0);
 }
 
-// gstart[g] = first block-row whose first block lies in group g's share
-// [g * n / G, (g+1) * n / G) of the n blocks; gstart[G] = nbr.
+// The split of split_at, a thread per block-row.
 __global__ void k_partition(int nbr, const int* __restrict__ brptr, int ngroups, int* __restrict__ gstart) {
     const long nblocks = brptr[nbr];
-    for (long rr = long(blockIdx.x) * blockDim.x + threadIdx.x; rr <= nbr; rr += long(gridDim.x) * blockDim.x) {
-        // bucket of block-row rr (nbr -> G); groups in (bucket(rr-1), bucket(rr)] start at rr
-        auto bucket = [&](long q) -> long {
-            if (q >= nbr) return ngroups;
-            if (nblocks == 0) return 0;
-            const long bk = (long(brptr[q]) * ngroups) / nblocks;
-            return bk < ngroups ? bk : ngroups - 1;
-        };
-        const long hi = bucket(rr);
-        const long lo = rr == 0 ? -1 : bucket(rr - 1);
-        for (long g = lo + 1; g <= hi && g <= ngroups; ++g) gstart[g] = int(rr);
-    }
-}
-
-template <class K>
-void set_smem(K kernel, int bytes) {
-    SPC5_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    for (long rr = long(blockIdx.x) * blockDim.x + threadIdx.x; rr <= nbr; rr += long(gridDim.x) * blockDim.x)
+        split_at(int(rr), nbr, brptr, nblocks, ngroups, gstart);
 }
 
 template <class LT, class V, class X, class A, class Y>
@@ -504,9 +492,9 @@ void launch_impl(const BetaView& m, const X* x, Y* y, cudaStream_t s) {
         const int ctas = (m.ngroups + G::GPC - 1) / G::GPC;                                      \
         auto kern = k_spmv<LT, R_, V, X, A, Y>;                                                  \
         set_smem(kern, G::SMEM);                                                                 \
-        kern<<<ctas, G::THREADS, G::SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr,      \
-                                               m.gstart, m.ngroups, x, y, m.run_if,              \
-                                               m.run_if_value);                                  \
+        launch_after(kern, dim3(unsigned(ctas)), G::THREADS, G::SMEM, m.follows, s, m.nrows,     \
+                     m.brptr, m.headers, vals, m.valptr, m.gstart, m.ngroups, x, y, m.run_if,    \
+                     m.run_if_value);                                                            \
     }
     switch (m.r) {
         case 1: SPC5_LAUNCH(1); break;

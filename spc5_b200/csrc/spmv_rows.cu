@@ -53,11 +53,6 @@ constexpr int ROWS_THREADS = rows::THREADS;
 constexpr int ROWS_WARPS = rows::WARPS;
 constexpr int ROWS_CTAS_PER_SM = 16;
 
-// The narrow kernel runs when at least 7 of 8 sampled blocks are narrow.
-__host__ __device__ inline bool rows_narrow(int narrow, int sampled) {
-    return sampled > 0 && long(narrow) * 8 >= long(sampled) * 7;
-}
-
 // CTAs per SM asked of the compiler.  Wide: 6 (80 registers).  Narrow: 7 (72 registers: the 5-point Poisson
 // 512^2 at r = 2 then takes two chunks per warp instead of three, 8.3 against
 // 9.4 us on the device; 160^3 at r = 4 197 against 203 us), 6 at r = 8, whose
@@ -75,8 +70,12 @@ __global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, A>(NARROW))
     k_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
            const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart, int nwarps,
            const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
-    // a launch gated on a device word (see BetaView::run_if)
-    if (run_if && __ldg(run_if) != run_if_value) return;
+    // a launch gated on a device word (see BetaView::run_if): resident early, it
+    // waits for the launch before it
+    if (run_if) {
+        asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+        if (__ldg(run_if) != run_if_value) return;
+    }
     using G = rows::Geo<LT, R, V, R>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
@@ -93,11 +92,6 @@ __global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, A>(NARROW))
                             [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
                                 chunk_spmv<LT, R, V, X, A, Y, NARROW>(ch, hw, vbuf, x, y, nrows, pol_x);
                             });
-}
-
-template <class K>
-void set_smem(K kernel, int bytes) {
-    SPC5_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
 // Calls f(std::integral_constant<int, R>{}) for r in {1, 2, 4, 8}.
@@ -135,27 +129,14 @@ void launch_rows_impl(const BetaView& m, const X* x, Y* y, cudaStream_t s) {
         using G = rows::Geo<LT, R_, V, R_>;
         auto kern = m.narrow ? k_rows<LT, R_, V, X, A, Y, true> : k_rows<LT, R_, V, X, A, Y, false>;
         set_smem(kern, G::SMEM);
-        kern<<<ctas, ROWS_THREADS, G::SMEM, s>>>(m.nrows, m.brptr, m.headers, vals, m.valptr, m.wstart, m.nwarps, x, y,
-                                                 m.run_if, m.run_if_value);
+        launch_after(kern, dim3(unsigned(ctas)), ROWS_THREADS, G::SMEM, m.follows, s, m.nrows, m.brptr, m.headers, vals,
+                     m.valptr, m.wstart, m.nwarps, x, y, m.run_if, m.run_if_value);
     });
     SPC5_CUDA(cudaGetLastError());
 }
 
-// flag[0] = 0 when a block-row of stats[0] blocks and stats[1] values does not
-// fit the staging buffers (the test of rows_fit, on the device), else 1 for the
-// wide row kernel, 2 for the narrow one (stats[2] of stats[3] sampled blocks).
-__global__ void k_fit_flag(const int* __restrict__ stats, int stride, int vbytes, int hb, int vb,
-                           int* __restrict__ flag) {
-    const long hneed = long(stats[0]) * stride + 32;
-    const long vneed = (long(stats[1]) + 2 * (16 / vbytes)) * vbytes;
-    flag[0] = (hneed <= hb && vneed <= vb) ? (rows_narrow(stats[2], stats[3]) ? 2 : 1) : 0;
-}
-
 // Of at most SAMPLED blocks spread over the matrix: how many, and how many
-// whose every sub-row mask spans at most NS columns.  At r = VS the narrow
-// kernel's steps of 3 blocks pay for themselves only on block-rows of several
-// steps (measured on B200, FP64, wide / narrow us: 27-point stencil 127^3, 18
-// blocks per block-row, 234 / 181; 5-point Poisson 900^2, 4 blocks, 29.4 / 31.5).
+// whose every sub-row mask spans at most NS columns.
 constexpr int SAMPLED = 1 << 15;
 template <class LT, int R>
 __global__ void __launch_bounds__(256) k_narrow_sample(int nbr, const int* __restrict__ brptr,
@@ -164,7 +145,7 @@ __global__ void __launch_bounds__(256) k_narrow_sample(int nbr, const int* __res
     const long step = max(1L, nblocks / SAMPLED);
     const long i = (long(blockIdx.x) * blockDim.x + threadIdx.x) * step;
     const bool in = i < nblocks && i / step < SAMPLED;
-    bool narrow = in && (R < Layout<LT>::VS || nblocks >= 6L * nbr);
+    bool narrow = in;
     if (in) {
         uint32_t mw[Header<LT, R>::MASK_WORDS];
         load_header<LT, R>(headers, i, mw);
@@ -235,56 +216,26 @@ int rows_warps(int vt, int r, bool narrow) {
     return n;
 }
 
-// Staging buffer sizes of RowGeo (every instantiation).
-constexpr int ROWS_HB = rows::HB;
-constexpr int ROWS_VB = rows::VB;
-
-bool rows_fit(int vt, int r, int max_blocks, int max_values) {
-    // every block-row alone must fit the staging buffers, alignment included
-    const int stride = 4 + r * (vt == SPC5CUDA_F32 ? 2 : 1);
-    const int vbytes = vt == SPC5CUDA_F64 ? 8 : 4;
-    const long hneed = long(max_blocks) * stride + 32;
-    const long vneed = (long(max_values) + 2 * (16 / vbytes)) * vbytes;
-    return hneed <= ROWS_HB && vneed <= ROWS_VB;
-}
-
-namespace {
-
-// stats[0], stats[1]: the largest block and value counts of any block-row;
-// stats[2], stats[3]: narrow and all sampled blocks (headers may be null: none).
-void enqueue_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers, int* stats,
-                   cudaStream_t s) {
-    SPC5_CUDA(cudaMemsetAsync(stats, 0, 4 * sizeof(int), s));
-    if (nbr <= 0) return;
-    const int threads = 256;
-    const int blocks = std::max(1, std::min(div_up(nbr, threads), sm_count() * 4));
-    k_blockrow_max<<<blocks, threads, 0, s>>>(nbr, brptr, valptr, stats);
-    if (headers) {
-        if (vt == SPC5CUDA_F32) narrow_sample<float>(r, nbr, brptr, headers, stats + 2, s);
-        else narrow_sample<double>(r, nbr, brptr, headers, stats + 2, s);
-    }
-    SPC5_CUDA(cudaGetLastError());
-}
-
-}  // namespace
-
 RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
-                   cudaStream_t s) {
+                   long nblocks, cudaStream_t s) {
+    // the largest block and value counts of any block-row; narrow and all sampled blocks
     PoolBuf d(4 * sizeof(int), s);
-    enqueue_stats(vt, r, nbr, brptr, valptr, headers, d.as<int>(), s);
+    int* stats = d.as<int>();
+    SPC5_CUDA(cudaMemsetAsync(stats, 0, 4 * sizeof(int), s));
+    if (nbr > 0) {
+        const int threads = 256;
+        const int blocks = std::max(1, std::min(div_up(nbr, threads), sm_count() * 4));
+        k_blockrow_max<<<blocks, threads, 0, s>>>(nbr, brptr, valptr, stats);
+        if (headers) {
+            if (vt == SPC5CUDA_F32) narrow_sample<float>(r, nbr, brptr, headers, stats + 2, s);
+            else narrow_sample<double>(r, nbr, brptr, headers, stats + 2, s);
+        }
+        SPC5_CUDA(cudaGetLastError());
+    }
     int h[4] = {0, 0, 0, 0};
     SPC5_CUDA(cudaMemcpyAsync(h, d.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     SPC5_CUDA(cudaStreamSynchronize(s));
-    return RowStats{rows_fit(vt, r, h[0], h[1]), rows_narrow(h[2], h[3])};
-}
-
-void launch_rows_fit_flag(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
-                          int* work, cudaStream_t s) {
-    enqueue_stats(vt, r, nbr, brptr, valptr, headers, work + 1, s);
-    const int stride = 4 + r * (vt == SPC5CUDA_F32 ? 2 : 1);
-    const int vbytes = vt == SPC5CUDA_F64 ? 8 : 4;
-    k_fit_flag<<<1, 1, 0, s>>>(work + 1, stride, vbytes, ROWS_HB, ROWS_VB, work);
-    SPC5_CUDA(cudaGetLastError());
+    return RowStats{rows::fit(vt, r, h[0], h[1]), rows::narrow(vt, r, nbr, nblocks, h[2], h[3])};
 }
 
 void launch_rows_kind(int kind, const BetaView& m, const void* x, void* y, cudaStream_t s) {

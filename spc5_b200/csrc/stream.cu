@@ -100,19 +100,10 @@ __device__ __forceinline__ void end_launch(bool follows) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Launches kern; follows: it may begin before the previous launch on s ends.
+// (launch_after, with this file's CTA.)
 template <class... P, class... Q>
 void launch(void (*kern)(P...), dim3 grid, bool follows, cudaStream_t s, Q... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(THREADS);
-    cfg.stream = s;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = follows ? 1 : 0;
-    SPC5_CUDA(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+    launch_after(kern, grid, THREADS, 0, follows, s, args...);
 }
 
 // The long rows: one warp per slab.
