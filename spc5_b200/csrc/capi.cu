@@ -44,15 +44,15 @@ void copy_in(Owned& dst, const void* src, size_t bytes, int on_device, cudaStrea
                                   on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
 }
 
-// Runs the validation kernel and turns its flag into a status.
+// Runs the validation kernel and turns its result into a status.
 void validate_csr(const spc5cuda_mat* m, cudaStream_t s) {
-    DevBuf flag(sizeof(int), s);
+    DevBuf out(2 * sizeof(int), s);
     launch_validate_csr(m->nrows, m->ncols, m->nnz, m->rowptr.as<int>(), m->colidx.as<int>(),
-                        flag.as<int>(), s);
-    int h = 0;
-    SPC5_CUDA(cudaMemcpyAsync(&h, flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+                        out.as<int>(), s);
+    int h[2] = {0, 0};
+    SPC5_CUDA(cudaMemcpyAsync(h, out.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     SPC5_CUDA(cudaStreamSynchronize(s));
-    if (h != 0) throw Error(SPC5CUDA_ERR_INVALID, "malformed CSR");
+    if (h[0] != 0 || h[1] != 0) throw Error(SPC5CUDA_ERR_INVALID, "malformed CSR");
 }
 
 }  // namespace

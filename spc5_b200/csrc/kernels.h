@@ -13,11 +13,12 @@ long scan_tmp_ints(long n);
 void exclusive_scan_i32(const int* in, int* out, long n, int* tmp, cudaStream_t s);
 
 // ---- CSR checks and conversion (convert.cu) -------------------------------
-// Writes 0 to *d_flag when the CSR is well formed (monotone rowptr starting
-// at 0, columns in [0, ncols), strictly increasing inside a row), else an
-// error code (1 rowptr, 2 column range, 3 order/duplicate).
+// Writes two zeros to d_out when the CSR is well formed (monotone rowptr
+// starting at 0, columns in [0, ncols), strictly increasing inside a row);
+// d_out[0]: 1 rowptr, 2 column range; d_out[1]: order or duplicate.  colidx is
+// 16-byte aligned.
 void launch_validate_csr(int nrows, int ncols, long nnz, const int* rowptr, const int* colidx,
-                         int* d_flag, cudaStream_t s);
+                         int* d_out, cudaStream_t s);
 
 // counts[br] = blocks of block-row br for rows-per-block r and VS columns.
 void launch_blockrow_counts(int vs, int r, int nrows, const int* rowptr, const int* colidx,

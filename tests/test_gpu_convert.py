@@ -66,3 +66,35 @@ def test_release_leaves_a_relaxed_capture_alone(cuda):
     graph.replay()
     torch.cuda.synchronize()
     assert z[0].item() == 2.0
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 8, 4099])
+def test_malformed_csr_is_refused(cuda, n):
+    """Rows of two entries whose columns fall from one row to the next (allowed)
+    and, one fault at a time, inside a row (not); entries on both sides of the
+    quads that a thread reads, the last ones among them."""
+    rowptr = np.arange(0, 2 * n + 1, 2, dtype=np.int32)
+    colidx = np.tile(np.array([3, 7], np.int32), n)
+    vals = np.ones(2 * n)
+
+    def refused(rp, ci):
+        try:
+            S.csr_matrix(rp, ci, vals, 8)
+        except S.SPC5Error:
+            return True
+        return False
+
+    assert not refused(rowptr, colidx)
+    single = np.concatenate([[0], np.arange(1, 2 * n + 1)]).astype(np.int32)
+    assert not refused(single, colidx[::-1].copy())
+    for row in {0, 1, n // 2, n - 1} & set(range(n)):
+        for at, value in ((2 * row, 7), (2 * row, 8), (2 * row + 1, 3), (2 * row + 1, 8), (2 * row + 1, -1), (2 * row, -1)):
+            bad = colidx.copy()
+            bad[at] = value
+            assert refused(rowptr, bad), (row, at, value)
+        bad = rowptr.copy()
+        bad[row + 1] += 2 * n + 1
+        assert refused(bad, colidx)
+        bad = rowptr.copy()
+        bad[row] = -1
+        assert refused(bad, colidx)
