@@ -58,11 +58,11 @@ struct BetaView {
     // device word written by an earlier kernel on the same stream)
     const int* run_if = nullptr;
     int run_if_value = 0;
+    bool follows = false;  // may become resident before the launch before it ends (run_if launches wait for it)
 };
 
 // Number of VS-lane groups the SpMV kernels launch on the current device
 // for rows-per-block r: one wave of resident CTAs.
-    bool follows = false;  // may become resident before the launch before it ends (run_if launches wait for it)
 int spmv_groups(int vs, int r);
 
 // gstart[0..ngroups] = block-row ranges holding ~nblocks/ngroups blocks each.
