@@ -192,10 +192,12 @@ def _check(status: int, what: str = "") -> None:
 
 
 def _stream(stream=None):
+    """CUDA stream handle: of the given stream, else of torch's current one (read without
+    building a Stream object)."""
+    if stream is not None:
+        return stream.cuda_stream
     import torch
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(stream.cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _dptr(t, dtype=None, what="tensor"):
@@ -207,7 +209,7 @@ def _dptr(t, dtype=None, what="tensor"):
         raise ValueError(f"{what} must be contiguous")
     if dtype is not None and t.dtype != dtype:
         raise TypeError(f"{what} must be {dtype}, got {t.dtype}")
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _np_ptr(a):
@@ -231,6 +233,7 @@ class SPC5Mat:
     def __init__(self, handle, keep=None):
         self._h = handle
         self._keep = keep
+        self._vt = None  # value type: the handle's for life
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -294,11 +297,13 @@ class SPC5Mat:
     @property
     def dtype(self):
         """Value dtype (float32 for both F32 and F32_V8 handles)."""
-        return np.float64 if self.info().value_type == F64 else np.float32
+        return np.float64 if self.value_type == F64 else np.float32
 
     @property
     def value_type(self) -> int:
-        return self.info().value_type
+        if self._vt is None:
+            self._vt = self.info().value_type
+        return self._vt
 
     def arrays(self):
         """Host copies of (rowsSize, blocksColumnIndexesWithMasks, values)."""
