@@ -4,12 +4,12 @@
 // admitted against an HBM budget that also covers the per-slot staging
 // buffers.  A request is y = A_id x for device vectors x (ncols) and y
 // (nrows).  One scheduler thread owns `slots` CUDA streams, each with
-// column-major staging blocks X (ncols x max_k) and Y (nrows x max_k):
+// row-major staging blocks X (ncols x max_k) and Y (nrows x max_k):
 //   * whenever a slot is free and requests are pending, it takes the matrix
 //     whose oldest request waits longest, coalesces up to max_k of its
-//     requests (copies each x into a column of X), runs one multi-RHS SpMM
-//     (spmm.cu, spmm_rows.cu) and copies each column of Y to its request's
-//     y; a lone request runs the matrix's SpMV into its own y instead;
+//     requests (one launch makes their x the columns of X), runs one
+//     multi-RHS SpMM (spmm.cu, spmm_rows.cu, stream.cu) and one launch that
+//     makes the columns of Y their y; a lone request runs the matrix's SpMV into its own y instead;
 //   * requests that arrive while launches are in flight wait for the next
 //     free slot and are batched then, so up to `slots` launches overlap on
 //     the device and the batch size adapts to the arrival rate;
@@ -48,6 +48,49 @@ struct Request {
     double t_done = 0.0;
     bool done = false;
 };
+
+// Vectors of one launch's requests.
+constexpr int MAX_K = 16;
+struct Vectors {
+    void* v[MAX_K];
+};
+
+// Between k vectors of n elements and an n x ldx row-major block: IN, the block
+// from the vectors (its columns k .. ldx - 1 are zero), else the vectors from the
+// block.  A tile of ROWS rows goes through shared memory, so that both sides are
+// read and written along memory.  One launch instead of a copy per request: the
+// copies (two per request, about 3 us of the scheduler's time each) took longer
+// than the products, and a row-major block is what the SpMM kernels read as
+// vectors.
+constexpr int TILE_ROWS = 256;
+template <class T, bool IN>
+__global__ void __launch_bounds__(TILE_ROWS) k_vectors(const __grid_constant__ Vectors vec, int k, long n, int ldx,
+                                                       T* __restrict__ block) {
+    __shared__ T tile[TILE_ROWS * (MAX_K + 1)];  // one element more per row: no bank conflicts down a column
+    const long i0 = long(blockIdx.x) * TILE_ROWS;
+    const long i = i0 + threadIdx.x;
+    const int rows = int(min(long(TILE_ROWS), n - i0));
+    const int pitch = ldx + 1 - (ldx & 1);  // odd
+    T* mine = tile + threadIdx.x * pitch;
+    if constexpr (IN) {
+        if (i < n)
+            for (int q = 0; q < ldx; ++q) mine[q] = q < k ? static_cast<const T*>(vec.v[q])[i] : T(0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < rows * ldx; e += TILE_ROWS) block[i0 * ldx + e] = tile[e / ldx * pitch + e % ldx];
+    } else {
+        for (int e = threadIdx.x; e < rows * ldx; e += TILE_ROWS) tile[e / ldx * pitch + e % ldx] = block[i0 * ldx + e];
+        __syncthreads();
+        if (i < n)
+            for (int q = 0; q < k; ++q) static_cast<T*>(vec.v[q])[i] = mine[q];
+    }
+}
+
+template <class T, bool IN>
+void launch_vectors(const Vectors& vec, int k, long n, int ldx, void* block, cudaStream_t s) {
+    if (n <= 0) return;
+    k_vectors<T, IN><<<unsigned(div_up(n, TILE_ROWS)), TILE_ROWS, 0, s>>>(vec, k, n, ldx, static_cast<T*>(block));
+    SPC5_CUDA(cudaGetLastError());
+}
 
 struct Slot {
     cudaStream_t stream = nullptr;
@@ -143,7 +186,6 @@ bool spc5cuda_server::dispatch(Slot& sl) {
     const int k = int(sl.reqs.size());
     const size_t xb = cfg.mixed ? 4 : 8;
     const size_t yb = 8;
-    const long ldX = max_cols, ldY = max_rows;
     std::vector<std::pair<const void*, void*>> io;
     {
         std::lock_guard<std::mutex> lk(mu);
@@ -166,26 +208,31 @@ bool spc5cuda_server::dispatch(Slot& sl) {
                             sl.stream);
         return finish_dispatch(sl, k);
     }
-    char* X = sl.X.as<char>();
-    char* Y = sl.Y.as<char>();
-    for (int q = 0; q < k; ++q)
-        SPC5_CUDA(cudaMemcpyAsync(X + size_t(q) * ldX * xb, io[size_t(q)].first, size_t(m->ncols) * xb,
-                                  cudaMemcpyDeviceToDevice, sl.stream));
-    SPC5_CUDA(cudaMemsetAsync(Y, 0, size_t(k) * ldY * yb, sl.stream));
+    // whole 16-byte vectors per row of X and Y where the slot has room for them
+    const int per = int(16 / xb);
+    const int ld = (k + per - 1) / per * per <= cfg.max_k ? (k + per - 1) / per * per : k;
+    void* X = sl.X.p;
+    void* Y = sl.Y.p;
+    Vectors xs{}, ys{};
+    for (int q = 0; q < k; ++q) {
+        xs.v[q] = const_cast<void*>(io[size_t(q)].first);
+        ys.v[q] = io[size_t(q)].second;
+    }
+    if (cfg.mixed) launch_vectors<float, true>(xs, k, m->ncols, ld, X, sl.stream);
+    else launch_vectors<double, true>(xs, k, m->ncols, ld, X, sl.stream);
+    SPC5_CUDA(cudaMemsetAsync(Y, 0, size_t(ld) * size_t(m->nrows) * yb, sl.stream));
     if (m->use_plan())
-        plan_spmm(m, k, X, 1, ldX, Y, 1, ldY, cfg.mixed, sl.stream);
+        plan_spmm(m, ld, X, ld, 1, Y, ld, 1, cfg.mixed, sl.stream);
     else if (cfg.mixed && m->value_type == SPC5CUDA_F32_V8)
-        launch_spmm_mixed8(m->spmm_view(), k, reinterpret_cast<const float*>(X), 1, ldX,
-                           reinterpret_cast<double*>(Y), 1, ldY, sl.stream);
+        launch_spmm_mixed8(m->spmm_view(), ld, static_cast<const float*>(X), ld, 1, static_cast<double*>(Y), ld, 1,
+                           sl.stream);
     else if (cfg.mixed)
-        launch_spmm_mixed(m->spmm_view(), k, reinterpret_cast<const float*>(X), 1, ldX,
-                          reinterpret_cast<double*>(Y), 1, ldY, sl.stream);
+        launch_spmm_mixed(m->spmm_view(), ld, static_cast<const float*>(X), ld, 1, static_cast<double*>(Y), ld, 1,
+                          sl.stream);
     else
-        launch_spmm_f64(m->spmm_view(), k, reinterpret_cast<const double*>(X), 1, ldX,
-                        reinterpret_cast<double*>(Y), 1, ldY, sl.stream);
-    for (int q = 0; q < k; ++q)
-        SPC5_CUDA(cudaMemcpyAsync(io[size_t(q)].second, Y + size_t(q) * ldY * yb, size_t(m->nrows) * yb,
-                                  cudaMemcpyDeviceToDevice, sl.stream));
+        launch_spmm_f64(m->spmm_view(), ld, static_cast<const double*>(X), ld, 1, static_cast<double*>(Y), ld, 1,
+                        sl.stream);
+    launch_vectors<double, false>(ys, k, m->nrows, ld, Y, sl.stream);
     return finish_dispatch(sl, k);
 }
 
