@@ -839,7 +839,7 @@ def serve_leg(args, rates, seconds, precisions=(False, True), plan_serial=False)
             for csr in distinct:
                 m = S.csr_matrix(csr.rowptr, csr.colidx, csr.values.astype(dt), csr.ncols,
                                  value_type=S.F32_V8 if mixed else None)
-                # default kernel choice: the length-sorted plan for the
+                # default kernel choice: the sorted plan for the
                 # power-law matrices (its single copy of the arrays serves
                 # lone requests and batches alike), the row kernels for the
                 # stencils
@@ -930,7 +930,7 @@ TRAFFIC_RATIO = {"powerlaw": {1: 1.199, 2: 1.203, 4: 1.168, 8: 1.593},
 
 # spc5cuda_mat_kernel codes: SPC5CUDA_KERNEL_GROUPS = 1, SPC5CUDA_KERNEL_ROWS = 2
 KERNEL_NAME = {1: "k_spmv (group per block-row stream)", 2: "k_rows (thread per sub-row)",
-               3: "sorted plan (k_rows by block-row size; largest block-rows as multiply-add chains, k_chain_spmv)", 0: "unconverted"}
+               3: "sorted plan (long rows as warp streams, k_stream_spmv; short rows one per lane, k_short_spmv)", 0: "unconverted"}
 
 
 def select_kernel(m, which):

@@ -90,7 +90,7 @@ SPC5CUDA_API void spc5cuda_set_stream(void* stream);
  * the group kernel (both enqueued, each gated on that device flag: no host
  * round trip).  Scratch (block-row offsets and work splits) comes from a
  * stream-ordered memory pool the library keeps per device.  The handle API
- * below keeps the offsets resident and adds the length-sorted plan for
+ * below keeps the offsets resident and adds the sorted plan for
  * irregular matrices.  Errors: spc5cuda_get_last_error().
  * ---------------------------------------------------------------------- */
 SPC5CUDA_API void core_SPC5_1rVc_Spmv_double(const long int nbRows, const int* rowsSizes,
@@ -189,7 +189,7 @@ SPC5CUDA_API spc5cuda_status spc5cuda_mat_info(const spc5cuda_mat* mat, spc5cuda
  * kernel per r and instruction set).  Both kernels give the same bits.
  *   AUTO   -- the thread-per-sub-row kernel when every block-row fits its
  *             per-warp staging buffers (stencils, Poisson, banded); the
- *             length-sorted plan (below) when some block-row does not;
+ *             sorted plan (below) when some block-row does not;
  *   GROUPS -- always the group kernel (one group of VS lanes per block-row
  *             stream);
  *   ROWS   -- the thread-per-sub-row kernel; SPC5CUDA_ERR_UNSUPPORTED on a
@@ -254,7 +254,7 @@ SPC5CUDA_API spc5cuda_status spc5cuda_spmv_mixed(const spc5cuda_mat* mat, const 
  * ldx >= k (the k values of one matrix column are contiguous), Y row-major
  * nrows x k with ldy >= k.  Column j of Y is bit-identical to spc5cuda_spmv
  * with column j of X.  The kernel follows the handle's choice (see
- * spc5cuda_mat_set_kernel): through the length-sorted plan when the handle
+ * spc5cuda_mat_set_kernel): through the sorted plan when the handle
  * has one; the staged SpMM when every block-row fits the row kernels'
  * buffers; the group SpMM for SPC5CUDA_KERNEL_GROUPS.  Up to 16 right-hand
  * sides run in one pass over the matrix (fewer at larger r: at most 32

@@ -15,12 +15,12 @@ namespace {
 // B200 cost model of one SpMV through a converted handle's default kernel
 // choice (spc5_b200/tune_fit.py fits it from timings on a B200, 148 SMs at
 // 1.965 GHz): for value type, r and regime (0: the row kernel, every
-// block-row fits its staging buffers; 1: the length-sorted plan),
+// block-row fits its staging buffers; 1: the sorted plan),
 //     t_us = t0 + nnz * (d0 + d1 / a + d2 / a^2),  a = nnz / blocks_r,
 // the time per value keyed by the average number of values per block, as the
 // reference's SPC5_find_best model is (src/spc5.hpp:1157-1212).
 // Value type (F64, F32, F32_V8) x r (1, 2, 4, 8) x regime: {t0, d0, d1, d2}.
-// The sorted-plan rows were refitted after the plan's chain part (r = 2, 4,
+// The sorted-plan rows were fitted on an earlier form of the plan (r = 2, 4,
 // 8) on the plan-regime calibration matrices alone (power-law and random,
 // tune_fit.plan_calibration_set), keeping the row-kernel t0.
 constexpr double kModel[3][4][2][4] = {
@@ -66,7 +66,7 @@ int plan_regime(const spc5cuda_mat* m, int r, const int* brptr, cudaStream_t s) 
 
 // A trial run: a temporary handle holding a copy of the CSR matrix is
 // converted to r the usual way (its default kernel choice: the row kernel or
-// the length-sorted plan) and its SpMV is timed (2 warm-up calls, which also
+// the sorted plan) and its SpMV is timed (2 warm-up calls, which also
 // load its kernels and size the library's scratch pool, then 5 timed calls);
 // returns microseconds per SpMV.
 double measure_us(const spc5cuda_mat* m, int r, cudaStream_t s) {
