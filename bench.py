@@ -925,8 +925,8 @@ def run_serve(args):
 # so roofline.traffic of the full workloads is these ratios times their bytes.
 L2_BYTES = 126e6  # B200 L2
 
-TRAFFIC_RATIO = {"powerlaw": {1: 1.199, 2: 1.203, 4: 1.168, 8: 1.593},
-                 "stencil27": {1: 0.999, 2: 0.984, 4: 0.978, 8: 0.994}}
+TRAFFIC_RATIO = {"powerlaw": {1: 1.210, 2: 1.178, 4: 1.102, 8: 0.971},
+                 "stencil27": {1: 1.000, 2: 0.988, 4: 0.982, 8: 0.979}}
 
 # spc5cuda_mat_kernel codes: SPC5CUDA_KERNEL_GROUPS = 1, SPC5CUDA_KERNEL_ROWS = 2
 KERNEL_NAME = {1: "k_spmv (group per block-row stream)", 2: "k_rows (thread per sub-row)",
