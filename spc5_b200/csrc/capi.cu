@@ -4,8 +4,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "handle.h"
@@ -74,50 +72,6 @@ void spc5cuda::valptr_from_headers(int mask_bytes, int r, int nbr, const int* br
     DevBuf tmp(sizeof(int) * size_t(scan_tmp_ints(nbr) + 1), s);
     launch_blockrow_value_counts(mask_bytes, r, nbr, brptr, headers, valptr, s);
     exclusive_scan_i32(valptr, valptr, nbr, tmp.as<int>(), s);
-}
-
-// One pool and one allocation stream per device for the process lifetime.
-namespace {
-struct DeviceMemory {
-    cudaMemPool_t pool = nullptr;
-    cudaStream_t stream = nullptr;
-    void* anchor = nullptr;  // keeps the memory mapped that wait_device() takes and frees
-};
-
-const DeviceMemory& device_memory() {
-    static std::mutex mu;
-    static DeviceMemory mem[64];
-    constexpr uint64_t keep = uint64_t(4) << 30;
-    int dev = 0;
-    SPC5_CUDA(cudaGetDevice(&dev));
-    require(dev >= 0 && dev < 64, SPC5CUDA_ERR_UNSUPPORTED, "device index");
-    std::lock_guard<std::mutex> lk(mu);
-    DeviceMemory& m = mem[dev];
-    if (!m.stream) {
-        if (!m.pool) {
-            cudaMemPoolProps props;
-            std::memset(&props, 0, sizeof(props));
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            SPC5_CUDA(cudaMemPoolCreate(&m.pool, &props));
-            uint64_t bytes = keep;
-            SPC5_CUDA(cudaMemPoolSetAttribute(m.pool, cudaMemPoolAttrReleaseThreshold, &bytes));
-        }
-        if (!m.anchor) SPC5_CUDA(cudaMalloc(&m.anchor, 16));
-        SPC5_CUDA(cudaStreamCreateWithFlags(&m.stream, cudaStreamNonBlocking));
-    }
-    return m;
-}
-}  // namespace
-
-cudaMemPool_t spc5cuda::scratch_pool() { return device_memory().pool; }
-cudaStream_t spc5cuda::alloc_stream() { return device_memory().stream; }
-
-void spc5cuda::wait_device() {
-    void* p = nullptr;
-    if (cudaMalloc(&p, 16) == cudaSuccess) cudaFree(p);
-    else cudaDeviceSynchronize();
 }
 
 namespace {

@@ -4,10 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <stdexcept>
-#include <string>
-
-#include "spc5cuda.h"
+#include "errors.h"
 
 namespace spc5cuda {
 
@@ -38,21 +35,6 @@ struct Header {
     // least one byte of the record, so none reads past the array.
     static constexpr int LOAD_WORDS = (STRIDE % 4 == 0) ? STRIDE / 4 : 2;
 };
-
-// Thrown inside the host layer, turned into a status code at the C ABI.
-struct Error : std::runtime_error {
-    spc5cuda_status status;
-    Error(spc5cuda_status s, const std::string& what) : std::runtime_error(what), status(s) {}
-};
-
-inline void check_cuda(cudaError_t e, const char* what) {
-    if (e != cudaSuccess) {
-        throw Error(e == cudaErrorMemoryAllocation ? SPC5CUDA_ERR_NOMEM : SPC5CUDA_ERR_CUDA,
-                    std::string(what) + ": " + cudaGetErrorString(e));
-    }
-}
-
-#define SPC5_CUDA(call) ::spc5cuda::check_cuda((call), #call)
 
 inline int div_up(long a, long b) { return int((a + b - 1) / b); }
 

@@ -10,91 +10,9 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "memory.h"
 
 namespace spc5cuda {
-
-// The library's memory pool on the current device (capi.cu): per-call scratch
-// and the handles' buffers come from it.  It keeps up to 4 GiB of freed memory
-// for the next allocation (mapping memory afresh for every buffer took most of
-// a conversion's time) and gives the rest back.
-cudaMemPool_t scratch_pool();
-// A stream of the current device that only orders the pool's persistent
-// buffers.
-cudaStream_t alloc_stream();
-
-// Waits for all work on the current device, as freeing memory does: unlike
-// cudaDeviceSynchronize(), that leaves another stream's relaxed capture alone.
-void wait_device();
-
-// Stream-ordered scratch.
-struct PoolBuf {
-    void* p = nullptr;
-    size_t bytes = 0;
-    cudaStream_t s;
-    PoolBuf(size_t n, cudaStream_t st) : bytes(n), s(st) {
-        SPC5_CUDA(cudaMallocFromPoolAsync(&p, n < 16 ? size_t(16) : n, scratch_pool(), st));
-    }
-    ~PoolBuf() {
-        if (p) cudaFreeAsync(p, s);
-    }
-    PoolBuf(const PoolBuf&) = delete;
-    PoolBuf& operator=(const PoolBuf&) = delete;
-    template <class U>
-    U* as() const { return static_cast<U*>(p); }
-};
-using DevBuf = PoolBuf;
-
-// Persistent device buffer owned by a matrix handle.  alloc() returns memory
-// that every stream may use; release() waits for the device first, as kernels
-// on any stream may still use the buffer.
-struct Owned {
-    void* p = nullptr;
-    size_t bytes = 0;
-    int dev = 0;
-    void alloc(size_t n) {
-        release();
-        if (n) {
-            SPC5_CUDA(cudaGetDevice(&dev));
-            const cudaStream_t s = alloc_stream();
-            SPC5_CUDA(cudaMallocFromPoolAsync(&p, n, scratch_pool(), s));
-            SPC5_CUDA(cudaStreamSynchronize(s));
-        }
-        bytes = n;
-    }
-    void release() {
-        if (p) {
-            int now = 0;
-            cudaGetDevice(&now);
-            if (now != dev) cudaSetDevice(dev);
-            wait_device();
-            cudaFreeAsync(p, alloc_stream());
-            if (now != dev) cudaSetDevice(now);
-        }
-        p = nullptr;
-        bytes = 0;
-    }
-    Owned() = default;
-    Owned(const Owned&) = delete;
-    Owned& operator=(const Owned&) = delete;
-    Owned(Owned&& o) noexcept : p(o.p), bytes(o.bytes), dev(o.dev) {
-        o.p = nullptr;
-        o.bytes = 0;
-    }
-    Owned& operator=(Owned&& o) noexcept {
-        if (this != &o) {
-            release();
-            p = o.p;
-            bytes = o.bytes;
-            dev = o.dev;
-            o.p = nullptr;
-            o.bytes = 0;
-        }
-        return *this;
-    }
-    ~Owned() { release(); }
-    template <class T>
-    T* as() const { return static_cast<T*>(p); }
-};
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
