@@ -11,6 +11,26 @@ namespace spc5cuda {
 
 namespace {
 
+// The calling thread's captures, and those of other threads in the global mode,
+// refuse calls that are unsafe beside them (cudaMalloc, cudaFree, cudaFreeAsync)
+// and are spoilt by them; in this scope the calls are allowed, for memory that no
+// capture uses.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Waits for all work on the current device, as freeing memory does: unlike
+// cudaDeviceSynchronize(), that leaves a capture that is open on another stream
+// alone.  False when the wait was refused.
+bool wait_device() {
+    void* p = nullptr;
+    if (cudaMalloc(&p, 16) == cudaSuccess && cudaFree(p) == cudaSuccess) return true;
+    cudaGetLastError();
+    return cudaDeviceSynchronize() == cudaSuccess;
+}
+
 // One pool and one allocation stream per device for the process lifetime.
 struct DeviceMemory {
     cudaMemPool_t pool = nullptr;
@@ -49,10 +69,14 @@ const DeviceMemory& device_memory() {
 cudaMemPool_t scratch_pool() { return device_memory().pool; }
 cudaStream_t alloc_stream() { return device_memory().stream; }
 
-void wait_device() {
-    void* p = nullptr;
-    if (cudaMalloc(&p, 16) == cudaSuccess) cudaFree(p);
-    else cudaDeviceSynchronize();
+void give_back(void* p, int dev) {
+    const RelaxedCapture relaxed;
+    int now = 0;
+    cudaGetDevice(&now);
+    if (now != dev) cudaSetDevice(dev);
+    // a refusal is not left for the next call's check to report
+    if (!wait_device() || cudaFreeAsync(p, alloc_stream()) != cudaSuccess) cudaGetLastError();
+    if (now != dev) cudaSetDevice(now);
 }
 
 }  // namespace spc5cuda

@@ -18,9 +18,9 @@ cudaMemPool_t scratch_pool();
 // buffers.
 cudaStream_t alloc_stream();
 
-// Waits for all work on the current device, as freeing memory does: unlike
-// cudaDeviceSynchronize(), that leaves another stream's relaxed capture alone.
-void wait_device();
+// Gives a persistent buffer on device dev back to the pool after all work of the
+// device; keeps it out of the pool when it could not wait.
+void give_back(void* p, int dev);
 
 // Stream-ordered scratch.
 struct PoolBuf {
@@ -58,14 +58,7 @@ struct Owned {
         bytes = n;
     }
     void release() {
-        if (p) {
-            int now = 0;
-            cudaGetDevice(&now);
-            if (now != dev) cudaSetDevice(dev);
-            wait_device();
-            cudaFreeAsync(p, alloc_stream());
-            if (now != dev) cudaSetDevice(now);
-        }
+        if (p) give_back(p, dev);
         p = nullptr;
         bytes = 0;
     }
