@@ -69,14 +69,17 @@ const DeviceMemory& device_memory() {
 cudaMemPool_t scratch_pool() { return device_memory().pool; }
 cudaStream_t alloc_stream() { return device_memory().stream; }
 
-void give_back(void* p, int dev) {
-    const RelaxedCapture relaxed;
+void give_back(void* p, int dev, cudaStream_t s) noexcept {
     int now = 0;
-    cudaGetDevice(&now);
-    if (now != dev) cudaSetDevice(dev);
-    // a refusal is not left for the next call's check to report
-    if (!wait_device() || cudaFreeAsync(p, alloc_stream()) != cudaSuccess) cudaGetLastError();
+    if (cudaGetDevice(&now) != cudaSuccess) {  // the runtime unloads
+        cudaGetLastError();
+        return;
+    }
+    const RelaxedCapture relaxed;
+    bool ok = now == dev || cudaSetDevice(dev) == cudaSuccess;
+    ok = ok && wait_device() && cudaFreeAsync(p, s) == cudaSuccess;
     if (now != dev) cudaSetDevice(now);
+    if (!ok) cudaGetLastError();  // not left for the next call's check to report
 }
 
 }  // namespace spc5cuda

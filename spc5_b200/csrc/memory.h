@@ -18,9 +18,10 @@ cudaMemPool_t scratch_pool();
 // buffers.
 cudaStream_t alloc_stream();
 
-// Gives a persistent buffer on device dev back to the pool after all work of the
-// device; keeps it out of the pool when it could not wait.
-void give_back(void* p, int dev);
+// Gives a persistent buffer of device dev, whose allocation stream is s, back to
+// the pool after all work of the device; keeps it out of the pool when it could
+// not wait.
+void give_back(void* p, int dev, cudaStream_t s) noexcept;
 
 // Stream-ordered scratch.
 struct PoolBuf {
@@ -47,25 +48,26 @@ struct Owned {
     void* p = nullptr;
     size_t bytes = 0;
     int dev = 0;
+    cudaStream_t s = nullptr;  // the device's allocation stream
     void alloc(size_t n) {
         release();
         if (n) {
             SPC5_CUDA(cudaGetDevice(&dev));
-            const cudaStream_t s = alloc_stream();
+            s = alloc_stream();
             SPC5_CUDA(cudaMallocFromPoolAsync(&p, n, scratch_pool(), s));
             SPC5_CUDA(cudaStreamSynchronize(s));
         }
         bytes = n;
     }
-    void release() {
-        if (p) give_back(p, dev);
+    void release() noexcept {
+        if (p) give_back(p, dev, s);
         p = nullptr;
         bytes = 0;
     }
     Owned() = default;
     Owned(const Owned&) = delete;
     Owned& operator=(const Owned&) = delete;
-    Owned(Owned&& o) noexcept : p(o.p), bytes(o.bytes), dev(o.dev) {
+    Owned(Owned&& o) noexcept : p(o.p), bytes(o.bytes), dev(o.dev), s(o.s) {
         o.p = nullptr;
         o.bytes = 0;
     }
@@ -75,6 +77,7 @@ struct Owned {
             p = o.p;
             bytes = o.bytes;
             dev = o.dev;
+            s = o.s;
             o.p = nullptr;
             o.bytes = 0;
         }

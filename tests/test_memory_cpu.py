@@ -41,3 +41,9 @@ def test_a_buffer_is_kept_when_the_wait_is_refused(fake):
     the refusals are not left for the next call to report."""
     assert fake("no_wait") == ["cudaMalloc refused", "cudaDeviceSynchronize refused", "mode as before", "last error 0",
                                "done"]
+
+
+def test_a_release_does_not_throw(fake):
+    """While the runtime unloads, a destructor has nothing to give back and must
+    not end the process."""
+    assert fake("unloading") == ["cudaGetDevice refused", "mode as before", "last error 0", "done"]
