@@ -11,7 +11,8 @@
  *
  * All pointers passed to the compute entry points are DEVICE pointers
  * (cudaMalloc, cudaMallocAsync or torch allocations) with at least 16-byte
- * alignment for the header and value arrays; work is enqueued on the given
+ * alignment for the value arrays and 4-byte alignment for the header arrays
+ * (16-byte aligned headers are faster); work is enqueued on the given
  * stream (NULL = legacy default stream) and is asynchronous unless stated.
  * No entry point falls back to the CPU.
  *
@@ -86,9 +87,10 @@ SPC5CUDA_API void spc5cuda_set_stream(void* stream);
  * y[0..nbRows) += A x.  The value offset of every block-row is not stored
  * in the format, so each call first derives it from the headers (one extra
  * pass over the header array), tests on the device whether every block-row
- * fits the row kernel's staging buffers, and runs the row kernel if so, else
- * the group kernel (both enqueued, each gated on that device flag: no host
- * round trip).  Scratch (block-row offsets and work splits) comes from a
+ * fits the row kernel's staging buffers, and runs the row kernel if so (one
+ * of two instantiations, by the masks), else the group kernel (all three
+ * enqueued, each gated on that device flag: no host round trip; headers that
+ * are not 16-byte aligned: the group kernel alone).  Scratch (block-row offsets and work splits) comes from a
  * stream-ordered memory pool the library keeps per device.  The handle API
  * below keeps the offsets resident and adds the sorted plan for
  * irregular matrices.  Errors: spc5cuda_get_last_error().

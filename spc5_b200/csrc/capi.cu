@@ -81,7 +81,8 @@ namespace {
 // must know about the arrays (core_prep.cu); then the two instantiations of the
 // row kernel and the group kernel are enqueued, gated on a device word: a row
 // kernel runs when every block-row fits its staging buffers, the group kernel
-// otherwise.  All give the reference's bits.
+// otherwise (alone when the headers are not 16-byte aligned).  All give the
+// reference's bits.
 template <class T>
 void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* headers,
                const T* values, const T* x, T* y, cudaStream_t s) {
@@ -121,10 +122,19 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     v.run_if_value = 0;   // group kernel: some block-row does not fit
     vr.run_if_value = 1;  // row kernel: every block-row fits
     vn.run_if_value = 2;  // and the masks are narrow
-    for (const BetaView& one : {vn, vr, v}) {
+    auto launch = [&](const BetaView& one) {
         if constexpr (sizeof(T) == 8) launch_spmv_f64(one, x, y, s);
         else launch_spmv_f32(one, x, y, s);
+    };
+    if (!aligned(headers, 16)) {
+        // the row kernels stage 16 header bytes at a time from the array's base
+        // on; the group kernel reads aligned 4-byte words
+        v.run_if = nullptr;
+        v.follows = false;
+        launch(v);
+        return;
     }
+    for (const BetaView& one : {vn, vr, v}) launch(one);
 }
 
 }  // namespace
