@@ -12,6 +12,7 @@
 // the scan, two splits, a memset, the maxima, a sample, the flag) and the gated
 // kernels one after the other it took 122.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "handle.h"
@@ -24,15 +25,24 @@ namespace {
 using rows::NS;
 
 constexpr int THREADS = 256;
-constexpr int TILE = THREADS;  // block-rows per CTA: 100^3 at r = 4 has 977 tiles
+constexpr int TILE = THREADS;  // block-rows per CTA of the second launch
 // Lanes per block-row in the counting pass: a 27-point stencil's 9 blocks take
-// three loads per lane, a row of 900 blocks 225.
-constexpr int L = 4;
-// Up to this many tiles (1M block-rows) a CTA sums the tiles before its own
-// itself, 16 loads per thread at most; more are scanned by a launch between.
+// three loads per lane.  The smallest parts have the threads for 16.
+constexpr int L = 4, MOST_L = 16;
+// Up to this many parts a CTA sums the parts before its own tile itself, 16 loads
+// per thread at most; more are scanned by a launch between.
 constexpr int MAX_DIRECT = 4096;
+// Parts of a tile: 256, 64 or 16 block-rows, the largest with enough CTAs for the
+// chip, since the threads of a CTA share its block-rows' headers and a few long
+// block-rows are as much work as many short ones.  With whole tiles, 50,000 rows of
+// 400 values at r = 8 (25 tiles) made a call of 3452 us on a B200, now 1227.
+int part_rows(int nbr) {
+    for (int part : {TILE, TILE / 4})
+        if (div_up(long(nbr) + 1, part) >= 2 * sm_count()) return part;
+    return TILE / MOST_L;
+}
 
-// Per tile: values, most blocks and most values of a block-row, blocks whose
+// Per part: values, most blocks and most values of a block-row, blocks whose
 // every sub-row mask spans at most NS columns.
 struct TileStats {
     int values, blocks, most_values, narrow;
@@ -41,21 +51,22 @@ struct TileStats {
 __device__ __forceinline__ int warp_sum(int v) { return int(__reduce_add_sync(0xffffffffu, unsigned(v))); }
 __device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 
-// counts[i] = values of block-row i (0 for i = nbr), and the tile's stats.
-template <class LT, int R>
+// counts[i] = values of block-row i (0 for i = nbr), and the stats of the part of
+// ROWS block-rows; LANES lanes per block-row.
+template <class LT, int R, int ROWS, int LANES>
 __global__ void __launch_bounds__(THREADS) k_core_count(int nbr, const int* __restrict__ brptr,
                                                         const uint8_t* __restrict__ headers, int* __restrict__ counts,
                                                         TileStats* __restrict__ stats) {
     asm volatile("griddepcontrol.launch_dependents;");
     __shared__ TileStats part[THREADS / 32];
-    const int q = threadIdx.x % L;
-    const long base = long(blockIdx.x) * TILE;
+    const int q = threadIdx.x % LANES;
+    const long base = long(blockIdx.x) * ROWS;
     TileStats t{0, 0, 0, 0};
-    for (int i0 = threadIdx.x / L; i0 < TILE; i0 += THREADS / L) {  // uniform
+    for (int i0 = threadIdx.x / LANES; i0 < ROWS; i0 += THREADS / LANES) {  // uniform
         const long i = base + i0;
         const long b0 = i < nbr ? __ldg(brptr + i) : 0, b1 = i < nbr ? __ldg(brptr + i + 1) : 0;
         int v = 0;
-        for (long b = b0 + q; b < b1; b += L) {
+        for (long b = b0 + q; b < b1; b += LANES) {
             uint32_t mw[Header<LT, R>::MASK_WORDS];
             load_header<LT, R>(headers, b, mw);
             bool narrow = true;
@@ -68,7 +79,7 @@ __global__ void __launch_bounds__(THREADS) k_core_count(int nbr, const int* __re
             t.narrow += narrow ? 1 : 0;
         }
 #pragma unroll
-        for (int d = L / 2; d >= 1; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        for (int d = LANES / 2; d >= 1; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
         if (q == 0) {
             if (i <= nbr) counts[i] = v;
             t.values += v;
@@ -90,15 +101,15 @@ __global__ void __launch_bounds__(THREADS) k_core_count(int nbr, const int* __re
     }
 }
 
-// One CTA: before[t] = values of the tiles before tile t.
-__global__ void __launch_bounds__(THREADS) k_core_tiles(int ntiles, const TileStats* __restrict__ stats,
+// One CTA: before[t] = values of the parts before part t.
+__global__ void __launch_bounds__(THREADS) k_core_parts(int nparts, const TileStats* __restrict__ stats,
                                                         int* __restrict__ before) {
     __shared__ int sums[THREADS / 32];
     int carry = 0;
     const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
-    for (int t0 = 0; t0 < ntiles; t0 += THREADS) {  // uniform
+    for (int t0 = 0; t0 < nparts; t0 += THREADS) {  // uniform
         const int t = t0 + threadIdx.x;
-        const int v = t < ntiles ? stats[t].values : 0;
+        const int v = t < nparts ? stats[t].values : 0;
         int incl = v;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -113,16 +124,16 @@ __global__ void __launch_bounds__(THREADS) k_core_tiles(int ntiles, const TileSt
             carry += sums[k];
         }
         __syncthreads();
-        if (t < ntiles) before[t] = at;
+        if (t < nparts) before[t] = at;
     }
 }
 
 // valptr (in: counts) = value offset of every block-row, the splits, and (CTA
 // 0) flag = 0 when some block-row does not fit the row kernel's buffers, else
-// 1 for its wide, 2 for its narrow instantiation.  before: see k_core_tiles,
-// null when the CTA adds up the tiles itself.
-__global__ void __launch_bounds__(THREADS) k_core_split(int nbr, const int* __restrict__ brptr, int* valptr,
-                                                        const TileStats* stats, const int* before, int ngroups,
+// 1 for its wide, 2 for its narrow instantiation.  nparts stats, `per` of them to
+// a tile; before: see k_core_parts, null when the CTA adds up the parts itself.
+__global__ void __launch_bounds__(THREADS) k_core_split(int nbr, const int* __restrict__ brptr, int* valptr, int nparts,
+                                                        int per, const TileStats* stats, const int* before, int ngroups,
                                                         int* __restrict__ gstart, int nwarps, int* __restrict__ wstart,
                                                         int value_type, int r, int* __restrict__ flag) {
     __shared__ TileStats part[THREADS / 32];
@@ -138,10 +149,11 @@ __global__ void __launch_bounds__(THREADS) k_core_split(int nbr, const int* __re
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the counts
     // ---- values of the tiles before this one
     int carry = 0;
+    const int first = int(blockIdx.x) * per;
     if (!before)
-        for (int t = threadIdx.x; t < int(blockIdx.x); t += THREADS) carry += __ldcg(&stats[t].values);
+        for (int t = threadIdx.x; t < first; t += THREADS) carry += __ldcg(&stats[t].values);
     else if (threadIdx.x == 0)
-        carry = __ldcg(before + blockIdx.x);
+        carry = __ldcg(before + first);
     carry = warp_sum(carry);
     // ---- the tile
     const int v = i <= nbr ? __ldcg(valptr + i) : 0;
@@ -164,7 +176,7 @@ __global__ void __launch_bounds__(THREADS) k_core_split(int nbr, const int* __re
     // ---- the kernel that runs
     __syncthreads();
     TileStats m{0, 0, 0, 0};
-    for (unsigned t = threadIdx.x; t < gridDim.x; t += THREADS) {
+    for (int t = threadIdx.x; t < nparts; t += THREADS) {
         m.blocks = max(m.blocks, __ldcg(&stats[t].blocks));
         m.most_values = max(m.most_values, __ldcg(&stats[t].most_values));
         m.narrow += __ldcg(&stats[t].narrow);
@@ -188,7 +200,7 @@ constexpr size_t round_up(size_t n) { return (n + 255) / 256 * 256; }  // whole 
 }  // namespace
 
 CoreScratch core_scratch(int nbr, int ngroups, int nwarps) {
-    const size_t ntiles = size_t(div_up(long(nbr) + 1, TILE));
+    const size_t nparts = size_t(div_up(long(nbr) + 1, part_rows(nbr)));
     CoreScratch c;
     size_t at = 0;
     auto take = [&](size_t ints) {
@@ -197,8 +209,8 @@ CoreScratch core_scratch(int nbr, int ngroups, int nwarps) {
         return here;
     };
     c.valptr = take(size_t(nbr) + 1);
-    c.stats = take(ntiles * sizeof(TileStats) / sizeof(int));
-    c.before = take(ntiles > MAX_DIRECT ? ntiles : 0);
+    c.stats = take(nparts * sizeof(TileStats) / sizeof(int));
+    c.before = take(nparts > MAX_DIRECT ? nparts : 0);
     c.gstart = take(size_t(ngroups) + 1);
     c.wstart = take(size_t(nwarps) + 1);
     c.flag = take(1);
@@ -208,17 +220,25 @@ CoreScratch core_scratch(int nbr, int ngroups, int nwarps) {
 
 void launch_core_prep(int value_type, int r, int nbr, const int* brptr, const uint8_t* headers, int ngroups, int nwarps,
                       const CoreScratch& c, unsigned char* mem, cudaStream_t s) {
-    const int ntiles = div_up(long(nbr) + 1, TILE);
+    const int rows = part_rows(nbr), nparts = div_up(long(nbr) + 1, rows), ntiles = div_up(long(nbr) + 1, TILE);
     int* valptr = reinterpret_cast<int*>(mem + c.valptr);
     TileStats* stats = reinterpret_cast<TileStats*>(mem + c.stats);
-    int* before = ntiles > MAX_DIRECT ? reinterpret_cast<int*>(mem + c.before) : nullptr;
-    auto count = [&](auto lt) {
+    int* before = nparts > MAX_DIRECT ? reinterpret_cast<int*>(mem + c.before) : nullptr;
+    auto count_r = [&](auto lt, auto RC) {
         using LT = decltype(lt);
+        constexpr int R = decltype(RC)::value;
+        auto kern = rows == TILE ? k_core_count<LT, R, TILE, L>
+                                 : (rows == TILE / 4 ? k_core_count<LT, R, TILE / 4, L>
+                                                     : k_core_count<LT, R, TILE / MOST_L, MOST_L>);
+        kern<<<nparts, THREADS, 0, s>>>(nbr, brptr, headers, valptr, stats);
+    };
+    auto count = [&](auto lt) {
+        using std::integral_constant;
         switch (r) {
-            case 1: k_core_count<LT, 1><<<ntiles, THREADS, 0, s>>>(nbr, brptr, headers, valptr, stats); return;
-            case 2: k_core_count<LT, 2><<<ntiles, THREADS, 0, s>>>(nbr, brptr, headers, valptr, stats); return;
-            case 4: k_core_count<LT, 4><<<ntiles, THREADS, 0, s>>>(nbr, brptr, headers, valptr, stats); return;
-            case 8: k_core_count<LT, 8><<<ntiles, THREADS, 0, s>>>(nbr, brptr, headers, valptr, stats); return;
+            case 1: count_r(lt, integral_constant<int, 1>{}); return;
+            case 2: count_r(lt, integral_constant<int, 2>{}); return;
+            case 4: count_r(lt, integral_constant<int, 4>{}); return;
+            case 8: count_r(lt, integral_constant<int, 8>{}); return;
         }
         throw Error(SPC5CUDA_ERR_FORMAT, "r must be 1, 2, 4 or 8");
     };
@@ -226,10 +246,10 @@ void launch_core_prep(int value_type, int r, int nbr, const int* brptr, const ui
     else count(double{});
     SPC5_CUDA(cudaGetLastError());
     if (before) {
-        k_core_tiles<<<1, THREADS, 0, s>>>(ntiles, stats, before);
+        k_core_parts<<<1, THREADS, 0, s>>>(nparts, stats, before);
         SPC5_CUDA(cudaGetLastError());
     }
-    launch_after(k_core_split, dim3(unsigned(ntiles)), THREADS, 0, !before, s, nbr, brptr, valptr,
+    launch_after(k_core_split, dim3(unsigned(ntiles)), THREADS, 0, !before, s, nbr, brptr, valptr, nparts, TILE / rows,
                  static_cast<const TileStats*>(stats), static_cast<const int*>(before), ngroups,
                  reinterpret_cast<int*>(mem + c.gstart), nwarps, reinterpret_cast<int*>(mem + c.wstart), value_type, r,
                  reinterpret_cast<int*>(mem + c.flag));
