@@ -64,9 +64,10 @@ inline void require(bool cond, spc5cuda_status s, const char* what) {
 
 
 // The sorted plan of an irregular matrix (plan.cu): the rows sorted by size,
-// the long rows stored as warp streams, the short rows one per lane
+// the long rows stored as warp streams or chains, the short rows one per lane
 // (stream.cuh); it holds the plan's only copy of the values.  Launches share
-// no state, so calls on different streams overlap freely.
+// no state (the chains' sums are scratch of the call), so calls on different
+// streams overlap freely.
 struct SortedPlan {
     static constexpr int CLASSES = 5;
     static constexpr int SHORT_VALUES = 16;
@@ -83,12 +84,25 @@ struct SortedPlan {
     int short_rows[SHORT_VALUES + 1] = {0};  // rows of n values; they follow the long ones
     int short_slabs = 0;
     long long_values = 0;
+    // the chain part: the first chain_rows sorted rows
+    int chain_rows = 0;
+    long nchains = 0;       // non-empty chains
+    long chain_values = 0;  // their values
+    Owned chain;            // all of it, in one buffer:
+    void* cval = nullptr;         // entries: values,
+    int* ccol = nullptr;          // x indices
+    int* clen = nullptr;          // per chain: entries,
+    int* cid = nullptr;           // id
+    long* cfirst = nullptr;       // chain slabs + 1: first entry of each
+    uint16_t* cmask = nullptr;    // per row: its non-empty chains
     long bytes() const {
         return long(perm.bytes + key.bytes + val.bytes + col.bytes + mask.bytes + sstep.bytes + sval.bytes +
-                    chains.bytes);
+                    chains.bytes + chain.bytes);
     }
-    // kernel launches of one SpMV: the long rows', the short rows'
-    int launches() const { return (slab_end[CLASSES - 1] > 0 ? 1 : 0) + (short_slabs > 0 ? 1 : 0); }
+    // kernel launches of one SpMV: the chains' and their rows', the long rows', the short rows'
+    int launches() const {
+        return (chain_rows > 0 ? 2 : 0) + (slab_end[CLASSES - 1] > 0 ? 1 : 0) + (short_slabs > 0 ? 1 : 0);
+    }
 };
 
 // The sorted plan of a converted matrix (synchronises s).

@@ -2,17 +2,20 @@
 //
 // Power-law and other irregular matrices mix block-rows of one block with
 // block-rows of hundreds; no single work split suits both.  The plan sorts the
-// rows of the matrix by size and stores the long ones as warp streams and the
-// short ones one per lane (stream.cuh): every chain of multiply-adds keeps its
-// values in block order, so y is bit-identical.  The plan holds the only copy
+// rows of the matrix by size and stores the long ones as warp streams or as chains
+// (chain_rows says which) and the short ones one per lane (stream.cuh): every chain
+// of multiply-adds keeps its values in block order, so y is bit-identical.  The plan holds the only copy
 // of the values; the handle keeps the reference-order headers, from which the
 // values can be put back in the reference order (rebuild_values).
 //
 // Build, all on the device: row-blocks and values of every row (k_row_stats),
 // a radix sort of the rows by size, the sizes of the long rows' slabs
 // (k_slab_size) and their scans, then one warp per slab writes its masks, x
-// indices and values (k_stream_fill, k_short_fill).
+// indices and values (k_stream_fill, k_short_fill).  The chains: their lengths
+// (k_chain_len), a radix sort by length class, the slabs (k_chain_slabs), then one
+// warp per row writes its entries (k_chain_fill).
 #include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_scan.cuh>
 
 #include <algorithm>
 
@@ -72,20 +75,38 @@ __global__ void __launch_bounds__(256) k_row_stats(int nrows, int nbr, const int
     }
 }
 
-// counts[j] = sorted rows of more than class_min(j) row-blocks (the last class
-// takes the long rows' rest); counts[CLASSES + n] = sorted rows of at least n
-// values (all long rows among them).
-__global__ void k_class_counts(int nrows, const int* __restrict__ key, int* __restrict__ counts) {
+constexpr int OCTAVES = CLASSES + SHORT_VALUES + 1;
+struct Counts {
+    int rows[OCTAVES + 31];
+    int longest;                // row-blocks of the longest row
+    unsigned long long blocks;  // of all long rows
+};
+
+// rows[j] = sorted rows of more than class_min(j) row-blocks (the last class
+// takes the long rows' rest); rows[CLASSES + n] = sorted rows of at least n
+// values (all long rows among them); rows[OCTAVES + b] = sorted rows of at least
+// 2^b row-blocks.
+__global__ void k_class_counts(int nrows, const int* __restrict__ key, Counts* __restrict__ out) {
+    unsigned long long blocks = 0;
     for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < nrows; i += long(gridDim.x) * blockDim.x) {
         const int k = key[i], next = i + 1 < nrows ? key[i + 1] : -1;
+        blocks += static_cast<unsigned long long>(max(k - LONG_KEY, 0));
+        if (i == 0) out->longest = max(k - LONG_KEY, 0);
         if (k == next) continue;
 #pragma unroll
         for (int j = 0; j < CLASSES; ++j) {
             const int least = LONG_KEY + class_min(j);
-            if (k > least && next <= least) counts[j] = int(i + 1);
+            if (k > least && next <= least) out->rows[j] = int(i + 1);
         }
-        for (int n = max(next + 1, 0); n <= min(k, SHORT_VALUES); ++n) counts[CLASSES + n] = int(i + 1);
+        for (int b = 0; b < 31; ++b) {
+            const long least = LONG_KEY + (1L << b);
+            if (k >= least && next < least) out->rows[OCTAVES + b] = int(i + 1);
+        }
+        for (int n = max(next + 1, 0); n <= min(k, SHORT_VALUES); ++n) out->rows[CLASSES + n] = int(i + 1);
     }
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) blocks += __shfl_xor_sync(FULL, blocks, d);
+    if ((threadIdx.x & 31) == 0 && blocks) atomicAdd(&out->blocks, blocks);
 }
 
 // Steps and values of every slab.
@@ -296,6 +317,151 @@ __global__ void __launch_bounds__(256) k_short_fill(View p, const int* __restric
     }
 }
 
+// Length class of a chain of n entries: n itself below 8, then eight classes per
+// octave (monotone in n; the lengths of one class differ by an eighth at most).
+__device__ __forceinline__ int length_class(int n) {
+    if (n < 8) return n;
+    const int b = 31 - __clz(n);
+    return 8 * (b - 2) + ((n >> (b - 3)) & 7);
+}
+constexpr int CLASS_BITS = 8;  // of a class: below 8 * 29
+
+// Chain ids i VS + c, their entries and length classes, and the rows' masks of
+// non-empty chains, for the first nrows sorted rows, a warp per row; totals: their
+// values, the non-empty chains.
+template <class LT, int R>
+__global__ void __launch_bounds__(256) k_chain_len(int nrows, const int* __restrict__ perm, const int* __restrict__ brptr,
+                                                   const uint8_t* __restrict__ hdr, int* __restrict__ len,
+                                                   int* __restrict__ cls, int* __restrict__ ids,
+                                                   uint16_t* __restrict__ mask, unsigned long long* __restrict__ totals) {
+    constexpr int VS = Layout<LT>::VS;
+    const int lane = threadIdx.x & 31;
+    const long warps = long(gridDim.x) * blockDim.x / 32;
+    for (long i = (long(blockIdx.x) * blockDim.x + threadIdx.x) / 32; i < nrows; i += warps) {
+        const int row = perm[i], br = row / R, s = row % R;
+        const long b1 = brptr[br + 1];
+        int n[VS];
+#pragma unroll
+        for (int c = 0; c < VS; ++c) n[c] = 0;
+        for (long b = brptr[br] + lane; b < b1; b += 32) {
+            uint32_t mw[Header<LT, R>::MASK_WORDS];
+            load_header<LT, R>(hdr, b, mw);
+            uint32_t m = 0u;
+#pragma unroll
+            for (int q = 0; q < R; ++q) m = q == s ? mask_of<LT, R>(mw, q) : m;
+#pragma unroll
+            for (int c = 0; c < VS; ++c) n[c] += int((m >> c) & 1u);
+        }
+        int mine = 0, all = 0;  // lane c: chain c
+#pragma unroll
+        for (int c = 0; c < VS; ++c) {
+            const int t = int(__reduce_add_sync(FULL, unsigned(n[c])));
+            mine = lane == c ? t : mine;
+            all += t;
+        }
+        const uint32_t some = __ballot_sync(FULL, lane < VS && mine > 0);
+        if (lane < VS) {
+            len[i * VS + lane] = mine;
+            cls[i * VS + lane] = length_class(mine);
+            ids[i * VS + lane] = int(i * VS + lane);
+        }
+        if (lane == 0) {
+            mask[i] = uint16_t(some);
+            atomicAdd(totals, static_cast<unsigned long long>(all));
+            atomicAdd(totals + 1, static_cast<unsigned long long>(__popc(some)));
+        }
+    }
+}
+
+// A warp per slab of sorted chains: their lengths, and the slab's entries (0 for
+// slab = nslabs).
+__global__ void __launch_bounds__(256) k_chain_slabs(long nchains, int nslabs, const int* __restrict__ id,
+                                                     const int* __restrict__ len_of, int* __restrict__ len,
+                                                     long* __restrict__ entries) {
+    const int lane = threadIdx.x & 31;
+    const long warps = long(gridDim.x) * blockDim.x / 32;
+    for (long slab = (long(blockIdx.x) * blockDim.x + threadIdx.x) / 32; slab <= nslabs; slab += warps) {
+        const long q = slab * 32 + lane;
+        const int n = q < nchains ? len_of[id[q]] : 0;
+        if (q < nchains) len[q] = n;
+        const int most = __reduce_max_sync(FULL, n);
+        if (lane == 0) entries[slab] = slab < nslabs ? long(chains_of(nchains, slab)) * most : 0L;
+    }
+}
+
+// place[id] = sorted place of every non-empty chain.
+__global__ void __launch_bounds__(256) k_chain_places(long nchains, const int* __restrict__ id, int* __restrict__ place) {
+    for (long q = long(blockIdx.x) * blockDim.x + threadIdx.x; q < nchains; q += long(gridDim.x) * blockDim.x)
+        place[id[q]] = int(q);
+}
+
+// The chains' entries, a warp per row, 32 blocks at a time (a value's entry is its
+// chain's entries in the blocks before).  BACK: the values only, back to the
+// reference order.
+template <class LT, int R, class V, bool BACK>
+__global__ void __launch_bounds__(256) k_chain_fill(int nrows, long nchains, const int* __restrict__ perm, const int* __restrict__ brptr,
+                                                    const int* __restrict__ valptr, const uint8_t* __restrict__ hdr,
+                                                    const uint16_t* __restrict__ mask, const int* __restrict__ place,
+                                                    const long* __restrict__ first, const V* __restrict__ in,
+                                                    V* __restrict__ out, int* __restrict__ xcol) {
+    constexpr int VS = Layout<LT>::VS;
+    const int lane = threadIdx.x & 31;
+    const uint32_t before = (1u << lane) - 1u;
+    const long warps = long(gridDim.x) * blockDim.x / 32;
+    for (long i = (long(blockIdx.x) * blockDim.x + threadIdx.x) / 32; i < nrows; i += warps) {
+        const int row = perm[i], br = row / R, s = row % R;
+        const int b1 = brptr[br + 1];
+        long v0 = valptr[br];
+        long next = 0;  // lane c: chain c's next entry, and the distance to the one after it
+        int pitch = 0;
+        if (lane < VS && (mask[i] >> lane) & 1u) {
+            const int q = place[i * VS + lane];
+            next = first[q / 32] + q % 32;
+            pitch = chains_of(nchains, q / 32);
+        }
+        for (int b0 = brptr[br]; b0 < b1; b0 += 32) {
+            int col = 0, tot = 0, low = 0;
+            uint32_t m = 0u;
+            if (b0 + lane < b1) {
+                uint32_t mw[Header<LT, R>::MASK_WORDS];
+                col = load_header<LT, R>(hdr, long(b0) + lane, mw);
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    const uint32_t mq = mask_of<LT, R>(mw, q);
+                    tot += __popc(mq);
+                    low += q < s ? __popc(mq) : 0;
+                    m = q == s ? mq : m;
+                }
+            }
+            int incl = tot;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int t = __shfl_up_sync(FULL, incl, d);
+                if (lane >= d) incl += t;
+            }
+            long ref = v0 + incl - tot + low;
+            int steps = 0;
+#pragma unroll
+            for (int c = 0; c < VS; ++c) {
+                const uint32_t has = __ballot_sync(FULL, (m >> c) & 1u);
+                const long e = __shfl_sync(FULL, next, c) + long(__shfl_sync(FULL, pitch, c)) * __popc(has & before);
+                if ((m >> c) & 1u) {
+                    if constexpr (BACK) {
+                        out[ref] = in[e];
+                    } else {
+                        out[e] = in[ref];
+                        xcol[e] = col + c;
+                    }
+                    ++ref;
+                }
+                steps = lane == c ? __popc(has) : steps;
+            }
+            next += long(pitch) * steps;
+            v0 += __shfl_sync(FULL, incl, 31);
+        }
+    }
+}
+
 // Calls f(layout tag, std::integral_constant<int, R>, value tag) for a handle.
 template <class F>
 void dispatch_layout(const spc5cuda_mat* m, F&& f) {
@@ -315,6 +481,109 @@ void dispatch_layout(const spc5cuda_mat* m, F&& f) {
     }
 }
 
+// Sorted rows of the chain part.  All long rows where they are about as long as one
+// another: a stream's step has a lane per column of a row-block, most of them
+// idle at few values per row-block, and a chain's lanes idle only where chains
+// differ.  Else the streams share a row-block's sectors, and the few longest rows
+// are chains if their steps, one after the other, would outlast the rest.
+// Measured on B200 (us per SpMV, FP64, streams / chains): 50,000 rows of 400 random
+// values 157 / 63, 1,000,000 of 40 400 / 178, 20,000 of 100 runs of 8 64 / 39;
+// longest row at 24 (1M power-law) and 50 times (log-normal) the mean, all long rows
+// as chains 111 / 138 and 312 / 520.
+int chain_rows(const spc5cuda_mat* m, const Counts& c) {
+    const int rows = c.rows[CLASSES - 1], vs = vs_of(m->value_type);
+    if (rows == 0 || long(rows) * vs >= 1L << 31) return 0;  // (chain ids are int)
+    if (c.longest <= 8.0 * double(c.blocks) / rows) return rows;
+    // about 31 ps per warp step (of G row-blocks) and 3.2 ps per value for all rows;
+    // 50 ns per step of one row, of which all above half that time go to the chains.  Power-law of 20,000 rows, rows of more than 32
+    // row-blocks: 45 us, now 31; 100,000 rows, 128: 64 / 50; 300,000, 512: 84 / 84
+    const int G = 32 / vs;
+    const double rest_us = 31e-6 * double(c.blocks) / G + 3.2e-6 * double(m->nnz);
+    if (50e-3 * c.longest < 2.0 * rest_us) return 0;
+    for (int b = 4; b < 31; ++b)
+        if (2.0 * 50e-3 * double(1L << b) >= rest_us) return c.rows[OCTAVES + b];
+    return 0;
+}
+
+int warps_for(long n) { return grid_for(n * 32, 256); }
+
+// The chain part of the first p.chain_rows sorted rows (synchronises s).
+void build_chains(const spc5cuda_mat* m, SortedPlan& p, cudaStream_t s) {
+    const int vs = vs_of(m->value_type), rows = p.chain_rows;
+    const long nids = long(rows) * vs;
+    const size_t id_ints = sizeof(int) * size_t(nids);
+    DevBuf len(id_ints, s), cls(id_ints, s), ids(id_ints, s), sorted(id_ints, s), order(id_ints, s),
+        totals(2 * sizeof(long), s), mask(sizeof(uint16_t) * size_t(rows), s);
+    SPC5_CUDA(cudaMemsetAsync(totals.p, 0, totals.bytes, s));
+    dispatch_layout(m, [&](auto lt, auto RC, auto) {
+        k_chain_len<decltype(lt), decltype(RC)::value><<<warps_for(rows), 256, 0, s>>>(
+            rows, p.perm.as<int>(), m->brptr.as<int>(), m->headers.as<uint8_t>(), len.as<int>(), cls.as<int>(),
+            ids.as<int>(), mask.as<uint16_t>(), totals.as<unsigned long long>());
+    });
+    SPC5_CUDA(cudaGetLastError());
+    size_t temp = 0;
+    SPC5_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, temp, cls.as<int>(), sorted.as<int>(), ids.as<int>(),
+                                                        order.as<int>(), int(nids), 0, CLASS_BITS, s));
+    DevBuf tmp(temp, s);
+    SPC5_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.p, temp, cls.as<int>(), sorted.as<int>(), ids.as<int>(),
+                                                        order.as<int>(), int(nids), 0, CLASS_BITS, s));
+    long sums[2] = {0, 0};
+    SPC5_CUDA(cudaMemcpyAsync(sums, totals.p, sizeof(sums), cudaMemcpyDeviceToHost, s));
+    SPC5_CUDA(cudaStreamSynchronize(s));
+    p.chain_values = sums[0];
+    p.nchains = sums[1];
+    const int slabs = div_up(p.nchains, 32);
+    DevBuf entries(sizeof(long) * size_t(slabs + 1), s), first(sizeof(long) * size_t(slabs + 1), s);
+    k_chain_slabs<<<warps_for(slabs + 1L), 256, 0, s>>>(p.nchains, slabs, order.as<int>(), len.as<int>(),
+                                                        sorted.as<int>(), entries.as<long>());
+    SPC5_CUDA(cudaGetLastError());
+    SPC5_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, entries.as<long>(), first.as<long>(), slabs + 1, s));
+    DevBuf scan(temp, s);
+    SPC5_CUDA(cub::DeviceScan::ExclusiveSum(scan.p, temp, entries.as<long>(), first.as<long>(), slabs + 1, s));
+    long total = 0;
+    SPC5_CUDA(cudaMemcpyAsync(&total, first.as<long>() + slabs, sizeof(long), cudaMemcpyDeviceToHost, s));
+    SPC5_CUDA(cudaStreamSynchronize(s));
+    // ---- the buffer and what is known of it (the entries: fill_chains)
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t here = at;
+        at += (bytes + 255) / 256 * 256;
+        return here;
+    };
+    const size_t chain_ints = sizeof(int) * size_t(p.nchains);
+    const size_t a_first = take(first.bytes), a_val = take(size_t(value_bytes_of(m->value_type)) * size_t(total)),
+                 a_col = take(sizeof(int) * size_t(total)), a_len = take(chain_ints), a_id = take(chain_ints),
+                 a_mask = take(mask.bytes);
+    p.chain.alloc(at);
+    unsigned char* base = p.chain.as<unsigned char>();
+    p.cfirst = reinterpret_cast<long*>(base + a_first);
+    p.cval = base + a_val;
+    p.ccol = reinterpret_cast<int*>(base + a_col);
+    p.clen = reinterpret_cast<int*>(base + a_len);
+    p.cid = reinterpret_cast<int*>(base + a_id);
+    p.cmask = reinterpret_cast<uint16_t*>(base + a_mask);
+    SPC5_CUDA(cudaMemcpyAsync(p.cfirst, first.p, first.bytes, cudaMemcpyDeviceToDevice, s));
+    SPC5_CUDA(cudaMemcpyAsync(p.clen, sorted.p, chain_ints, cudaMemcpyDeviceToDevice, s));
+    SPC5_CUDA(cudaMemcpyAsync(p.cid, order.p, chain_ints, cudaMemcpyDeviceToDevice, s));
+    SPC5_CUDA(cudaMemcpyAsync(p.cmask, mask.p, mask.bytes, cudaMemcpyDeviceToDevice, s));
+}
+
+// The chains' values: from the reference order (in) to the chains and their x
+// indices, or (BACK) from the chains to the reference order (out).
+template <bool BACK>
+void fill_chains(const spc5cuda_mat* m, const SortedPlan& p, const void* in, void* out, cudaStream_t s) {
+    DevBuf place(sizeof(int) * size_t(p.chain_rows) * size_t(vs_of(m->value_type)), s);
+    k_chain_places<<<grid_for(p.nchains, 256), 256, 0, s>>>(p.nchains, p.cid, place.as<int>());
+    dispatch_layout(m, [&](auto lt, auto RC, auto val) {
+        using V = decltype(val);
+        k_chain_fill<decltype(lt), decltype(RC)::value, V, BACK><<<warps_for(p.chain_rows), 256, 0, s>>>(
+            p.chain_rows, p.nchains, p.perm.as<int>(), m->brptr.as<int>(), m->valptr.as<int>(),
+            m->headers.as<uint8_t>(), p.cmask, place.as<int>(), p.cfirst, static_cast<const V*>(in), static_cast<V*>(out),
+            BACK ? nullptr : p.ccol);
+    });
+    SPC5_CUDA(cudaGetLastError());
+}
+
 }  // namespace
 
 void build_sorted_plan(spc5cuda_mat* m, cudaStream_t s) {
@@ -330,10 +599,11 @@ void build_sorted_plan(spc5cuda_mat* m, cudaStream_t s) {
     p.perm.alloc(row_ints);
     p.key.alloc(row_ints);
     DevBuf rv(row_ints, s);
-    int counts[CLASSES + SHORT_VALUES + 1] = {0};
+    Counts found{};
+    const int* counts = found.rows;
     {
         // ---- the rows by size, largest first (stable)
-        DevBuf key(row_ints, s), ids(row_ints, s), dc(sizeof(counts), s);
+        DevBuf key(row_ints, s), ids(row_ints, s), dc(sizeof(Counts), s);
         dispatch_layout(m, [&](auto lt, auto RC, auto) {
             using LT = decltype(lt);
             constexpr int VS = Layout<LT>::VS;
@@ -348,13 +618,15 @@ void build_sorted_plan(spc5cuda_mat* m, cudaStream_t s) {
         SPC5_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.p, temp, key.as<int>(), p.key.as<int>(),
                                                             ids.as<int>(), p.perm.as<int>(), nrows, 0, 31, s));
         SPC5_CUDA(cudaMemsetAsync(dc.p, 0, dc.bytes, s));
-        k_class_counts<<<grid_for(nrows, 256), 256, 0, s>>>(nrows, p.key.as<int>(), dc.as<int>());
+        k_class_counts<<<grid_for(nrows, 256), 256, 0, s>>>(nrows, p.key.as<int>(), dc.as<Counts>());
         SPC5_CUDA(cudaGetLastError());
-        SPC5_CUDA(cudaMemcpyAsync(counts, dc.p, dc.bytes, cudaMemcpyDeviceToHost, s));
+        SPC5_CUDA(cudaMemcpyAsync(&found, dc.p, sizeof(found), cudaMemcpyDeviceToHost, s));
         SPC5_CUDA(cudaStreamSynchronize(s));
     }
+    p.chain_rows = chain_rows(m, found);
+    if (p.chain_rows > 0) build_chains(m, p, s);
     // ---- classes (a class without rows ends where the one before it ends)
-    int rows = 0, slabs = 0;
+    int rows = p.chain_rows, slabs = 0;
     for (int j = 0; j < CLASSES; ++j) {
         const int end = std::max(rows, counts[j]);
         slabs += div_up(end - rows, G * class_rounds(j));
@@ -410,13 +682,14 @@ void build_sorted_plan(spc5cuda_mat* m, cudaStream_t s) {
                 p.val.as<V>(), p.chains.as<uint16_t>(), p.col.as<int>());
     });
     SPC5_CUDA(cudaGetLastError());
+    if (p.chain_rows > 0) fill_chains<false>(m, p, m->values.p, p.cval, s);
     SPC5_CUDA(cudaStreamSynchronize(s));
     m->plan = std::move(plan);
     // the streams serve every SpMV now: the reference-order values are put
     // back together when a call needs them (restore_values), if the rows hold
     // all of them (the caller's arrays may hold more: values of the rows past
     // the last one of a block-row that is not full, or past the masks')
-    long held = m->plan->long_values;
+    long held = m->plan->chain_values + m->plan->long_values;
     for (int n = 0; n <= SHORT_VALUES; ++n) held += long(n) * m->plan->short_rows[n];
     if (m->use_plan() && held == m->nnz) {
         m->values.release();
@@ -441,6 +714,7 @@ void rebuild_values(const spc5cuda_mat* m, void* values, cudaStream_t s) {
                 static_cast<V*>(values), nullptr, nullptr);
     });
     SPC5_CUDA(cudaGetLastError());
+    if (p.chain_rows > 0) fill_chains<true>(m, p, p.cval, values, s);
 }
 
 }  // namespace spc5cuda

@@ -1,5 +1,5 @@
 // stream.cu -- SpMV and SpMM over the sorted plan (stream.cuh; plan.cu builds
-// it).
+// it; chain.cuh has the kernels of its chain part).
 //
 // Arithmetic (bit-identical to the reference kernels core_SPC5_{r}rVc_Spmv_*,
 // src/spc5.hpp:2309-2715): every (row, column class c) chain is one
@@ -8,13 +8,18 @@
 // is the _mm512_reduce_add tree over its VS accumulators (+0 for a class
 // without values) and y[row] += sum.
 //
-// What bounds it: an x gather costs one L2 -> L1 sector (32 bytes) per
-// distinct sector that its instruction touches, about one per cycle and SM on
-// a B200.  The long rows' streams keep a row-block's columns side by side, so
-// that n neighbouring columns cost 1 + (n - 1) / 4 sectors instead of n.
+// What bounds it: latency.  In a window of steps the index loads, the x gathers and
+// the multiply-adds follow one another, and the longest rows are the tail (power-law
+// of 1,000,000 rows on a B200: L1 45%, issue 33%, 22% of the warps active).  An x
+// gather costs one L2 -> L1 sector (32 bytes) per distinct sector that its
+// instruction touches, about one per cycle and SM; the long rows' streams keep a
+// row-block's columns side by side, so that n neighbouring columns cost 1 + (n - 1) /
+// 4 sectors instead of n.
 #include <algorithm>
+#include <memory>
 #include <type_traits>
 
+#include "chain.cuh"
 #include "stream.cuh"
 
 namespace spc5cuda {
@@ -25,10 +30,6 @@ using namespace stream;
 
 constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
-
-// y[row] += sum: red.add.f64 (y + sum rounded once) or load, add, store.
-__device__ __forceinline__ void add_to(double* y, double v) { atomicAdd(y, v); }
-__device__ __forceinline__ void add_to(float* y, float v) { *y = *y + v; }
 
 // The long rows' SpMV: steps per window, staged values (at least one step's 32),
 // gathers in flight per lane, steps per multiply-add batch, CTAs per SM asked
@@ -89,27 +90,20 @@ __device__ __forceinline__ void ld_if(uint4& v, const void* p, uint32_t on) {
                  : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"(on));
 }
 
-// The kernels of one SpMV or SpMM write disjoint rows of y: each lets the next
-// one begin while its own last warps run (the longest rows decide when a
-// kernel ends), and the last block of a kernel that follows another waits for
-// the one before it, so that the end of the last launch is the end of all.
-// (That block's first warp always has a slab and reaches end_launch.)
-__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void end_launch(bool follows) {
-    if (follows && blockIdx.x == gridDim.x - 1)
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // (launch_after, with this file's CTA.)
 template <class... P, class... Q>
 void launch(void (*kern)(P...), dim3 grid, bool follows, cudaStream_t s, Q... args) {
     launch_after(kern, grid, THREADS, 0, follows, s, args...);
 }
 
-// The long rows: one warp per slab.
-template <class V, class X, class A, class Y, int VS>
+// The long rows: one warp per slab.  STRIDED: a column of row-major X and Y, element
+// i at i ldx and i ldy.  FOLLOWS: after another launch of the product (a kernel of its
+// own: with the wait at its end the 1,000,000-row power-law matrix, 8-column mixed
+// layout, took 118 us instead of 109).
+template <class V, class X, class A, class Y, int VS, bool STRIDED, bool FOLLOWS>
 __global__ void __launch_bounds__(THREADS, LONG_CTAS)
-    k_stream_spmv(const __grid_constant__ View p, const V* __restrict__ val, const X* __restrict__ x, Y* __restrict__ y) {
+    k_stream_spmv(const __grid_constant__ View p, const V* __restrict__ val, const X* __restrict__ x, long ldx,
+                  Y* __restrict__ y, long ldy) {
     using Buf = WarpBuf<V, X>;
     griddep_launch();
     constexpr int G = 32 / VS;
@@ -140,7 +134,7 @@ __global__ void __launch_bounds__(THREADS, LONG_CTAS)
 #pragma unroll
         for (int d = VS / 2; d >= 1; d >>= 1) acc = acc + __shfl_xor_sync(FULL, acc, d);
         const int yrow = __shfl_sync(FULL, row, (q * G + g) & 31);
-        if (c == 0 && q * G + g < nrows) add_to(y + yrow, Y(acc));
+        if (c == 0 && q * G + g < nrows) add_to(STRIDED ? y + long(yrow) * ldy : y + yrow, Y(acc));
         acc = A(0);
         ++q;
         end += __shfl_sync(FULL, nb, q);
@@ -192,7 +186,7 @@ __global__ void __launch_bounds__(THREADS, LONG_CTAS)
                 }
 #pragma unroll
                 for (int u = 0; u < UG; ++u)
-                    if (i0 + u * 32 + lane < nv) xv[u] = ld_x(x + col[u], pol_x);
+                    if (i0 + u * 32 + lane < nv) xv[u] = ld_x(STRIDED ? x + long(col[u]) * ldx : x + col[u], pol_x);
 #pragma unroll
                 for (int u = 0; u < UG; ++u) {
                     const int i = i0 + u * 32 + lane;
@@ -231,15 +225,16 @@ __global__ void __launch_bounds__(THREADS, LONG_CTAS)
         }
         base += total;
     }
+    if constexpr (FOLLOWS) end_launch(true);
 }
 
 // The short rows: one warp per slab, one lane per row.  A lane runs its chains
 // one after the other and leaves their results in its own column of shared
 // memory, in chain order (slot 0 takes what precedes the first chain).
-template <class V, class X, class A, class Y, int VS>
+template <class V, class X, class A, class Y, int VS, bool STRIDED>
 __global__ void __launch_bounds__(THREADS, SHORT_CTAS)
-    k_short_spmv(const __grid_constant__ View p, const V* __restrict__ val, const X* __restrict__ x,
-                 Y* __restrict__ y, bool follows) {
+    k_short_spmv(const __grid_constant__ View p, const V* __restrict__ val, const X* __restrict__ x, long ldx,
+                 Y* __restrict__ y, long ldy, bool follows) {
     griddep_launch();
     __shared__ A chain[WARPS][VS + 1][32];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -267,7 +262,10 @@ __global__ void __launch_bounds__(THREADS, SHORT_CTAS)
             }
 #pragma unroll
             for (int u = 0; u < SU; ++u)
-                if (live && j0 + u < sr.len) xv[u] = ld_x(x + (uint32_t(col[u]) & ~FIRST), pol_x);
+                if (live && j0 + u < sr.len) {
+                    const uint32_t xi = uint32_t(col[u]) & ~FIRST;
+                    xv[u] = ld_x(STRIDED ? x + long(xi) * ldx : x + xi, pol_x);
+                }
 #pragma unroll
             for (int u = 0; u < SU; ++u) {
                 if (live && j0 + u < sr.len) {
@@ -290,7 +288,7 @@ __global__ void __launch_bounds__(THREADS, SHORT_CTAS)
 #pragma unroll
             for (int k = 0; k < d; ++k) a[k] = a[k] + a[k + d];
         }
-        if (live) add_to(y + row, Y(a[0]));
+        if (live) add_to(STRIDED ? y + long(row) * ldy : y + row, Y(a[0]));
     }
     end_launch(follows);
 }
@@ -532,15 +530,38 @@ __global__ void __launch_bounds__(THREADS) k_short_spmm(const __grid_constant__ 
     end_launch(follows);
 }
 
+// The streams and the short rows for one x; follows: a launch of this product came before.
+template <class V, class X, class A, class Y, int VS, bool STRIDED>
+void run_rows(const SortedPlan& p, const X* x, long ldx, Y* y, long ldy, bool& follows, cudaStream_t s) {
+    const View v = view_of(p);
+    const V* val = p.val.as<V>();
+    if (v.long_slabs() > 0) {
+        auto kern = follows ? k_stream_spmv<V, X, A, Y, VS, STRIDED, true> : k_stream_spmv<V, X, A, Y, VS, STRIDED, false>;
+        launch(kern, dim3(div_up(v.long_slabs(), WARPS)), follows, s, v, val, x, ldx, y, ldy);
+        follows = true;
+    }
+    if (v.short_slabs() > 0) {
+        launch(k_short_spmv<V, X, A, Y, VS, STRIDED>, dim3(div_up(v.short_slabs(), WARPS)), follows, s, v, val, x, ldx, y,
+               ldy, follows);
+        follows = true;
+    }
+}
+
 template <class V, class X, class A, class Y, int VS>
 void run_spmv(const spc5cuda_mat* m, const X* x, Y* y, cudaStream_t s) {
     const SortedPlan& p = *m->plan;
-    const View v = view_of(p);
-    const V* val = p.val.as<V>();
-    const bool longs = v.long_slabs() > 0;
-    if (longs) launch(k_stream_spmv<V, X, A, Y, VS>, dim3(div_up(v.long_slabs(), WARPS)), false, s, v, val, x, y);
-    if (v.short_slabs() > 0)
-        launch(k_short_spmv<V, X, A, Y, VS>, dim3(div_up(v.short_slabs(), WARPS)), longs, s, v, val, x, y, longs);
+    bool follows = false;
+    if (p.chain_rows == 0) {
+        run_rows<V, X, A, Y, VS, false>(p, x, 1L, y, 1L, follows, s);
+        return;
+    }
+    const ChainView c = chain_view_of(p);
+    PoolBuf sums(sizeof(A) * size_t(c.rows) * VS, s);
+    auto kern = c.slabs <= 8 * sm_count() ? k_chain_spmv<V, X, A, CHAIN_DEEP> : k_chain_spmv<V, X, A, CHAIN_U>;
+    launch(kern, dim3(div_up(c.slabs, CHAIN_THREADS / 32)), false, s, c, static_cast<const V*>(p.cval), x, sums.as<A>());
+    follows = true;
+    run_rows<V, X, A, Y, VS, false>(p, x, 1L, y, 1L, follows, s);
+    launch(k_chain_rows<A, Y, VS, 1>, dim3(div_up(c.rows, CHAIN_THREADS)), false, s, c, 1, sums.as<A>(), y, 1L, 1L);
 }
 
 template <class V, class X, class A, class Y, int VS>
@@ -575,9 +596,31 @@ void run_spmm(const spc5cuda_mat* m, int k, const X* x, long ldx, long xcs, Y* y
             launch(k_short_spmm<V, X, A, Y, VS, decltype(kcc)::value>, dim3(div_up(v.short_slabs(), WARPS)), follows, s,
                    v, val, kc, xp, ldx, xcs, yp, ldy, ycs, follows);
     };
+    // the chain part's launches, before and after the others
+    std::unique_ptr<PoolBuf> sums;
+    auto chains = [&](auto kcc, int kc, const X* xp) {
+        constexpr int KC = decltype(kcc)::value;
+        if (p.chain_rows == 0) return;
+        const ChainView c = chain_view_of(p);
+        const size_t bytes = sizeof(A) * size_t(c.rows) * VS * KC;
+        if (!sums || sums->bytes < bytes) sums = std::make_unique<PoolBuf>(bytes, s);
+        const int warps = div_up(c.chains, 32 / KC);
+        launch(k_chain_spmm<V, X, A, KC>, dim3(div_up(warps, CHAIN_THREADS / 32)), false, s, c,
+               static_cast<const V*>(p.cval), kc, xp, ldx, xcs, sums->as<A>());
+        follows = true;
+    };
+    auto chain_rows = [&](auto kcc, int kc, Y* yp) {
+        constexpr int KC = decltype(kcc)::value;
+        if (p.chain_rows == 0) return;
+        launch(k_chain_rows<A, Y, VS, KC>, dim3(div_up(long(p.chain_rows) * KC, CHAIN_THREADS)), false, s,
+               chain_view_of(p), kc, sums->as<A>(), yp, ldy, ycs);
+    };
     using std::integral_constant;
+    // right-hand sides per pass: 16, fewer where the chains' scratch would be more than 1 GiB
+    int per = 16;
+    while (per > 4 && sizeof(A) * size_t(p.chain_rows) * VS * size_t(per) > (size_t(1) << 30)) per /= 2;
     for (int q0 = 0; q0 < k;) {
-        const int kc = std::min(16, k - q0);
+        const int kc = std::min(per, k - q0);
         follows = false;
         const X* xp = x + long(q0) * xcs;
         Y* yp = y + long(q0) * ycs;
@@ -586,17 +629,23 @@ void run_spmm(const spc5cuda_mat* m, int k, const X* x, long ldx, long xcs, Y* y
         constexpr integral_constant<int, 1> one{};
         constexpr integral_constant<int, 4> deep{};
         if (kc > 8) {
+            chains(integral_constant<int, 16>{}, kc, xp);
             longs(integral_constant<int, 16 / G>{}, deep, one, 0, a, kc, xp, yp);
             longs(integral_constant<int, 16 / G>{}, one, all, a, b, kc, xp, yp);
             shorts(integral_constant<int, 16>{}, kc, xp, yp);
+            chain_rows(integral_constant<int, 16>{}, kc, yp);
         } else if (kc > 4) {
+            chains(integral_constant<int, 8>{}, kc, xp);
             longs(integral_constant<int, 8 / G>{}, deep, one, 0, a, kc, xp, yp);
             longs(integral_constant<int, 8 / G>{}, integral_constant<int, 2>{}, all, a, b, kc, xp, yp);
             shorts(integral_constant<int, 8>{}, kc, xp, yp);
+            chain_rows(integral_constant<int, 8>{}, kc, yp);
         } else {
+            chains(integral_constant<int, 4>{}, kc, xp);
             longs(integral_constant<int, 4 / G>{}, integral_constant<int, 8>{}, one, 0, a, kc, xp, yp);
             longs(integral_constant<int, 4 / G>{}, integral_constant<int, 2>{}, all, a, b, kc, xp, yp);
             shorts(integral_constant<int, 4>{}, kc, xp, yp);
+            chain_rows(integral_constant<int, 4>{}, kc, yp);
         }
         q0 += kc;
     }

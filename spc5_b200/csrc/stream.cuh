@@ -18,6 +18,14 @@
 // rounds of G rows.  Rows of more than 32 row-blocks run one round per slab;
 // shorter ones 2, 4, 8 or 16 rounds, so that a slab has about 32 to 64 steps.
 //
+// Chain part: the first sorted rows of a plan may be stored as their (row, column)
+// chains instead: chain (sorted row i, column c) has id i VS + c and holds the
+// row's values in column c of its blocks, in block order, each with its x index.
+// The non-empty chains are sorted by length class (length_class, longest first,
+// stable, so that neighbouring lanes often run neighbouring columns of a row) and
+// cut into slabs of 32 (the last one of n), one lane per chain: entry j of lane l is
+// at the slab's first entry + 32 j + l (n j + l), with room for the longest chain.
+//
 // Short rows: one lane per row, 32 rows of the same number of values per slab
 // (the last slab of a length has fewer); entry j of lane l is at the slab's
 // first entry + 32 j + l.  A row's entries are in chain order -- column class 0
@@ -40,7 +48,8 @@ constexpr int CLASSES = SortedPlan::CLASSES;  // long rows of > 32, > 16, > 8, >
 __host__ __device__ constexpr int class_rounds(int j) { return 1 << j; }  // ... run 1, 2, 4, 8, 16 rounds per slab
 __host__ __device__ constexpr int class_min(int j) { return j < CLASSES - 1 ? 32 >> j : 0; }  // class j: more than this
 
-// Device pointers of a plan.
+// Device pointers of a plan without its chain part (sorted rows are counted from the
+// first one after that).
 struct View {
     const uint32_t* mask;
     const int* col;
@@ -66,11 +75,11 @@ inline View view_of(const SortedPlan& p) {
     v.col = p.col.as<int>();
     v.sstep = p.sstep.as<int>();
     v.sval = p.sval.as<int>();
-    v.key = p.key.as<int>();
-    v.perm = p.perm.as<int>();
+    v.key = p.key.as<int>() + p.chain_rows;
+    v.perm = p.perm.as<int>() + p.chain_rows;
     v.chains = p.chains.as<uint16_t>();
     for (int j = 0; j < CLASSES; ++j) {
-        v.row_end[j] = p.row_end[j];
+        v.row_end[j] = p.row_end[j] - p.chain_rows;
         v.slab_end[j] = p.slab_end[j];
     }
     int row = v.long_rows(), slab = 0;
@@ -88,6 +97,42 @@ inline View view_of(const SortedPlan& p) {
     v.short_slab[0] = slab;
     return v;
 }
+
+// Chains of a slab.
+__host__ __device__ inline int chains_of(long nchains, long slab) {
+    const long left = nchains - slab * 32;
+    return left < 32 ? int(left) : 32;
+}
+
+// Device pointers of the chain part.
+struct ChainView {
+    const int* len;       // entries of every chain
+    const int* id;        // its id
+    const long* first;    // first entry of every slab
+    const int* col;       // x indices
+    const uint16_t* mask; // non-empty chains of every row
+    const int* perm;
+    int rows, slabs;
+    long chains;
+};
+
+inline ChainView chain_view_of(const SortedPlan& p) {
+    ChainView v;
+    v.len = p.clen;
+    v.id = p.cid;
+    v.first = p.cfirst;
+    v.col = p.ccol;
+    v.mask = p.cmask;
+    v.perm = p.perm.as<int>();
+    v.rows = p.chain_rows;
+    v.slabs = div_up(p.nchains, 32);
+    v.chains = p.nchains;
+    return v;
+}
+
+// y[row] += sum: red.add.f64 (y + sum rounded once) or load, add, store.
+__device__ __forceinline__ void add_to(double* y, double v) { atomicAdd(y, v); }
+__device__ __forceinline__ void add_to(float* y, float v) { *y = *y + v; }
 
 // First sorted row, end of the sorted rows and rounds of a slab of long rows.
 struct SlabRows {
