@@ -530,6 +530,11 @@ __global__ void __launch_bounds__(THREADS) k_short_spmm(const __grid_constant__ 
     end_launch(follows);
 }
 
+// Two right-hand sides run as an SpMV each from this many values in the streams on
+// (power-law on B200, FP64, r = 1, us: 300,000 rows, 3.2M values 152 together, 178 one
+// after the other; 1,000,000 rows 440, 193).
+constexpr long PAIR_VALUES = 4L << 20;
+
 // The streams and the short rows for one x; follows: a launch of this product came before.
 template <class V, class X, class A, class Y, int VS, bool STRIDED>
 void run_rows(const SortedPlan& p, const X* x, long ldx, Y* y, long ldy, bool& follows, cudaStream_t s) {
@@ -624,6 +629,10 @@ void run_spmm(const spc5cuda_mat* m, int k, const X* x, long ldx, long xcs, Y* y
         follows = false;
         const X* xp = x + long(q0) * xcs;
         Y* yp = y + long(q0) * ycs;
+        if (k - q0 == 1 && ldx == 1 && ldy == 1) {  // one contiguous right-hand side
+            run_spmv<V, X, A, Y, VS>(m, xp, yp, s);
+            return;
+        }
         const int a = v.slab_end[0], b = v.long_slabs();
         constexpr integral_constant<int, G> all{};
         constexpr integral_constant<int, 1> one{};
@@ -640,6 +649,12 @@ void run_spmm(const spc5cuda_mat* m, int k, const X* x, long ldx, long xcs, Y* y
             longs(integral_constant<int, 8 / G>{}, integral_constant<int, 2>{}, all, a, b, kc, xp, yp);
             shorts(integral_constant<int, 8>{}, kc, xp, yp);
             chain_rows(integral_constant<int, 8>{}, kc, yp);
+        } else if (kc == 1 || (kc == 2 && p.long_values >= PAIR_VALUES)) {
+            // an SpMV each
+            chains(integral_constant<int, 2>{}, kc, xp);
+            for (int j = 0; j < kc; ++j)
+                run_rows<V, X, A, Y, VS, true>(p, xp + j * xcs, ldx, yp + j * ycs, ldy, follows, s);
+            chain_rows(integral_constant<int, 2>{}, kc, yp);
         } else {
             chains(integral_constant<int, 4>{}, kc, xp);
             longs(integral_constant<int, 4 / G>{}, integral_constant<int, 8>{}, one, 0, a, kc, xp, yp);
