@@ -364,9 +364,11 @@ typedef struct spc5cuda_server_stats {
 SPC5CUDA_API spc5cuda_status spc5cuda_server_create(spc5cuda_server** out,
                                                     const spc5cuda_server_config* cfg);
 /* Registers a converted matrix (the handle stays owned by the caller and
- * must outlive the server).  SPC5CUDA_ERR_NOMEM when the resident bytes
- * plus staging would exceed the HBM budget.  Only while no request is in
- * flight. */
+ * must outlive the server).  A matrix with the sorted plan by default that
+ * fits the HBM budget only without it is switched to the group kernel
+ * (spc5cuda_mat_set_kernel: no call may use the handle meanwhile).
+ * SPC5CUDA_ERR_NOMEM when the resident bytes plus staging would exceed the
+ * budget even so.  Only while no request is in flight. */
 SPC5CUDA_API spc5cuda_status spc5cuda_server_add_matrix(spc5cuda_server* srv, spc5cuda_mat* mat,
                                                         int* id);
 SPC5CUDA_API spc5cuda_status spc5cuda_server_submit(spc5cuda_server* srv, int id, const void* x,

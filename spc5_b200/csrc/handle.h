@@ -218,6 +218,11 @@ struct spc5cuda_mat {
         return long(rowptr.bytes + colidx.bytes + values.bytes + brptr.bytes + headers.bytes +
                     valptr.bytes + gstart.bytes + wstart.bytes) + (plan ? plan->bytes() : 0L);
     }
+    // The same without a plan: the reference order alone.
+    long beta_bytes() const {
+        return device_bytes() - (plan ? plan->bytes() : 0L) +
+               (values_dropped ? std::max(long(value_bytes()), 16L) : 0L);
+    }
     // The per-group block-row ranges for the current device, and the per-warp
     // ranges of the thread-per-sub-row kernel when every block-row fits it.
     void build_partition(cudaStream_t s) {

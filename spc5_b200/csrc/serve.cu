@@ -325,8 +325,14 @@ spc5cuda_status spc5cuda_server_add_matrix(spc5cuda_server* sv, spc5cuda_mat* m,
         require(sv->inflight == 0, SPC5CUDA_ERR_INVALID, "add matrices while the server is idle");
         const int rows = std::max(sv->max_rows, m->nrows);
         const int cols = std::max(sv->max_cols, m->ncols);
-        const long need = sv->resident_bytes + m->device_bytes() + sv->slot_bytes(rows, cols);
-        require(need <= sv->cfg.hbm_budget, SPC5CUDA_ERR_NOMEM, "HBM budget exceeded");
+        const long room = sv->cfg.hbm_budget - sv->resident_bytes - sv->slot_bytes(rows, cols);
+        if (m->device_bytes() > room && m->kernel == SPC5CUDA_KERNEL_AUTO && m->use_plan() && m->beta_bytes() <= room) {
+            // the sorted plan keeps an x index beside every value: without room for it
+            // the matrix is served from its beta arrays, by the group kernel
+            const spc5cuda_status st = spc5cuda_mat_set_kernel(m, SPC5CUDA_KERNEL_GROUPS);
+            if (st != SPC5CUDA_OK) throw Error(st, "spc5cuda_mat_set_kernel");
+        }
+        require(m->device_bytes() <= room, SPC5CUDA_ERR_NOMEM, "HBM budget exceeded");
         if (rows != sv->max_rows || cols != sv->max_cols) {
             const size_t xb = sv->cfg.mixed ? 4 : 8;
             for (auto& sl : sv->slots) {
