@@ -36,6 +36,7 @@ struct SubRowOf {
 #pragma unroll
         for (int w = 0; w < MW; ++w) low[w] = w < wq ? 0xFFFFFFFFu : (w == wq ? (1u << sh) - 1u : 0u);
     }
+    static_assert(MW == 1 || MW == 2 || MW == 4, "mask words of a block");
     // the block at header offset off, empty when !ok
     __device__ __forceinline__ void load(const uint32_t* hw, int off, bool ok, Block<LT, R>& b) const {
         constexpr uint32_t FMASK = MB == 1 ? 0xFFu : 0xFFFFu;
@@ -43,9 +44,13 @@ struct SubRowOf {
 #pragma unroll
         for (int w = 0; w < MW; ++w) b.mw[w] = 0u;
         if (ok) b.col = rows::decode_staged<LT, R>(hw, off, b.mw);
+        // (a select per word: a loop of them became an array in local memory at four words)
         uint32_t word = b.mw[0];
-#pragma unroll
-        for (int w = 1; w < MW; ++w) word = w == wq ? b.mw[w] : word;
+        if constexpr (MW == 2) word = wq & 1 ? b.mw[1] : b.mw[0];
+        if constexpr (MW == 4) {
+            const uint32_t lo = wq & 1 ? b.mw[1] : b.mw[0], hi = wq & 1 ? b.mw[3] : b.mw[2];
+            word = wq & 2 ? hi : lo;
+        }
         b.m = R == 1 ? word : (word >> sh) & FMASK;
     }
     __device__ __forceinline__ int before(const Block<LT, R>& b) const {
