@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "handle.h"
+#include "rows_blocks.cuh"
 
 namespace spc5cuda {
 namespace {
@@ -111,7 +112,7 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
                         kc = batch_kc(m->r, left);
                     } else if (k[i] == 1 && ldx[i] == 1 && ldy[i] == 1) {
                         kc = 1;
-                        how = m->rows_narrow ? SPMV_NARROW : SPMV_WIDE;
+                        how = m->rows_form == rows::NARROW ? SPMV_NARROW : SPMV_WIDE;
                     } else if (spmm_columns(vs, value_bytes_of(m->value_type), m->r, m->full_blocks(), left)) {
                         kc = spmm_cols_kc(vs, m->r, left);
                         how = COLUMNS;

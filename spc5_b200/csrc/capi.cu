@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "handle.h"
+#include "rows_blocks.cuh"
 
 namespace spc5cuda {
 
@@ -96,7 +97,7 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     constexpr int vt = sizeof(T) == 8 ? SPC5CUDA_F64 : SPC5CUDA_F32;
     const int nbr = div_up(nbRows, r);
     const int ngroups = spmv_groups(vs_of(vt), r);
-    const int nwarps = rows_warps(vt, r, true);  // one wave of either instantiation, about
+    const int nwarps = rows_warps(vt, r, rows::NARROW);  // one wave of the narrow form; the wide one's is a little less
     const CoreScratch at = core_scratch(nbr, ngroups, nwarps);
     PoolBuf scratch(at.bytes, s);
     unsigned char* mem = scratch.as<unsigned char>();
@@ -117,7 +118,7 @@ void core_spmv(int r, long nbRows, const int* rowsSizes, const unsigned char* he
     vr.wstart = reinterpret_cast<int*>(mem + at.wstart);
     vr.nwarps = nwarps;
     BetaView vn = vr;
-    vn.narrow = true;
+    vn.form = rows::NARROW;
     vn.follows = false;  // the splits are complete before any of the three begins
     v.run_if_value = 0;   // group kernel: some block-row does not fit
     vr.run_if_value = 1;  // row kernel: every block-row fits

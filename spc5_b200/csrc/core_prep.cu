@@ -177,20 +177,22 @@ __global__ void __launch_bounds__(THREADS) k_core_split(int nbr, const int* __re
     __syncthreads();
     TileStats m{0, 0, 0, 0};
     for (int t = threadIdx.x; t < nparts; t += THREADS) {
+        m.values += __ldcg(&stats[t].values);
         m.blocks = max(m.blocks, __ldcg(&stats[t].blocks));
         m.most_values = max(m.most_values, __ldcg(&stats[t].most_values));
         m.narrow += __ldcg(&stats[t].narrow);
     }
-    m = TileStats{0, warp_max(m.blocks), warp_max(m.most_values), warp_sum(m.narrow)};
+    m = TileStats{warp_sum(m.values), warp_max(m.blocks), warp_max(m.most_values), warp_sum(m.narrow)};
     if (lane == 0) part[w] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int k = 1; k < THREADS / 32; ++k) {
+            m.values += part[k].values;
             m.blocks = max(m.blocks, part[k].blocks);
             m.most_values = max(m.most_values, part[k].most_values);
             m.narrow += part[k].narrow;
         }
-        const bool narrow = rows::narrow(value_type, r, nbr, nblocks, m.narrow, nblocks);
+        const bool narrow = rows::narrow(value_type, r, nbr, nblocks, m.values, m.narrow, nblocks);
         *flag = rows::fit(value_type, r, m.blocks, m.most_values) ? (narrow ? 2 : 1) : 0;
     }
 }

@@ -142,7 +142,7 @@ struct spc5cuda_mat {
     int nwarps = 0;
     int kernel = SPC5CUDA_KERNEL_AUTO;  // SpMV kernel choice (spc5cuda_mat_set_kernel)
     bool rows_ok = false;               // every block-row fits the row kernel's buffers
-    bool rows_narrow = false;           // its narrow instantiation suits the masks
+    int rows_form = 0;                  // its form that suits the matrix
     std::unique_ptr<spc5cuda::SortedPlan> plan;  // rows sorted by size (irregular matrices)
     // the plan holds the only copy of the values (set when the plan is built
     // and serves SpMV): the reference order is rebuilt on demand
@@ -164,7 +164,7 @@ struct spc5cuda_mat {
         if (use_rows()) {
             v.wstart = wstart.as<int>();
             v.nwarps = nwarps;
-            v.narrow = rows_narrow;
+            v.form = rows_form;
         }
         return v;
     }
@@ -179,7 +179,7 @@ struct spc5cuda_mat {
         if (rows_ok && nwarps > 0 && kernel != SPC5CUDA_KERNEL_GROUPS) {
             v.wstart = wstart.as<int>();
             v.nwarps = nwarps;
-            v.narrow = rows_narrow;
+            v.form = rows_form;
         }
         return v;
     }
@@ -231,11 +231,11 @@ struct spc5cuda_mat {
         gstart.alloc(sizeof(int) * size_t(ngroups + 1));
         spc5cuda::launch_partition(nbr(), brptr.as<int>(), ngroups, gstart.as<int>(), s);
         const spc5cuda::RowStats stats = spc5cuda::row_stats(value_type, r, nbr(), brptr.as<int>(), valptr.as<int>(),
-                                                             headers.as<uint8_t>(), nblocks, s);
+                                                             headers.as<uint8_t>(), nblocks, nnz, s);
         rows_ok = stats.fits;
-        rows_narrow = stats.narrow;
+        rows_form = stats.form;
         if (rows_ok) {
-            nwarps = spc5cuda::rows_warps(value_type, r, rows_narrow);
+            nwarps = spc5cuda::rows_warps(value_type, r, rows_form);
             wstart.alloc(sizeof(int) * size_t(nwarps + 1));
             spc5cuda::launch_partition(nbr(), brptr.as<int>(), nwarps, wstart.as<int>(), s);
         } else {

@@ -52,7 +52,7 @@ struct BetaView {
     // starts of the per-warp ranges; null selects the group kernel
     const int* wstart = nullptr;
     int nwarps = 0;
-    bool narrow = false;  // row kernel: the instantiation for narrow masks
+    int form = 0;  // of the row kernel: rows::WIDE or NARROW (rows_blocks.cuh)
     bool full_blocks = false;  // at least two values per sub-row and block on average
     // when set, the launch does its work only if *run_if == run_if_value (a
     // device word written by an earlier kernel on the same stream)
@@ -74,14 +74,14 @@ void launch_spmv_f64(const BetaView& m, const double* x, double* y, cudaStream_t
 // whether block-rows of at most max_blocks blocks / max_values values fit its
 // staging buffers, and what a converted matrix asks of it (synchronises s).
 // (vt: the handle's value type, SPC5CUDA_F64 / F32 / F32_V8.)
-int rows_warps(int vt, int r, bool narrow);
+int rows_warps(int vt, int r, int form);
 struct RowStats {
     bool fits;    // every block-row fits the row kernel's buffers
-    bool narrow;  // most blocks' sub-row masks span few columns
+    int form;     // of the row kernel that suits the matrix
 };
-// (headers may be null: narrow is not asked for.)
+// (headers may be null: the form is not asked for.)
 RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
-                   long nblocks, cudaStream_t s);
+                   long nblocks, long nnz, cudaStream_t s);
 // What the drop-in symbols find out about bare arrays, without a host round
 // trip (core_prep.cu): byte offsets in a 256-byte aligned scratch block of
 // valptr, gstart and wstart (as in BetaView) and of flag = 0 when some

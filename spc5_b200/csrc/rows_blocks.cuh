@@ -118,14 +118,21 @@ __host__ __device__ inline bool fit(int vt, int r, int max_blocks, int max_value
 }
 
 // Whether the narrow kernel runs: at least 7 of 8 of the blocks looked at keep
-// every sub-row mask within NS columns.  At r = VS its steps of 3 blocks pay for
-// themselves only on block-rows of several steps (measured on B200, FP64, wide /
-// narrow us: 27-point stencil 127^3, 18 blocks per block-row, 234 / 181; 5-point
-// Poisson 900^2, 4 blocks, 29.4 / 31.5).
-__host__ __device__ inline bool narrow(int vt, int r, int nbr, long nblocks, int narrow_blocks, int looked_at) {
+// every sub-row mask within NS columns, and at r > 1 a sub-row has at least 1.22
+// values per block, since a lane steps over the blocks that hold nothing of its
+// sub-row one by one (measured on B200, us, wide / narrow, a diagonal of 1,000,000
+// rows: FP64 r = 4 18.1 / 21.4, float layout r = 8 21.0 / 25.2; two values per row,
+// one of them far from the diagonal, FP64 r = 4 29.0 / 35.5; 5-point Poisson 900^2,
+// 1.67 values, float layout r = 4 28.4 / 25.1).  At r = VS its steps of 3 blocks pay
+// for themselves only on block-rows of several steps (FP64: 27-point stencil 127^3,
+// 18 blocks per block-row, 234 / 181; Poisson 900^2, 4 blocks, 25.7 / 28.2; float
+// values 32.0 / 30.4).
+__host__ __device__ inline bool narrow(int vt, int r, int nbr, long nblocks, long nnz, int narrow_blocks, int looked_at) {
     const int vs = vt == SPC5CUDA_F32 ? 16 : 8;
-    return looked_at > 0 && long(narrow_blocks) * 8 >= long(looked_at) * 7 && (r < vs || nblocks >= 6L * nbr);
+    return looked_at > 0 && long(narrow_blocks) * 8 >= long(looked_at) * 7 && (r == 1 || 50 * nnz >= 61 * r * nblocks) &&
+           (r < vs || vt == SPC5CUDA_F32_V8 || nblocks >= 6L * nbr);
 }
+
 template <class LT, int R, class V, class X, class A>
 __device__ __forceinline__ void narrow_blocks(const uint32_t* hw, const V* vbuf, const X* __restrict__ x, int q,
                                               SubRow at, uint64_t pol_x, A (&acc)[Layout<LT>::VS]) {
@@ -241,6 +248,9 @@ __device__ __forceinline__ SubRow sub_row_at(const Chunk& ch, int lane) {
     return at;
 }
 
+// The forms of the row kernel (spmv_rows.cu).
+constexpr int WIDE = 0, NARROW = 1;
+
 // The row sum of VS accumulators: the _mm512_reduce_add tree (distance VS/2,
 // ..., 1).
 template <class A, int VS>
@@ -259,7 +269,7 @@ __device__ __forceinline__ void add_to(float* y, float v) { *y = *y + v; }
 
 // One chunk of block-rows for one x and y: the lane of every sub-row runs its
 // blocks and adds the row sum to y.
-template <class LT, int R, class V, class X, class A, class Y, bool NARROW>
+template <class LT, int R, class V, class X, class A, class Y, int FORM>
 __device__ __forceinline__ void chunk_spmv(const Chunk& ch, const uint32_t* hw, const V* vbuf,
                                            const X* __restrict__ x, Y* __restrict__ y, int nrows, uint64_t pol_x) {
     constexpr int VS = Layout<LT>::VS;
@@ -268,7 +278,7 @@ __device__ __forceinline__ void chunk_spmv(const Chunk& ch, const uint32_t* hw, 
     A acc[VS];
 #pragma unroll
     for (int c = 0; c < VS; ++c) acc[c] = A(0);
-    if constexpr (NARROW)
+    if constexpr (FORM == NARROW)
         narrow_blocks<LT, R, V, X, A>(hw, vbuf, x, lane % R, at, pol_x, acc);
     else
         // 16 columns per step (r = 8, FP64, 2 blocks and 6 CTAs per SM against 4 and

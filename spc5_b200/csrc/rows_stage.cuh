@@ -18,10 +18,6 @@ namespace rows {
 
 constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
-// One warp's staging buffer: 7.5 KB, so that 7 CTAs of 4 warps fit an SM
-// (measured on B200: 10 KB buffers, 5 per SM, were 3% slower on the
-// power-law matrix and 10% on the 27-point stencil; 5 KB chunks were too
-// small for the stencil).
 // First block-row of warp w of W: the boundaries wstart of a partition made for
 // nwarps warps (the SpMV's), interpolated for a kernel that keeps W resident.
 // The row counts are int, so the product stays in 64 bits.
@@ -32,6 +28,9 @@ __device__ __forceinline__ int part_start(const int* __restrict__ wstart, int nw
     return f == 0 ? a : a + int(long(__ldg(wstart + p + 1) - a) * f / W);
 }
 
+// One warp's staging buffer: 7.5 KB, so that 7 CTAs of 4 warps fit an SM
+// (measured on B200: 10 KB buffers, 5 per SM, were 10% slower on the 27-point
+// stencil; 5 KB chunks were too small for it).
 constexpr int HB = 1536;  // header bytes of one warp's staging buffer
 constexpr int VB = 6144;  // value bytes of one warp's staging buffer
 constexpr unsigned FULL = 0xffffffffu;

@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(MM_THREADS, MM_CTAS)
 
 // The jobs of one right-hand side with contiguous x and y: the row SpMV's
 // chunks.
-template <class LT, int R, class V, class X, class A, class Y, bool NARROW>
+template <class LT, int R, class V, class X, class A, class Y, int FORM>
 __global__ void __launch_bounds__(rows::THREADS, 5)
     k_spmv_rows_batch(const BatchMat* __restrict__ mats, const BatchJob* __restrict__ jobs, int njobs) {
     using G = rows::Geo<LT, R, V, R>;
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(rows::THREADS, 5)
         rows::walk<LT, R, V, R>(m.brptr, m.headers, static_cast<const V*>(m.values), m.valptr, job.r_begin, job.r_end,
                                 smem + wi * G::BUF_BYTES,
                                 [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
-                                    rows::chunk_spmv<LT, R, V, X, A, Y, NARROW>(ch, hw, vbuf, x, y, nrows, pol_x);
+                                    rows::chunk_spmv<LT, R, V, X, A, Y, FORM>(ch, hw, vbuf, x, y, nrows, pol_x);
                                 });
     }
 }
@@ -392,8 +392,8 @@ void batch_rows_impl(int r, int kc, bool narrow, const BatchMat* mats, const Bat
     if (kc == 1) {
         dispatch_r(r, [&](auto RC) {
             constexpr int R_ = decltype(RC)::value, SMEM = rows::Geo<LT, R_, V, R_>::SMEM;
-            if (narrow) launch_jobs(k_spmv_rows_batch<LT, R_, V, X, A, Y, true>, rows::THREADS, SMEM, mats, jobs, njobs, s);
-            else launch_jobs(k_spmv_rows_batch<LT, R_, V, X, A, Y, false>, rows::THREADS, SMEM, mats, jobs, njobs, s);
+            if (narrow) launch_jobs(k_spmv_rows_batch<LT, R_, V, X, A, Y, rows::NARROW>, rows::THREADS, SMEM, mats, jobs, njobs, s);
+            else launch_jobs(k_spmv_rows_batch<LT, R_, V, X, A, Y, rows::WIDE>, rows::THREADS, SMEM, mats, jobs, njobs, s);
         });
         return;
     }

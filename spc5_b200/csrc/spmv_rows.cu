@@ -10,7 +10,7 @@
 // lane s of a block-row works on its sub-row s from shared memory, all VS
 // columns, with VS accumulators in registers.
 //
-// Two instantiations.  The wide one tests every column of a block.  The narrow
+// Two forms.  The wide one tests every column of a block.  The narrow
 // one is for matrices whose sub-row masks span at most NS columns (stencils:
 // 3 of 8 or 16): a lane's masks keep to one window of NS columns from its
 // block-row's first column on (at r = 8, VS = 8 modulo VS), so it tests NS
@@ -59,14 +59,14 @@ constexpr int ROWS_CTAS_PER_SM = 16;
 // window wraps (127^3: 7 was 7% slower).  5 where 16 double accumulators (the
 // float layout in mixed precision) need the registers.
 template <class LT, int R, class A>
-constexpr int row_ctas(bool narrow) {
+constexpr int row_ctas(int form) {
     constexpr int VS = Layout<LT>::VS;
     if (VS * sizeof(A) > 64) return 5;
-    return narrow && R < 8 ? 7 : 6;
+    return form == NARROW && R < 8 ? 7 : 6;
 }
 
-template <class LT, int R, class V, class X, class A, class Y, bool NARROW>
-__global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, A>(NARROW))
+template <class LT, int R, class V, class X, class A, class Y, int FORM>
+__global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, A>(FORM))
     k_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
            const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart, int nwarps,
            const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, A>(NARROW))
     unsigned char* wbuf = smem + wi * G::BUF_BYTES;
     rows::walk<LT, R, V, R>(brptr, headers, values, valptr, r_begin, r_stop, wbuf,
                             [&](const rows::Chunk& ch, const uint32_t* hw, const V* vbuf) {
-                                chunk_spmv<LT, R, V, X, A, Y, NARROW>(ch, hw, vbuf, x, y, nrows, pol_x);
+                                chunk_spmv<LT, R, V, X, A, Y, FORM>(ch, hw, vbuf, x, y, nrows, pol_x);
                             });
 }
 
@@ -106,13 +106,19 @@ void dispatch_r(int r, F&& f) {
     throw Error(SPC5CUDA_ERR_FORMAT, "r must be 1, 2, 4 or 8");
 }
 
+// The kernel of a form.
+template <class LT, int R, class V, class X, class A, class Y>
+auto rows_kernel(int form) {
+    return form == NARROW ? k_rows<LT, R, V, X, A, Y, NARROW> : k_rows<LT, R, V, X, A, Y, WIDE>;
+}
+
 template <class LT, class V, class X, class A, class Y>
-int rows_occupancy(int r, bool narrow) {
+int rows_occupancy(int r, int form) {
     int n = 0;
     dispatch_r(r, [&](auto RC) {
         constexpr int R_ = decltype(RC)::value;
         using G = rows::Geo<LT, R_, V, R_>;
-        auto kern = narrow ? k_rows<LT, R_, V, X, A, Y, true> : k_rows<LT, R_, V, X, A, Y, false>;
+        auto kern = rows_kernel<LT, R_, V, X, A, Y>(form);
         set_smem(kern, G::SMEM);
         SPC5_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, ROWS_THREADS, G::SMEM));
     });
@@ -127,7 +133,7 @@ void launch_rows_impl(const BetaView& m, const X* x, Y* y, cudaStream_t s) {
     dispatch_r(m.r, [&](auto RC) {
         constexpr int R_ = decltype(RC)::value;
         using G = rows::Geo<LT, R_, V, R_>;
-        auto kern = m.narrow ? k_rows<LT, R_, V, X, A, Y, true> : k_rows<LT, R_, V, X, A, Y, false>;
+        auto kern = rows_kernel<LT, R_, V, X, A, Y>(m.form);
         set_smem(kern, G::SMEM);
         launch_after(kern, dim3(unsigned(ctas)), ROWS_THREADS, G::SMEM, m.follows, s, m.nrows, m.brptr, m.headers, vals,
                      m.valptr, m.wstart, m.nwarps, x, y, m.run_if, m.run_if_value);
@@ -189,13 +195,13 @@ __global__ void k_blockrow_max(int nbr, const int* __restrict__ brptr, const int
 
 }  // namespace
 
-int rows_warps(int vt, int r, bool narrow) {
+int rows_warps(int vt, int r, int form) {
     // cached per (device, value type, r, instantiation): the drop-in symbols ask on every call
     static std::mutex mu;
-    static std::map<std::tuple<int, int, int, bool>, int> cache;
+    static std::map<std::tuple<int, int, int, int>, int> cache;
     int dev = 0;
     SPC5_CUDA(cudaGetDevice(&dev));
-    const auto key = std::make_tuple(dev, vt, r, narrow);
+    const auto key = std::make_tuple(dev, vt, r, form);
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
@@ -203,12 +209,12 @@ int rows_warps(int vt, int r, bool narrow) {
     }
     int per_sm;
     if (vt == SPC5CUDA_F64) {
-        per_sm = rows_occupancy<double, double, double, double, double>(r, narrow);
+        per_sm = rows_occupancy<double, double, double, double, double>(r, form);
     } else if (vt == SPC5CUDA_F32_V8) {
-        per_sm = rows_occupancy<double, float, float, double, double>(r, narrow);
+        per_sm = rows_occupancy<double, float, float, double, double>(r, form);
     } else {
-        per_sm = std::min(rows_occupancy<float, float, float, float, float>(r, narrow),
-                          rows_occupancy<float, float, float, double, double>(r, narrow));
+        per_sm = std::min(rows_occupancy<float, float, float, float, float>(r, form),
+                          rows_occupancy<float, float, float, double, double>(r, form));
     }
     const int n = sm_count() * per_sm * ROWS_WARPS;
     std::lock_guard<std::mutex> lk(mu);
@@ -217,7 +223,7 @@ int rows_warps(int vt, int r, bool narrow) {
 }
 
 RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, const uint8_t* headers,
-                   long nblocks, cudaStream_t s) {
+                   long nblocks, long nnz, cudaStream_t s) {
     // the largest block and value counts of any block-row; narrow and all sampled blocks
     PoolBuf d(4 * sizeof(int), s);
     int* stats = d.as<int>();
@@ -235,7 +241,8 @@ RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, 
     int h[4] = {0, 0, 0, 0};
     SPC5_CUDA(cudaMemcpyAsync(h, d.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     SPC5_CUDA(cudaStreamSynchronize(s));
-    return RowStats{rows::fit(vt, r, h[0], h[1]), rows::narrow(vt, r, nbr, nblocks, h[2], h[3])};
+    const bool is_narrow = rows::narrow(vt, r, nbr, nblocks, nnz, h[2], h[3]);
+    return RowStats{rows::fit(vt, r, h[0], h[1]), is_narrow ? NARROW : WIDE};
 }
 
 void launch_rows_kind(int kind, const BetaView& m, const void* x, void* y, cudaStream_t s) {

@@ -61,7 +61,7 @@ int plan_regime(const spc5cuda_mat* m, int r, const int* brptr, cudaStream_t s) 
     const int nbr = div_up(m->nrows, r);
     DevBuf valptr(sizeof(int) * size_t(nbr + 1), s);
     launch_valptr_from_csr(r, m->nrows, m->rowptr.as<int>(), valptr.as<int>(), s);
-    return row_stats(m->value_type, r, nbr, brptr, valptr.as<int>(), nullptr, 0, s).fits ? 0 : 1;
+    return row_stats(m->value_type, r, nbr, brptr, valptr.as<int>(), nullptr, 0, 0, s).fits ? 0 : 1;
 }
 
 // A trial run: a temporary handle holding a copy of the CSR matrix is
