@@ -52,7 +52,7 @@ struct BetaView {
     // starts of the per-warp ranges; null selects the group kernel
     const int* wstart = nullptr;
     int nwarps = 0;
-    int form = 0;  // of the row kernel: rows::WIDE or NARROW (rows_blocks.cuh)
+    int form = 0;  // of the row kernel: rows::WIDE, NARROW or DEEP (rows_blocks.cuh)
     bool full_blocks = false;  // at least two values per sub-row and block on average
     // when set, the launch does its work only if *run_if == run_if_value (a
     // device word written by an earlier kernel on the same stream)

@@ -248,8 +248,9 @@ __device__ __forceinline__ SubRow sub_row_at(const Chunk& ch, int lane) {
     return at;
 }
 
-// The forms of the row kernel (spmv_rows.cu).
-constexpr int WIDE = 0, NARROW = 1;
+// The forms of the row kernel: the wide and the narrow one (spmv_rows.cu), and the
+// wide one with twice the blocks per step.
+constexpr int WIDE = 0, NARROW = 1, DEEP = 2;
 
 // The row sum of VS accumulators: the _mm512_reduce_add tree (distance VS/2,
 // ..., 1).
@@ -278,13 +279,14 @@ __device__ __forceinline__ void chunk_spmv(const Chunk& ch, const uint32_t* hw, 
     A acc[VS];
 #pragma unroll
     for (int c = 0; c < VS; ++c) acc[c] = A(0);
+    constexpr int UT = 16 / VS > 1 ? 16 / VS : 1;
     if constexpr (FORM == NARROW)
         narrow_blocks<LT, R, V, X, A>(hw, vbuf, x, lane % R, at, pol_x, acc);
     else
         // 16 columns per step (r = 8, FP64, 2 blocks and 6 CTAs per SM against 4 and
         // 4 on B200: banded 150,000 44 / 42 us, 5-point Poisson 700^2 19.2 / 21.1;
         // mixed, banded 200,000 14.2 / 19.1)
-        wide_blocks<LT, R, V, X, A, (16 / VS > 1 ? 16 / VS : 1)>(hw, vbuf, x, lane % R, at, pol_x, acc);
+        wide_blocks<LT, R, V, X, A, (FORM == DEEP ? 2 * UT : UT)>(hw, vbuf, x, lane % R, at, pol_x, acc);
     const A sum = reduce_tree<A, VS>(acc);
     const long yrow = long(ch.r0) * R + lane;  // sub-row `lane` of the chunk
     if (lane / R < ch.nrow && yrow < nrows) add_to(y + yrow, Y(sum));

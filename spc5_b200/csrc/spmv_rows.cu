@@ -10,7 +10,8 @@
 // lane s of a block-row works on its sub-row s from shared memory, all VS
 // columns, with VS accumulators in registers.
 //
-// Two forms.  The wide one tests every column of a block.  The narrow
+// Three forms.  The wide one tests every column of a block; the deep one is the wide
+// one with twice the blocks per step, for long block-rows.  The narrow
 // one is for matrices whose sub-row masks span at most NS columns (stencils:
 // 3 of 8 or 16): a lane's masks keep to one window of NS columns from its
 // block-row's first column on (at r = 8, VS = 8 modulo VS), so it tests NS
@@ -58,15 +59,29 @@ constexpr int ROWS_CTAS_PER_SM = 16;
 // 9.4 us on the device; 160^3 at r = 4 197 against 203 us), 6 at r = 8, whose
 // window wraps (127^3: 7 was 7% slower).  5 where 16 double accumulators (the
 // float layout in mixed precision) need the registers.
-template <class LT, int R, class A>
+// Deep: 4 for double x (106 and 121 registers), 7 for float x.
+template <class LT, int R, class X, class A>
 constexpr int row_ctas(int form) {
     constexpr int VS = Layout<LT>::VS;
+    if (form == DEEP) return sizeof(X) == 8 ? 4 : 7;
     if (VS * sizeof(A) > 64) return 5;
     return form == NARROW && R < 8 ? 7 : 6;
 }
 
+// Whether the deep form runs instead of the wide one: 8 columns, r >= 4, and long
+// block-rows, of which a chunk holds few, so that steps that wait for one another
+// count for more than warps in flight.  Measured on B200 (us, wide / deep, 60,000
+// rows of 41 values in a band of 401): FP64 r = 4 28.5 / 25.8, r = 8 31.9 / 28.2; float
+// values r = 8 50.8 / 40.2 (4 CTAs 52.9); 200,000 rows of 31 values in a band of 301,
+// 24 sub-rows per chunk, float values r = 8 73.2 / 71.0.
+bool deep(int vt, int r, int nbr, long nblocks, long nnz) {
+    if (vt == SPC5CUDA_F32 || r < 4) return false;
+    const int rows = chunk_rows(vt, r, nbr, nblocks, nnz);
+    return vt == SPC5CUDA_F64 ? rows < 24 : rows <= 24;
+}
+
 template <class LT, int R, class V, class X, class A, class Y, int FORM>
-__global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, A>(FORM))
+__global__ void __launch_bounds__(ROWS_THREADS, row_ctas<LT, R, X, A>(FORM))
     k_rows(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
            const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart, int nwarps,
            const X* __restrict__ x, Y* __restrict__ y, const int* __restrict__ run_if, int run_if_value) {
@@ -106,9 +121,11 @@ void dispatch_r(int r, F&& f) {
     throw Error(SPC5CUDA_ERR_FORMAT, "r must be 1, 2, 4 or 8");
 }
 
-// The kernel of a form.
+// The kernel of a form (the deep one exists for 8 columns and r >= 4).
 template <class LT, int R, class V, class X, class A, class Y>
 auto rows_kernel(int form) {
+    if constexpr (Layout<LT>::VS == 8 && R >= 4)
+        if (form == DEEP) return k_rows<LT, R, V, X, A, Y, DEEP>;
     return form == NARROW ? k_rows<LT, R, V, X, A, Y, NARROW> : k_rows<LT, R, V, X, A, Y, WIDE>;
 }
 
@@ -242,7 +259,8 @@ RowStats row_stats(int vt, int r, int nbr, const int* brptr, const int* valptr, 
     SPC5_CUDA(cudaMemcpyAsync(h, d.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     SPC5_CUDA(cudaStreamSynchronize(s));
     const bool is_narrow = rows::narrow(vt, r, nbr, nblocks, nnz, h[2], h[3]);
-    return RowStats{rows::fit(vt, r, h[0], h[1]), is_narrow ? NARROW : WIDE};
+    const int form = is_narrow ? NARROW : (deep(vt, r, nbr, nblocks, nnz) ? DEEP : WIDE);
+    return RowStats{rows::fit(vt, r, h[0], h[1]), form};
 }
 
 void launch_rows_kind(int kind, const BetaView& m, const void* x, void* y, cudaStream_t s) {
