@@ -123,13 +123,16 @@ __host__ __device__ inline bool fit(int vt, int r, int max_blocks, int max_value
 // sub-row one by one (measured on B200, us, wide / narrow, a diagonal of 1,000,000
 // rows: FP64 r = 4 18.1 / 21.4, float layout r = 8 21.0 / 25.2; two values per row,
 // one of them far from the diagonal, FP64 r = 4 29.0 / 35.5; 5-point Poisson 900^2,
-// 1.67 values, float layout r = 4 28.4 / 25.1).  At r = VS its steps of 3 blocks pay
+// 1.67 values, float layout r = 4 28.4 / 25.1).  Float values in 8 columns: only where
+// block-rows are short (60,000 rows of 40 random values, 80 blocks per block-row, r = 2
+// 168 / 147).  At r = VS its steps of 3 blocks pay
 // for themselves only on block-rows of several steps (FP64: 27-point stencil 127^3,
 // 18 blocks per block-row, 234 / 181; Poisson 900^2, 4 blocks, 25.7 / 28.2; float
 // values 32.0 / 30.4).
 __host__ __device__ inline bool narrow(int vt, int r, int nbr, long nblocks, long nnz, int narrow_blocks, int looked_at) {
     const int vs = vt == SPC5CUDA_F32 ? 16 : 8;
-    return looked_at > 0 && long(narrow_blocks) * 8 >= long(looked_at) * 7 && (r == 1 || 50 * nnz >= 61 * r * nblocks) &&
+    const bool few_empty = r == 1 || 50 * nnz >= 61 * r * nblocks || (vt == SPC5CUDA_F32_V8 && nblocks >= 3L * nbr);
+    return looked_at > 0 && long(narrow_blocks) * 8 >= long(looked_at) * 7 && few_empty &&
            (r < vs || vt == SPC5CUDA_F32_V8 || nblocks >= 6L * nbr);
 }
 

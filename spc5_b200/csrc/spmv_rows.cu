@@ -73,11 +73,12 @@ constexpr int row_ctas(int form) {
 // count for more than warps in flight.  Measured on B200 (us, wide / deep, 60,000
 // rows of 41 values in a band of 401): FP64 r = 4 28.5 / 25.8, r = 8 31.9 / 28.2; float
 // values r = 8 50.8 / 40.2 (4 CTAs 52.9); 200,000 rows of 31 values in a band of 301,
-// 24 sub-rows per chunk, float values r = 8 73.2 / 71.0.
+// 24 sub-rows per chunk, float values r = 8 73.2 / 71.0.  With float values only where
+// sub-rows have few values per block: 32^3 grid of 3 unknowns, three, r = 8 39 / 45.
 bool deep(int vt, int r, int nbr, long nblocks, long nnz) {
     if (vt == SPC5CUDA_F32 || r < 4) return false;
     const int rows = chunk_rows(vt, r, nbr, nblocks, nnz);
-    return vt == SPC5CUDA_F64 ? rows < 24 : rows <= 24;
+    return vt == SPC5CUDA_F64 ? rows < 24 : rows <= 24 && 2 * nnz < 3L * r * nblocks;
 }
 
 template <class LT, int R, class V, class X, class A, class Y, int FORM>
