@@ -48,12 +48,14 @@ __device__ __forceinline__ void with_pitch(const Chain& c, F&& f) {
     else f(c.pitch);
 }
 
-// acc += the chain's multiply-adds of the entries from j0 on, x element i at x[i ldx],
-// U entries at a time: the next step's values and x indices load while this step's
-// x are gathered.  Every load guarded: the chains of a slab differ in length.
-template <int U, class V, class X, class A, class P>
+// acc += the chain's multiply-adds of the entries from j0 on for W right-hand sides,
+// x element i at x[i ldx + w xcs], U entries at a time: the next step's values and x
+// indices load while this step's x are gathered.  Every load guarded: the chains of a
+// slab differ in length.
+template <int U, int W, class V, class X, class A, class P>
 __device__ __forceinline__ void run_guarded(const Chain& c, int j0, P pitch, const V* __restrict__ val,
-                                            const int* __restrict__ xcol, const X* __restrict__ x, long ldx, A& acc) {
+                                            const int* __restrict__ xcol, const X* __restrict__ x, long ldx, long xcs,
+                                            A (&acc)[W]) {
     const V* vp = val + c.at;
     const int* cp = xcol + c.at;
     const int width = __reduce_max_sync(FULL, c.len);
@@ -73,15 +75,20 @@ __device__ __forceinline__ void run_guarded(const Chain& c, int j0, P pitch, con
     };
     load(j0, v, col);
     for (; j0 < width; j0 += U) {
-        X xv[U];
+        X xv[U][W];
 #pragma unroll
-        for (int u = 0; u < U; ++u) xv[u] = j0 + u < c.len ? ld_x(x + long(col[u]) * ldx, pol) : X(0);
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int w = 0; w < W; ++w) xv[u][w] = j0 + u < c.len ? ld_x(x + long(col[u]) * ldx + w * xcs, pol) : X(0);
         V vn[U];
         int cn[U];
         load(j0 + U, vn, cn);
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (j0 + u < c.len) acc = fma(A(v[u]), A(xv[u]), acc);
+            if (j0 + u < c.len) {
+#pragma unroll
+                for (int w = 0; w < W; ++w) acc[w] = fma(A(v[u]), A(xv[u][w]), acc[w]);
+            }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             v[u] = vn[u];
@@ -95,9 +102,10 @@ __device__ __forceinline__ void run_guarded(const Chain& c, int j0, P pitch, con
 // load at a time (one row of 20,000 values, 8-column mixed layout 185 us, so 95;
 // several right-hand sides, 50,000 rows of 400 values, k = 1, mixed 168 / 59);
 // doubles with one x run faster guarded (97 / 154).
-template <int U, class V, class X, class A, class P>
+template <int U, int W, class V, class X, class A, class P>
 __device__ __forceinline__ void run_whole(const Chain& c, P pitch, const V* __restrict__ val,
-                                          const int* __restrict__ xcol, const X* __restrict__ x, long ldx, A& acc) {
+                                          const int* __restrict__ xcol, const X* __restrict__ x, long ldx, long xcs,
+                                          A (&acc)[W]) {
     const V* vp = val + c.at;
     const int* cp = xcol + c.at;
     const int whole = __reduce_min_sync(FULL, c.len) / U * U;
@@ -113,21 +121,25 @@ __device__ __forceinline__ void run_whole(const Chain& c, P pitch, const V* __re
     };
     if (whole > 0) load(0, v, col);
     for (int j0 = 0; j0 < whole; j0 += U) {
-        X xv[U];
+        X xv[U][W];
 #pragma unroll
-        for (int u = 0; u < U; ++u) xv[u] = ld_x(x + long(col[u]) * ldx, pol);
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int w = 0; w < W; ++w) xv[u][w] = ld_x(x + long(col[u]) * ldx + w * xcs, pol);
         V vn[U];
         int cn[U];
         load(min(j0 + U, whole - U), vn, cn);
 #pragma unroll
-        for (int u = 0; u < U; ++u) acc = fma(A(v[u]), A(xv[u]), acc);
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int w = 0; w < W; ++w) acc[w] = fma(A(v[u]), A(xv[u][w]), acc[w]);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             v[u] = vn[u];
             col[u] = cn[u];
         }
     }
-    run_guarded<CHAIN_U, V, X, A>(c, whole, pitch, val, xcol, x, ldx, acc);
+    run_guarded<CHAIN_U, W, V, X, A>(c, whole, pitch, val, xcol, x, ldx, xcs, acc);
 }
 
 // One warp per slab, one lane per chain.
@@ -138,31 +150,46 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_spmv(const __grid_const
     const long q = long(blockIdx.x) * CHAIN_THREADS + threadIdx.x;
     if (q / 32 >= p.slabs) return;  // warp-uniform
     const Chain c = chain_at(p, q);
-    A acc = A(0);
+    A acc[1] = {A(0)};
     with_pitch(c, [&](auto pitch) {
-        if constexpr (U == CHAIN_DEEP && sizeof(A) > sizeof(V)) run_whole<U, V, X, A>(c, pitch, val, p.col, x, 1L, acc);
-        else run_guarded<U, V, X, A>(c, 0, pitch, val, p.col, x, 1L, acc);
+        if constexpr (U == CHAIN_DEEP && sizeof(A) > sizeof(V)) run_whole<U, 1, V, X, A>(c, pitch, val, p.col, x, 1L, 0L, acc);
+        else run_guarded<U, 1, V, X, A>(c, 0, pitch, val, p.col, x, 1L, 0L, acc);
     });
-    if (q < p.chains) out[__ldg(p.id + q)] = acc;
+    if (q < p.chains) out[__ldg(p.id + q)] = acc[0];
 }
 
-// KC lanes per chain, one right-hand side each, 32 / KC neighbouring chains of a
-// slab per warp.
+// KC / W lanes per chain, W neighbouring right-hand sides each, 32 W / KC neighbouring
+// chains of a slab per warp.  W = 2 from 8 right-hand sides on: half the loads of values
+// and indices (20^3 grid of 6 unknowns, FP64, r = 8, k = 16 190 us, now 137).
+template <int KC>
+constexpr int chain_w = KC >= 8 ? 2 : 1;
+
 template <class V, class X, class A, int KC>
 __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_spmm(const __grid_constant__ ChainView p, const V* __restrict__ val,
                                                               int kc, const X* __restrict__ x, long ldx, long xcs,
                                                               A* __restrict__ out) {
     griddep_launch();
+    constexpr int W = chain_w<KC>, L = KC / W;  // lanes per chain
     const long t = long(blockIdx.x) * CHAIN_THREADS + threadIdx.x;
-    const long q = t / KC;
-    const int j = int(t % KC);
-    if (t / 32 * (32 / KC) >= p.chains) return;  // warp-uniform
+    const long q = t / L;
+    const int j = int(t % L) * W;
+    if (t / 32 * (32 / L) >= p.chains) return;  // warp-uniform
     const Chain c = chain_at(p, q);
-    A acc = A(0);
+    A acc[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) acc[w] = A(0);
+    // lanes past the last right-hand side read the last one's again (an odd one's
+    // second: the first again)
+    const long x0 = long(min(j, kc - 1)) * xcs, step = j + 1 < kc ? xcs : 0L;
     with_pitch(c, [&](auto pitch) {
-        run_whole<CHAIN_U, V, X, A>(c, pitch, val, p.col, x + long(min(j, kc - 1)) * xcs, ldx, acc);
+        run_whole<CHAIN_U, W, V, X, A>(c, pitch, val, p.col, x + x0, ldx, step, acc);
     });
-    if (q < p.chains && j < kc) out[__ldg(p.id + q) * long(KC) + j] = acc;
+    if (q < p.chains) {
+        const long at = __ldg(p.id + q) * long(KC) + j;
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+            if (j + w < kc) out[at + w] = acc[w];
+    }
 }
 
 // Y[row][j] += the reduce tree over the VS chains of every row of the chain part.

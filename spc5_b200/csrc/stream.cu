@@ -609,7 +609,7 @@ void run_spmm(const spc5cuda_mat* m, int k, const X* x, long ldx, long xcs, Y* y
         const ChainView c = chain_view_of(p);
         const size_t bytes = sizeof(A) * size_t(c.rows) * VS * KC;
         if (!sums || sums->bytes < bytes) sums = std::make_unique<PoolBuf>(bytes, s);
-        const int warps = div_up(c.chains, 32 / KC);
+        const int warps = div_up(c.chains, 32 * chain_w<KC> / KC);
         launch(k_chain_spmm<V, X, A, KC>, dim3(div_up(warps, CHAIN_THREADS / 32)), false, s, c,
                static_cast<const V*>(p.cval), kc, xp, ldx, xcs, sums->as<A>());
         follows = true;
