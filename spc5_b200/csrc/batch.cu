@@ -107,13 +107,15 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
                 while (kofs < k[i]) {
                     const bool staged = m->spmm_view().wstart != nullptr;
                     const int left = k[i] - kofs, vs = vs_of(m->value_type);
+                    const float fill = m->fill();
+                    const bool one = k[i] == 1 && ldx[i] == 1 && ldy[i] == 1;
                     int kc, how = GROUP;
                     if (!staged) {
                         kc = batch_kc(m->r, left);
-                    } else if (k[i] == 1 && ldx[i] == 1 && ldy[i] == 1) {
+                    } else if (one && !spmv_columns(m->r, fill, m->chunk_rows())) {
                         kc = 1;
                         how = m->rows_form == rows::NARROW ? SPMV_NARROW : SPMV_WIDE;
-                    } else if (spmm_columns(vs, value_bytes_of(m->value_type), m->r, m->full_blocks(), left)) {
+                    } else if (one || spmm_columns(vs, value_bytes_of(m->value_type), m->r, fill, m->list_rows(), left)) {
                         kc = spmm_cols_kc(vs, m->r, left);
                         how = COLUMNS;
                     } else {

@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "memory.h"
+#include "rows_stage.cuh"
 
 namespace spc5cuda {
 
@@ -160,7 +161,9 @@ struct spc5cuda_mat {
         v.valptr = valptr.as<int>();
         v.gstart = gstart.as<int>();
         v.ngroups = ngroups;
-        v.full_blocks = full_blocks();
+        v.fill = fill();
+        v.chunk_rows = chunk_rows();
+        v.list_rows = list_rows();
         if (use_rows()) {
             v.wstart = wstart.as<int>();
             v.nwarps = nwarps;
@@ -168,7 +171,10 @@ struct spc5cuda_mat {
         }
         return v;
     }
-    bool full_blocks() const { return nnz >= 2L * r * nblocks; }
+    // Values per sub-row and block, and sub-rows per chunk, on average.
+    float fill() const { return nblocks > 0 ? float(double(nnz) / (double(r) * double(nblocks))) : 0.f; }
+    int chunk_rows() const { return spc5cuda::rows::chunk_rows(value_type, r, nbr(), nblocks, nnz); }
+    int list_rows() const { return spc5cuda::rows::chunk_rows(value_type, r, nbr(), nblocks, nnz, 4096); }
     // The view of the SpMM kernels: the per-warp ranges of the staged kernel
     // whenever every block-row fits its buffers, unless the group kernel was
     // requested.

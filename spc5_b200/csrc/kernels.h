@@ -53,7 +53,9 @@ struct BetaView {
     const int* wstart = nullptr;
     int nwarps = 0;
     int form = 0;  // of the row kernel: rows::WIDE, NARROW or DEEP (rows_blocks.cuh)
-    bool full_blocks = false;  // at least two values per sub-row and block on average
+    float fill = 0.f;     // values per sub-row and block on average
+    int chunk_rows = 32;  // sub-rows of an average chunk of the row kernel (rows::chunk_rows),
+    int list_rows = 32;   // and of one of the value lists' (spmm_rows.cu: 4 KB of headers at least)
     // when set, the launch does its work only if *run_if == run_if_value (a
     // device word written by an earlier kernel on the same stream)
     const int* run_if = nullptr;
@@ -159,9 +161,10 @@ void launch_batch(int kind, int r, int kc, const BatchMat* mats, const BatchJob*
 // last pass may have fewer).
 int spmm_rows_kc(int k);
 // Whether a pass with k right-hand sides left runs with a lane per column
-// (spmm_cols.cu) instead: few right-hand sides on blocks of many rows.
-// full_blocks: at least two values per sub-row and block on average.
-bool spmm_columns(int vs, int value_bytes, int r, bool full_blocks, int k);
+// (spmm_cols.cu) instead (fill, list_rows, chunk_rows: as in BetaView), and whether
+// one contiguous right-hand side does instead of the row SpMV.
+bool spmm_columns(int vs, int value_bytes, int r, float fill, int list_rows, int k);
+bool spmv_columns(int r, float fill, int chunk_rows);
 // Right-hand sides of such a pass (a power of two), and its launch for a kind.
 int spmm_cols_kc(int vs, int r, int k);
 void launch_spmm_cols(int kind, const BetaView& m, int kc, const void* x, long ldx, long xcs, void* y, long ldy,
@@ -169,9 +172,10 @@ void launch_spmm_cols(int kind, const BetaView& m, int kc, const void* x, long l
 void launch_batch_cols(int kind, int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs,
                        cudaStream_t s);
 // Most right-hand sides of such a pass: r x (vs / lanes columns per lane) x kc
-// accumulators stay at most 32, kc at most 8.
+// accumulators stay at most 32, kc at most 16 (r <= 2) or 8.
 constexpr int mm_kc_limit(int vs, int r, int lanes) {
-    return 32 / (r * (vs / lanes)) > 8 ? 8 : 32 / (r * (vs / lanes));
+    const int most = r <= 2 ? 16 : 8, kc = 32 / (r * (vs / lanes));
+    return kc > most ? most : kc;
 }
 // The same for matrices whose block-rows fit the row kernels' buffers
 // (spmm_rows.cu): one warp per job at a time; kc from spmm_rows_kc, or 1 for

@@ -58,11 +58,11 @@ struct Geo {
     static constexpr int SMEM = WARPS * BUF_BYTES;
 };
 
-// Sub-rows of an average chunk: at most 32.
-inline int chunk_rows(int vt, int r, int nbr, long nblocks, long nnz) {
+// Sub-rows of an average chunk with hb bytes for headers: at most 32.
+inline int chunk_rows(int vt, int r, int nbr, long nblocks, long nnz, int hb = HB) {
     if (nbr <= 0 || nblocks <= 0 || nnz <= 0) return 32;
     const double stride = 4 + r * (vt == SPC5CUDA_F32 ? 2 : 1), vbytes = vt == SPC5CUDA_F64 ? 8 : 4;
-    const double most = std::min(HB / (stride * double(nblocks) / nbr), VB / (vbytes * double(nnz) / nbr));
+    const double most = std::min(hb / (stride * double(nblocks) / nbr), VB / (vbytes * double(nnz) / nbr));
     return r * std::max(1, int(std::min(most, 32.0 / r)));
 }
 

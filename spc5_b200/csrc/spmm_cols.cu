@@ -1,6 +1,7 @@
 // spmm_cols.cu -- staged multi-RHS SpMM with a lane per column, for few
-// right-hand sides on blocks of many rows (spmm_columns in kernels.h says
-// which; spmm_rows.cu has the other staged SpMM, and why it tests less).
+// right-hand sides on blocks of many rows and for long rows of full blocks
+// (spmm_columns in spmm_rows.cu says which; that file has the other staged SpMM, and
+// why it tests less).
 //
 // A warp walks its block-rows in chunks staged into shared memory; each
 // block-row of a chunk is served by L lanes (mm_lanes), and lane q owns the
@@ -21,6 +22,7 @@
 // float Y, exactly as the SpMV kernels).  Column j of the result is therefore
 // bit-identical to an SpMV with column j of X.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -35,16 +37,19 @@ using rows::FULL;
 // Registers limit this kernel to 4 CTAs per SM, so it stages larger chunks than
 // the SpMV (every block-row that fits the SpMV's buffers fits these).
 // One or two right-hand sides leave room for the SpMV's own chunks and 5 or 6
-// CTAs, except with double values at r = 8 (stencil 64^3, k = 2 on a B200: mixed
-// 77 us at 4 CTAs and larger chunks / 67 so, r = 4 46 / 38; FP64, r = 8 55 / 73).
-template <class V, int R, int KC>
-constexpr bool cols_small = KC <= 2 && (R < 8 || sizeof(V) == 4);
-template <class V, int R, int KC>
-constexpr int cols_hb = cols_small<V, R, KC> ? rows::HB : 2048;
-template <class V, int R, int KC>
-constexpr int cols_vb = cols_small<V, R, KC> ? rows::VB : 8192;
-template <class V, int R, int KC>
-constexpr int cols_ctas(int acc_bytes) { return cols_small<V, R, KC> ? (acc_bytes > 64 ? 5 : 6) : 1; }
+// CTAs, except with double values at r = 8, and where those chunks hold 32 sub-rows
+// (stencil 64^3, k = 2 on a B200: mixed 77 us at 4 CTAs and larger chunks / 67 so, r =
+// 4 46 / 38; FP64, r = 8 55 / 73; 32^3 grid of 3 unknowns, 81 values per row, FP64, r = 4
+// 31 / 41).
+constexpr bool cols_small(int value_bytes, int r, int kc, int chunk_rows) {
+    return kc <= 2 && (r < 8 || value_bytes == 4) && chunk_rows >= 32;
+}
+template <bool SMALL>
+constexpr int cols_hb = SMALL ? rows::HB : 2048;
+template <bool SMALL>
+constexpr int cols_vb = SMALL ? rows::VB : 8192;
+template <bool SMALL>
+constexpr int cols_ctas(int acc_bytes) { return SMALL ? (acc_bytes > 64 ? 5 : 6) : 1; }
 
 // Union of the sub-row masks (bit c: some sub-row has a value in column c).
 template <class LT, int R>
@@ -110,7 +115,7 @@ constexpr int mm_lanes() {
 
 // Y += A X over block-rows [r_begin, r_stop) of one matrix for right-hand
 // sides [0, KC) of xm / ym (already offset to the pass's first one).
-template <class LT, int R, int KC, class V, class X, class A, class Y>
+template <class LT, int R, int KC, bool SMALL, class V, class X, class A, class Y>
 __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brptr,
                                          const uint8_t* __restrict__ headers, const V* __restrict__ values,
                                          const int* __restrict__ valptr, int r_begin, int r_stop,
@@ -120,7 +125,7 @@ __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brpt
     constexpr int L = mm_lanes<LT, R>();  // lanes per block-row
     constexpr int CPL = VS / L;                // columns per lane: q + L k
     constexpr int LOGL = L == 16 ? 4 : (L == 8 ? 3 : (L == 4 ? 2 : (L == 2 ? 1 : 0)));
-    using G = rows::Geo<LT, R, V, L, cols_hb<V, R, KC>, cols_vb<V, R, KC>>;
+    using G = rows::Geo<LT, R, V, L, cols_hb<SMALL>, cols_vb<SMALL>>;
     constexpr int MB = G::MB, MW = G::MW;
     constexpr int FPW = 4 / MB;  // mask fields per 32-bit word
     constexpr int BITS = 8 * MB;
@@ -272,65 +277,81 @@ __device__ __forceinline__ void mm_range(int nrows, const int* __restrict__ brpt
         }
         flush(mine, ch.r0 + slot);
     };
-    rows::walk<LT, R, V, L, cols_hb<V, R, KC>, cols_vb<V, R, KC>>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
+    rows::walk<LT, R, V, L, cols_hb<SMALL>, cols_vb<SMALL>>(brptr, headers, values, valptr, r_begin, r_stop, wbuf, compute);
 }
 
 // One matrix: the grid's warps, one resident wave, share its block-rows
 // (part_start).  The SpMV's partition is for 5 to 7 CTAs per SM, of which 3 or 4
 // fit here: stencil 64^3, r = 8, on a B200 FP64 k = 4 74 us, now 60; k = 2 55 / 45;
 // mixed k = 5 148 / 121.
-template <class LT, int R, int KC, class V, class X, class A, class Y>
-__global__ void __launch_bounds__(rows::THREADS, cols_ctas<V, R, KC>(Layout<LT>::VS * int(sizeof(A))))
+template <class LT, int R, int KC, bool SMALL, class V, class X, class A, class Y>
+__global__ void __launch_bounds__(rows::THREADS, cols_ctas<SMALL>(Layout<LT>::VS * int(sizeof(A))))
     k_spmm_cols(int nrows, const int* __restrict__ brptr, const uint8_t* __restrict__ headers,
                 const V* __restrict__ values, const int* __restrict__ valptr, const int* __restrict__ wstart,
                 int nwarps, const X* __restrict__ xm, long ldx, long xcs, Y* __restrict__ ym, long ldy, long ycs) {
-    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), cols_hb<V, R, KC>, cols_vb<V, R, KC>>;
+    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), cols_hb<SMALL>, cols_vb<SMALL>>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
     const int warp = blockIdx.x * rows::WARPS + wi;
     const int W = gridDim.x * rows::WARPS;
     const int r_begin = rows::part_start(wstart, nwarps, warp, W), r_stop = rows::part_start(wstart, nwarps, warp + 1, W);
-    mm_range<LT, R, KC, V, X, A, Y>(nrows, brptr, headers, values, valptr, r_begin, r_stop, xm, ldx, xcs, ym, ldy, ycs,
+    mm_range<LT, R, KC, SMALL, V, X, A, Y>(nrows, brptr, headers, values, valptr, r_begin, r_stop, xm, ldx, xcs, ym, ldy, ycs,
                                     smem + wi * G::BUF_BYTES);
 }
 
 // Batched: warps walk the job list with the grid's warp count as stride; job
 // j is block-rows [r_begin, r_end) of mats[j.mat] for right-hand sides
 // [kofs, kofs + KC).  X and Y of a batch are row-major (xcs = ycs = 1).
-template <class LT, int R, int KC, class V, class X, class A, class Y>
-__global__ void __launch_bounds__(rows::THREADS, cols_ctas<V, R, KC>(Layout<LT>::VS * int(sizeof(A))))
+template <class LT, int R, int KC, bool SMALL, class V, class X, class A, class Y>
+__global__ void __launch_bounds__(rows::THREADS, cols_ctas<SMALL>(Layout<LT>::VS * int(sizeof(A))))
     k_spmm_cols_batch(const BatchMat* __restrict__ mats, const BatchJob* __restrict__ jobs, int njobs) {
-    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), cols_hb<V, R, KC>, cols_vb<V, R, KC>>;
+    using G = rows::Geo<LT, R, V, mm_lanes<LT, R>(), cols_hb<SMALL>, cols_vb<SMALL>>;
     extern __shared__ __align__(16) unsigned char smem[];
     const int wi = threadIdx.x >> 5;
     const int nw = gridDim.x * rows::WARPS;
     for (int j = blockIdx.x * rows::WARPS + wi; j < njobs; j += nw) {  // warp-uniform
         const BatchJob job = jobs[j];
         const BatchMat& m = mats[job.mat];
-        mm_range<LT, R, KC, V, X, A, Y>(m.nrows, m.brptr, m.headers, static_cast<const V*>(m.values), m.valptr,
+        mm_range<LT, R, KC, SMALL, V, X, A, Y>(m.nrows, m.brptr, m.headers, static_cast<const V*>(m.values), m.valptr,
                                         job.r_begin, job.r_end, static_cast<const X*>(m.x) + job.kofs, m.ldx, 1L,
                                         static_cast<Y*>(m.y) + job.kofs, m.ldy, 1L, smem + wi * G::BUF_BYTES);
     }
 }
 
-// Calls f(integral_constant<R>, integral_constant<KC>) for r in {4, 8}
-// and kc a power of two up to mm_kc_limit of the kernel's lanes.
-template <class LT, class F>
-void dispatch_rkc(int r, int kc, F&& f) {
+// Calls f(integral_constant<R>, integral_constant<KC>, bool_constant<SMALL>) for r in
+// {1, 2, 4, 8} and kc a power of two up to mm_kc_limit of the kernel's lanes.
+template <class LT, class V, class F>
+void dispatch_rkc(int r, int kc, int chunk_rows, F&& f) {
     using std::integral_constant;
     auto with_r = [&](auto RC) {
         constexpr int R_ = decltype(RC)::value;
         constexpr int KMAX = mm_kc_limit(Layout<LT>::VS, R_, mm_lanes<LT, R_>());
+        auto with_kc = [&](auto KCC) {
+            constexpr int KC_ = decltype(KCC)::value;
+            if constexpr (KC_ <= KMAX) {
+                if constexpr (cols_small(int(sizeof(V)), R_, KC_, 32))
+                    if (cols_small(int(sizeof(V)), R_, KC_, chunk_rows)) {
+                        f(RC, KCC, std::true_type{});
+                        return true;
+                    }
+                f(RC, KCC, std::false_type{});
+                return true;
+            }
+            return false;
+        };
         switch (kc) {
-            case 1: f(RC, integral_constant<int, 1>{}); return true;
-            case 2: if constexpr (KMAX >= 2) { f(RC, integral_constant<int, 2>{}); return true; } break;
-            case 4: if constexpr (KMAX >= 4) { f(RC, integral_constant<int, 4>{}); return true; } break;
-            case 8: if constexpr (KMAX >= 8) { f(RC, integral_constant<int, 8>{}); return true; } break;
+            case 1: return with_kc(integral_constant<int, 1>{});
+            case 2: return with_kc(integral_constant<int, 2>{});
+            case 4: return with_kc(integral_constant<int, 4>{});
+            case 8: return with_kc(integral_constant<int, 8>{});
+            case 16: return with_kc(integral_constant<int, 16>{});
         }
         return false;
     };
     bool done = false;
     switch (r) {
+        case 1: done = with_r(integral_constant<int, 1>{}); break;
+        case 2: done = with_r(integral_constant<int, 2>{}); break;
         case 4: done = with_r(integral_constant<int, 4>{}); break;
         case 8: done = with_r(integral_constant<int, 8>{}); break;
     }
@@ -340,10 +361,11 @@ void dispatch_rkc(int r, int kc, F&& f) {
 template <class LT, class V, class X, class A, class Y>
 void cols_pass(const BetaView& m, int kc, const void* x, long ldx, long xcs, void* y, long ldy, long ycs,
                cudaStream_t s) {
-    dispatch_rkc<LT>(m.r, kc, [&](auto RC, auto KCC) {
+    dispatch_rkc<LT, V>(m.r, kc, m.chunk_rows, [&](auto RC, auto KCC, auto SC) {
         constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), cols_hb<V, R_, KC_>, cols_vb<V, R_, KC_>>::SMEM;
-        auto kern = k_spmm_cols<LT, R_, KC_, V, X, A, Y>;
+        constexpr bool SMALL = decltype(SC)::value;
+        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), cols_hb<SMALL>, cols_vb<SMALL>>::SMEM;
+        auto kern = k_spmm_cols<LT, R_, KC_, SMALL, V, X, A, Y>;
         set_smem(kern, SMEM);
         static const int per_sm = resident_ctas(kern, rows::THREADS, SMEM);
         const int ctas = std::min((m.nwarps + rows::WARPS - 1) / rows::WARPS, sm_count() * per_sm);
@@ -356,10 +378,12 @@ void cols_pass(const BetaView& m, int kc, const void* x, long ldx, long xcs, voi
 
 template <class LT, class V, class X, class A, class Y>
 void cols_batch(int r, int kc, const BatchMat* mats, const BatchJob* jobs, int njobs, cudaStream_t s) {
-    dispatch_rkc<LT>(r, kc, [&](auto RC, auto KCC) {
+    // (the chunks of a class of jobs: as for full ones)
+    dispatch_rkc<LT, V>(r, kc, 32, [&](auto RC, auto KCC, auto SC) {
         constexpr int R_ = decltype(RC)::value, KC_ = decltype(KCC)::value;
-        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), cols_hb<V, R_, KC_>, cols_vb<V, R_, KC_>>::SMEM;
-        auto kern = k_spmm_cols_batch<LT, R_, KC_, V, X, A, Y>;
+        constexpr bool SMALL = decltype(SC)::value;
+        constexpr int SMEM = rows::Geo<LT, R_, V, mm_lanes<LT, R_>(), cols_hb<SMALL>, cols_vb<SMALL>>::SMEM;
+        auto kern = k_spmm_cols_batch<LT, R_, KC_, SMALL, V, X, A, Y>;
         set_smem(kern, SMEM);
         int per_sm = 0;
         SPC5_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, rows::THREADS, SMEM));

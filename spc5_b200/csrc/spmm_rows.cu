@@ -351,11 +351,13 @@ void spmm_rows_impl(const BetaView& m, int k, const X* x, long ldx, long xcs, Y*
     for (int k0 = 0; k0 < k;) {
         const X* xp = x + long(k0) * xcs;
         Y* yp = y + long(k0) * ycs;
-        if (k - k0 == 1 && ldx == 1 && ldy == 1) {  // one right-hand side, contiguous: the SpMV
+        const bool columns = spmm_columns(Layout<LT>::VS, int(sizeof(V)), m.r, m.fill, m.list_rows, k - k0);
+        const bool one = k - k0 == 1 && ldx == 1 && ldy == 1;
+        if (one && !spmv_columns(m.r, m.fill, m.chunk_rows)) {  // one contiguous right-hand side: the SpMV
             launch_rows_kind(KIND, m, xp, yp, s);
             return;
         }
-        if (spmm_columns(Layout<LT>::VS, int(sizeof(V)), m.r, m.full_blocks, k - k0)) {
+        if (columns || one) {
             const int kc = spmm_cols_kc(Layout<LT>::VS, m.r, k - k0);
             launch_spmm_cols(KIND, m, kc, xp, ldx, xcs, yp, ldy, ycs, s);
             k0 += kc;
@@ -417,10 +419,29 @@ void batch_rows_impl(int r, int kc, bool narrow, const BatchMat* mats, const Bat
 //   r = 1 and 2: lists (r = 2, k = 4 81 / 74 and 58 / 34).
 //   8 columns of float values (mixed): as FP64, but the columns' x are half as
 //     wide: r = 4, fill 3, k = 16 166 / 183; r = 8, k = 5 135 / 153.
-bool spmm_columns(int vs, int value_bytes, int r, bool full_blocks, int k) {
-    if (vs == 16) return r >= 4 && k <= 5 && k != 3;
-    if (r == 8) return k <= (value_bytes == 4 ? 5 : 4);
-    return r == 4 && full_blocks && k <= (value_bytes == 4 ? 16 : 12);
+//   Long rows of full blocks: a chunk holds fewer sub-rows than the lists have
+//     lanes for, and each lists its values alone.  FP64, 32^3 grid of 3 unknowns (81
+//     values per row, fill 4.5): r = 2, k = 2 39 / 90, k = 8 76 / 101; 20^3 of 6 (162,
+//     fill 4.5 to 6): r = 1, k = 2 35 / 140, k = 8 82 / 144; blocks of 8 at random
+//     columns, 480 per row: r = 1, k = 4 84 / 626.  Banded n = 60,000, 41 values per
+//     row, fill 1, r = 4, FP64, k = 2 31 / 44.
+bool spmm_columns(int vs, int value_bytes, int r, float fill, int list_rows, int k) {
+    const bool wide = value_bytes == 8;
+    if (r <= 2) {
+        if (list_rows > (wide ? 16 : 24) || k > (wide || list_rows < 6 ? 8 : 16)) return false;
+        return fill >= (r == 2 ? 2.f : (vs == 16 ? 2.5f : 4.f));
+    }
+    if (vs == 16) return (k <= 5 && k != 3) || (k <= 8 && fill >= 2.5f && list_rows <= 24);
+    if (r == 8) return k <= (wide ? 4 : 5);
+    return (fill >= 2.f && k <= (wide ? 12 : 16)) || (k == 2 && fill >= 0.9f && list_rows < 24);
+}
+
+// Measured on B200 (us, SpMV / one column of columns): 40,000 rows of 100 random values,
+// FP64, r = 1 150 / 115, 25,000 of 200 467 / 238; 60,000 of 40, r = 2 108 / 62; 20^3 grid
+// of 6 unknowns, r = 2 47 / 33; of 3 unknowns 35 / 66 and 37 / 41.
+bool spmv_columns(int r, float fill, int chunk_rows) {
+    if (r > 1 && fill < 0.7f && chunk_rows < 24) return true;
+    return r == 1 ? chunk_rows < 5 : (r == 2 ? chunk_rows < 8 : r == 4 && chunk_rows <= 8);
 }
 
 int spmm_rows_kc(int k) { return k > 8 ? 16 : (k > 4 ? 8 : (k > 2 ? 4 : 2)); }
