@@ -112,7 +112,7 @@ spc5cuda_status spc5cuda_batch_create(spc5cuda_batch** out, int n, spc5cuda_mat*
                     int kc, how = GROUP;
                     if (!staged) {
                         kc = batch_kc(m->r, left);
-                    } else if (one && !spmv_columns(m->r, fill, m->chunk_rows())) {
+                    } else if (one && !spmv_columns(vs, m->r, fill, m->chunk_rows())) {
                         kc = 1;
                         how = m->rows_form == rows::NARROW ? SPMV_NARROW : SPMV_WIDE;
                     } else if (one || spmm_columns(vs, value_bytes_of(m->value_type), m->r, fill, m->list_rows(), left)) {

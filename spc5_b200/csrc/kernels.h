@@ -164,7 +164,7 @@ int spmm_rows_kc(int k);
 // (spmm_cols.cu) instead (fill, list_rows, chunk_rows: as in BetaView), and whether
 // one contiguous right-hand side does instead of the row SpMV.
 bool spmm_columns(int vs, int value_bytes, int r, float fill, int list_rows, int k);
-bool spmv_columns(int r, float fill, int chunk_rows);
+bool spmv_columns(int vs, int r, float fill, int chunk_rows);
 // Right-hand sides of such a pass (a power of two), and its launch for a kind.
 int spmm_cols_kc(int vs, int r, int k);
 void launch_spmm_cols(int kind, const BetaView& m, int kc, const void* x, long ldx, long xcs, void* y, long ldy,

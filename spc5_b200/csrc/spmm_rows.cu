@@ -353,7 +353,8 @@ void spmm_rows_impl(const BetaView& m, int k, const X* x, long ldx, long xcs, Y*
         Y* yp = y + long(k0) * ycs;
         const bool columns = spmm_columns(Layout<LT>::VS, int(sizeof(V)), m.r, m.fill, m.list_rows, k - k0);
         const bool one = k - k0 == 1 && ldx == 1 && ldy == 1;
-        if (one && !spmv_columns(m.r, m.fill, m.chunk_rows)) {  // one contiguous right-hand side: the SpMV
+        // one contiguous right-hand side: the SpMV
+        if (one && !spmv_columns(Layout<LT>::VS, m.r, m.fill, m.chunk_rows)) {
             launch_rows_kind(KIND, m, xp, yp, s);
             return;
         }
@@ -424,11 +425,15 @@ void batch_rows_impl(int r, int kc, bool narrow, const BatchMat* mats, const Bat
 //     values per row, fill 4.5): r = 2, k = 2 39 / 90, k = 8 76 / 101; 20^3 of 6 (162,
 //     fill 4.5 to 6): r = 1, k = 2 35 / 140, k = 8 82 / 144; blocks of 8 at random
 //     columns, 480 per row: r = 1, k = 4 84 / 626.  Banded n = 60,000, 41 values per
-//     row, fill 1, r = 4, FP64, k = 2 31 / 44.
+//     row, fill 1, r = 4, FP64, k = 2 31 / 44.  From 9 right-hand sides on the rows of
+//     X at random columns count for more: the blocks, 240 values per row, r = 1, k = 16,
+//     FP64 549 / 232, mixed 305 / 270; 800 values per row, one sub-row per chunk, mixed
+//     523 / 1361.
 bool spmm_columns(int vs, int value_bytes, int r, float fill, int list_rows, int k) {
     const bool wide = value_bytes == 8;
     if (r <= 2) {
-        if (list_rows > (wide ? 16 : 24) || k > (wide || list_rows < 6 ? 8 : 16)) return false;
+        const bool lists16 = list_rows > (wide ? 1 : 2) && (wide || list_rows < 8);  // from 9 right-hand sides on
+        if (list_rows > (wide ? 16 : 24) || k > (lists16 ? 8 : 16)) return false;
         return fill >= (r == 2 ? 2.f : (vs == 16 ? 2.5f : 4.f));
     }
     if (vs == 16) return (k <= 5 && k != 3) || (k <= 8 && fill >= 2.5f && list_rows <= 24);
@@ -438,10 +443,11 @@ bool spmm_columns(int vs, int value_bytes, int r, float fill, int list_rows, int
 
 // Measured on B200 (us, SpMV / one column of columns): 40,000 rows of 100 random values,
 // FP64, r = 1 150 / 115, 25,000 of 200 467 / 238; 60,000 of 40, r = 2 108 / 62; 20^3 grid
-// of 6 unknowns, r = 2 47 / 33; of 3 unknowns 35 / 66 and 37 / 41.
-bool spmv_columns(int r, float fill, int chunk_rows) {
+// of 6 unknowns, r = 2 47 / 33; of 3 unknowns 35 / 66 and 37 / 41; 30 blocks of 8 at
+// random columns, r = 4, mixed 259 / 74, float layout 223 / 276.
+bool spmv_columns(int vs, int r, float fill, int chunk_rows) {
     if (r > 1 && fill < 0.7f && chunk_rows < 24) return true;
-    return r == 1 ? chunk_rows < 5 : (r == 2 ? chunk_rows < 8 : r == 4 && chunk_rows <= 8);
+    return r == 1 ? chunk_rows < 5 : (r == 2 ? chunk_rows < 8 : r == 4 && vs == 8 && chunk_rows <= 8);
 }
 
 int spmm_rows_kc(int k) { return k > 8 ? 16 : (k > 4 ? 8 : (k > 2 ? 4 : 2)); }
