@@ -20,27 +20,33 @@ namespace {
 // the time per value keyed by the average number of values per block, as the
 // reference's SPC5_find_best model is (src/spc5.hpp:1157-1212).
 // Value type (F64, F32, F32_V8) x r (1, 2, 4, 8) x regime: {t0, d0, d1, d2}.
-// The sorted-plan rows were fitted on an earlier form of the plan (r = 2, 4,
-// 8) on the plan-regime calibration matrices alone (power-law and random,
-// tune_fit.plan_calibration_set), keeping the row-kernel t0.
+// The sorted-plan rows hold one set per value type for every r, since the plan stores
+// rows: the first r of equal estimates is picked, r = 1, whose conversion is the
+// cheapest (96 SpMVs on a B200, power-law and random, estimate / measured 0.55 to 1.7;
+// at N = 1M and 2M 0.8 to 1.05).  The row-kernel rows were measured before the narrow
+// form: on the present kernels the estimates are 1.2 times too high in the median (10
+// to 90% of 723 SpMVs: 0.85 to 1.6), and 189 of 201 picks are within 10% or 3 us of the
+// best r.  A new fit picks 194 of 201 for one SpMV, but r = 1 nearly everywhere on
+// banded matrices, where batches take r = 4 and gain from it (64 matrices, up to 16
+// right-hand sides, FP64 942 us, with the new fit 978), so these rows stay.
 constexpr double kModel[3][4][2][4] = {
     {
-        {{1.027079e+01, -2.714134e-07, 9.285081e-06, 1.994012e-06}, {1.027079e+01, 1.113738e-05, 0.000000e+00, 0.000000e+00}},
-        {{1.046586e+01, 6.170896e-07, 9.230068e-06, 9.138698e-06}, {1.046586e+01, 1.212031e-05, 0.000000e+00, 0.000000e+00}},
-        {{1.004610e+01, 1.547721e-06, 1.189384e-05, 2.402879e-05}, {1.004610e+01, 8.274836e-06, 0.000000e+00, 0.000000e+00}},
-        {{1.004540e+01, 6.250567e-07, 5.782892e-05, -8.901463e-05}, {1.004540e+01, 7.059285e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.027079e+01, -2.714134e-07, 9.285081e-06, 1.994012e-06}, {3.415286e+01, 4.016372e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.046586e+01, 6.170896e-07, 9.230068e-06, 9.138698e-06}, {3.415286e+01, 4.016372e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.004610e+01, 1.547721e-06, 1.189384e-05, 2.402879e-05}, {3.415286e+01, 4.016372e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.004540e+01, 6.250567e-07, 5.782892e-05, -8.901463e-05}, {3.415286e+01, 4.016372e-06, 0.000000e+00, 0.000000e+00}},
     },
     {
-        {{1.009044e+01, 2.953275e-07, 6.279096e-06, 1.099184e-05}, {1.009044e+01, 9.763137e-06, 0.000000e+00, 0.000000e+00}},
-        {{1.008880e+01, 1.137428e-06, 1.740009e-06, 3.621405e-05}, {1.008880e+01, 1.172209e-05, 0.000000e+00, 0.000000e+00}},
-        {{1.020511e+01, 1.170424e-06, 1.023505e-05, 1.026359e-04}, {1.020511e+01, 6.684552e-06, 0.000000e+00, 0.000000e+00}},
-        {{1.034971e+01, -4.723864e-07, 8.071517e-05, -1.176461e-04}, {1.034971e+01, 5.902880e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.009044e+01, 2.953275e-07, 6.279096e-06, 1.099184e-05}, {2.167149e+01, 3.929946e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.008880e+01, 1.137428e-06, 1.740009e-06, 3.621405e-05}, {2.167149e+01, 3.929946e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.020511e+01, 1.170424e-06, 1.023505e-05, 1.026359e-04}, {2.167149e+01, 3.929946e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.034971e+01, -4.723864e-07, 8.071517e-05, -1.176461e-04}, {2.167149e+01, 3.929946e-06, 0.000000e+00, 0.000000e+00}},
     },
     {
-        {{9.690487e+00, -8.483423e-07, 1.129287e-05, 5.480109e-06}, {9.690487e+00, 1.023616e-05, 0.000000e+00, 0.000000e+00}},
-        {{9.904177e+00, 1.562250e-07, 1.131417e-05, 1.759617e-05}, {9.904177e+00, 1.203661e-05, 0.000000e+00, 0.000000e+00}},
-        {{1.008765e+01, 1.592180e-07, 2.480687e-05, 2.707475e-05}, {1.008765e+01, 7.725355e-06, 0.000000e+00, 0.000000e+00}},
-        {{1.044845e+01, -1.152926e-06, 8.811726e-05, -7.893453e-05}, {1.044845e+01, 6.381369e-06, 0.000000e+00, 0.000000e+00}},
+        {{9.690487e+00, -8.483423e-07, 1.129287e-05, 5.480109e-06}, {2.432020e+01, 3.783348e-06, 0.000000e+00, 0.000000e+00}},
+        {{9.904177e+00, 1.562250e-07, 1.131417e-05, 1.759617e-05}, {2.432020e+01, 3.783348e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.008765e+01, 1.592180e-07, 2.480687e-05, 2.707475e-05}, {2.432020e+01, 3.783348e-06, 0.000000e+00, 0.000000e+00}},
+        {{1.044845e+01, -1.152926e-06, 8.811726e-05, -7.893453e-05}, {2.432020e+01, 3.783348e-06, 0.000000e+00, 0.000000e+00}},
     },
 };
 

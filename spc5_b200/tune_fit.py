@@ -18,7 +18,12 @@ measured on a B200 with this project's kernels, for r = 1, 2, 4 and 8.
     python -m spc5_b200.tune_fit measure > calib.jsonl   # on a B200
     python -m spc5_b200.tune_fit fit calib.jsonl          # prints the C table
     python -m spc5_b200.tune_fit measure_plan > plan.jsonl           # plan regime only
+    python -m spc5_b200.tune_fit fit_plan plan.jsonl                 # its coefficients
     python -m spc5_b200.tune_fit refit_plan plan.jsonl spc5_b200/csrc/tune.cu
+
+The plan stores rows, not block-rows, so its times do not depend on r: ``fit_plan``
+gives one set per value type for every r, which csrc/tune.cu holds (``refit_plan``
+fits one cost per value for each r, beside the t0 that stands there).
 
 ``fit`` prints the table pasted into csrc/tune.cu (kModel) and the fraction of
 calibration matrices whose modelled pick is within 10% of the best measured r
@@ -134,6 +139,22 @@ def refit_plan(path: str, table: str) -> None:
             print(f"// value type {vt}, r = {r}: sorted-plan {{t0, d0}} = {{{t0:.6e}, {d0:.6e}}}")
 
 
+def fit_plan(path: str) -> dict:
+    """{t0, d0} of the sorted plan per value type, one for every r, from the timings
+    in ``path`` (least squares of the relative error)."""
+    rows = [json.loads(l) for l in open(path) if l.strip()]
+    out = {}
+    for vt in (0, 1, 2):
+        pts = [p for p in rows if p["vt"] == vt and p["plan"] == 1]
+        if not pts:
+            continue
+        nnz = np.array([float(p["nnz"]) for p in pts])
+        us = np.array([p["us"] for p in pts])
+        out[vt], *_ = np.linalg.lstsq(np.stack([1.0 / us, nnz / us], axis=1), np.ones(len(us)), rcond=None)
+        print(f"// value type {vt}: sorted-plan {{t0, d0}} = {{{out[vt][0]:.6e}, {out[vt][1]:.6e}}}")
+    return out
+
+
 def fit(path: str) -> None:
     rows = [json.loads(l) for l in open(path) if l.strip()]
     for p in rows:
@@ -190,6 +211,8 @@ if __name__ == "__main__":
         measure(mats=plan_calibration_set())
     elif len(sys.argv) >= 4 and sys.argv[1] == "refit_plan":
         refit_plan(sys.argv[2], sys.argv[3])
+    elif len(sys.argv) >= 3 and sys.argv[1] == "fit_plan":
+        fit_plan(sys.argv[2])
     elif len(sys.argv) >= 3 and sys.argv[1] == "fit":
         fit(sys.argv[2])
     else:
