@@ -930,7 +930,8 @@ TRAFFIC_RATIO = {"powerlaw": {1: 1.210, 2: 1.178, 4: 1.102, 8: 0.971},
 
 # spc5cuda_mat_kernel codes: SPC5CUDA_KERNEL_GROUPS = 1, SPC5CUDA_KERNEL_ROWS = 2
 KERNEL_NAME = {1: "k_spmv (group per block-row stream)", 2: "k_rows (thread per sub-row)",
-               3: "sorted plan (long rows as warp streams, k_stream_spmv; short rows one per lane, k_short_spmv)", 0: "unconverted"}
+               3: "sorted plan (long rows as warp streams, k_stream_spmv, or chains, k_chain_spmv; "
+                  "short rows one per lane, k_short_spmv)", 0: "unconverted"}
 
 
 def select_kernel(m, which):

@@ -197,11 +197,12 @@ SPC5CUDA_API spc5cuda_status spc5cuda_mat_info(const spc5cuda_mat* mat, spc5cuda
  *   ROWS   -- the thread-per-sub-row kernel; SPC5CUDA_ERR_UNSUPPORTED on a
  *             converted matrix with a block-row that does not fit;
  *   SORTED -- the sorted plan: the handle holds its values with the rows
- *             sorted by size, long rows four (float layout: two) to a warp,
- *             short rows one to a lane, each value with its x index, instead
- *             of in the reference order.  AUTO uses it when some block-row
- *             does not fit the row kernel (power-law and other irregular
- *             matrices).
+ *             sorted by size, long rows four (float layout: two) to a warp
+ *             or, where the plan's rule finds that faster, as multiply-add
+ *             chains one to a lane, short rows one to a lane, each value with
+ *             its x index, instead of in the reference order.  AUTO uses it
+ *             when some block-row does not fit the row kernel (power-law and
+ *             other irregular matrices).
  * spc5cuda_mat_kernel reports the kernel SpMV uses now (GROUPS, ROWS or
  * SORTED; AUTO before conversion).  Selecting SORTED (or AUTO, where it picks
  * the plan) on a converted matrix builds the plan and releases the
@@ -217,8 +218,8 @@ SPC5CUDA_API spc5cuda_status spc5cuda_mat_info(const spc5cuda_mat* mat, spc5cuda
 SPC5CUDA_API spc5cuda_status spc5cuda_mat_set_kernel(spc5cuda_mat* mat, int kernel);
 SPC5CUDA_API spc5cuda_status spc5cuda_mat_kernel(const spc5cuda_mat* mat, int* kernel);
 /* Kernel launches one spc5cuda_spmv of a converted handle makes now (the
- * sorted plan: one for its long rows, one for its short rows; else 1; 0 for an
- * empty matrix). */
+ * sorted plan: one for its long rows, one for its short rows, two for rows
+ * stored as chains; else 1; 0 for an empty matrix). */
 SPC5CUDA_API spc5cuda_status spc5cuda_mat_spmv_launches(const spc5cuda_mat* mat, int* launches);
 
 /* SPC5_{r}rVc_block_count (spc5.hpp:510-513, 635-638, 764-767, 890-893):

@@ -257,7 +257,7 @@ class SPC5Mat:
     @property
     def spmv_launches(self) -> int:
         """Kernel launches one SPC5_Spmv of this converted matrix makes (the sorted plan: one for
-        its long rows, one for its short rows; else 1)."""
+        its long rows, one for its short rows, two for rows stored as chains; else 1)."""
         n = C.c_int(0)
         _check(_lib().spc5cuda_mat_spmv_launches(self._h, C.byref(n)), "spc5cuda_mat_spmv_launches")
         return n.value

@@ -1,7 +1,7 @@
 // chain.cuh -- SpMV and SpMM over the chain part of the sorted plan (stream.cuh has
-// its layout; plan.cu builds it): one lane, or one lane per right-hand side, runs
-// one (row, column) chain of multiply-adds, and a last launch adds each row's VS
-// chains by the reduce tree.
+// its layout; plan.cu builds it): one lane runs one (row, column) chain of
+// multiply-adds (SpMM: for one or two right-hand sides), and a last launch adds each
+// row's VS chains by the reduce tree.
 #pragma once
 
 #include <type_traits>

@@ -4,9 +4,9 @@
 // block-rows of hundreds; no single work split suits both.  The plan sorts the
 // rows of the matrix by size and stores the long ones as warp streams or as chains
 // (chain_rows says which) and the short ones one per lane (stream.cuh): every chain
-// of multiply-adds keeps its values in block order, so y is bit-identical.  The plan holds the only copy
-// of the values; the handle keeps the reference-order headers, from which the
-// values can be put back in the reference order (rebuild_values).
+// of multiply-adds keeps its values in block order, so y is bit-identical.  The plan
+// holds the only copy of the values; the handle keeps the reference-order headers, from
+// which the values can be put back in the reference order (rebuild_values).
 //
 // Build, all on the device: row-blocks and values of every row (k_row_stats),
 // a radix sort of the rows by size, the sizes of the long rows' slabs
@@ -495,8 +495,9 @@ int chain_rows(const spc5cuda_mat* m, const Counts& c) {
     if (rows == 0 || long(rows) * vs >= 1L << 31) return 0;  // (chain ids are int)
     if (c.longest <= 8.0 * double(c.blocks) / rows) return rows;
     // about 31 ps per warp step (of G row-blocks) and 3.2 ps per value for all rows;
-    // 50 ns per step of one row, of which all above half that time go to the chains.  Power-law of 20,000 rows, rows of more than 32
-    // row-blocks: 45 us, now 31; 100,000 rows, 128: 64 / 50; 300,000, 512: 84 / 84
+    // 50 ns per step of one row, of which all above half that time go to the chains.
+    // Power-law of 20,000 rows, rows of more than 32 row-blocks: 45 us, now 31; 100,000
+    // rows, 128: 64 / 50; 300,000, 512: 84 / 84
     const int G = 32 / vs;
     const double rest_us = 31e-6 * double(c.blocks) / G + 3.2e-6 * double(m->nnz);
     if (50e-3 * c.longest < 2.0 * rest_us) return 0;

@@ -417,7 +417,7 @@ void batch_rows_impl(int r, int kc, bool narrow, const BatchMat* mats, const Bat
 //   float layout, r = 4: k = 2 55 / 55 and 32 / 35, k = 3 111 / 86 and 61 / 49, k =
 //     4 67 / 74 and 41 / 43, k = 5 126 / 135, k = 8 137 / 112 and 81 / 55; r = 8: k = 4 65 / 82 and
 //     43 / 49, k = 8 133 / 119 and 84 / 61;
-//   r = 1 and 2: lists (r = 2, k = 4 81 / 74 and 58 / 34).
+//   r = 1 and 2: lists (r = 2, k = 4 81 / 74 and 58 / 34), but for long rows (below).
 //   8 columns of float values (mixed): as FP64, but the columns' x are half as
 //     wide: r = 4, fill 3, k = 16 166 / 183; r = 8, k = 5 135 / 153.
 //   Long rows of full blocks: a chunk holds fewer sub-rows than the lists have

@@ -22,8 +22,8 @@ namespace {
 // Value type (F64, F32, F32_V8) x r (1, 2, 4, 8) x regime: {t0, d0, d1, d2}.
 // The sorted-plan rows hold one set per value type for every r, since the plan stores
 // rows: the first r of equal estimates is picked, r = 1, whose conversion is the
-// cheapest (96 SpMVs on a B200, power-law and random, estimate / measured 0.55 to 1.7;
-// at N = 1M and 2M 0.8 to 1.05).  The row-kernel rows were measured before the narrow
+// cheapest (81 SpMVs on a B200, power-law and random, estimate / measured 0.49 to 1.95;
+// power-law of 1M and 2M rows 0.8 to 1.05).  The row-kernel rows were measured before the narrow
 // form: on the present kernels the estimates are 1.2 times too high in the median (10
 // to 90% of 723 SpMVs: 0.85 to 1.6), and 189 of 201 picks are within 10% or 3 us of the
 // best r.  A new fit picks 194 of 201 for one SpMV, but r = 1 nearly everywhere on
